@@ -84,6 +84,22 @@ __device__ __forceinline__ R hum_region2(R x, R y)
     return re_div(nr, ni, dr, di);
 }
 
+/* FP32 region II with every rounding written out, so that the sums do not
+ * depend on which products the compiler contracts at a call site */
+template <>
+__device__ __forceinline__ float hum_region2<float>(float x, float y)
+{
+    const float c0 = (float)1.410474, c1 = (float).5641896;
+    const float ur = __fmaf_rn(-x, x, __fmul_rn(y, y)), ui = __fmul_rn(__fmul_rn(-2.f, x), y);
+    const float ar = __fmaf_rn(c1, ur, c0), ai = __fmul_rn(c1, ui);
+    const float nr = __fmaf_rn(x, ai, __fmul_rn(y, ar)), ni = __fmaf_rn(y, ai, -__fmul_rn(x, ar));
+    const float br = __fadd_rn(3.f, ur);
+    const float dr = __fadd_rn(.75f, __fmaf_rn(ur, br, -__fmul_rn(ui, ui)));
+    const float di = __fmaf_rn(ur, ui, __fmul_rn(ui, br));
+    return __fmul_rn(__fmaf_rn(nr, dr, __fmul_rn(ni, di)),
+                     rcp_approx(__fmaf_rn(dr, dr, __fmul_rn(di, di))));
+}
+
 template <typename R>
 __device__ __forceinline__ void cmul_add(R& pr, R& pi, R tr, R ti, R c)
 {
@@ -141,33 +157,72 @@ __device__ __forceinline__ R hum_region4(R x, R y)
     return expcos(ur, ui) - re_div(nr, ni, qr, qi);
 }
 
-/* Region IV for the FP32 form's core kernel: the rational part in FP64
- * (its real part comes out of a mostly imaginary quotient, so FP32 rounding
- * would be amplified), exp(U) cos(Im U) in FP32.  In region IV |x| < 5.5 and
- * y < 0.195|x| - 0.176, so Re U >= -30.25 (no underflow), |Im U| < 10, and
- * Re w = exp-term + a non-negative part: the FP32 error of the exp term
+/* 1/d in FP64: the hardware's approximate reciprocal refined by one step of
+ * Householder's third-order iteration, r (1 + e + e^2) with e = 1 - d r
+ * (e ~ 2^-20, so the truncation is ~2^-60): three FMAs against the longer
+ * instruction sequence of the IEEE division.  For finite d with 1/d normal
+ * (no special cases); within 1 ulp of the correctly rounded value. */
+__device__ __forceinline__ double rcp_f64(double d)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
+/* p(z) of a polynomial with real coefficients c[0..N] (ascending) at the
+ * complex z with s = 2 Re z and q = |z|^2, by division by z's quadratic
+ * factor (Knuth, TAOCP 2, 4.6.4): two FMAs per coefficient against four of
+ * the complex Horner form.  p = u + z v. */
+template <int N>
+__device__ __forceinline__ void quad_horner(const double (&c)[N + 1], double s, double q,
+                                            double& u, double& v)
+{
+    double b1 = c[N], b2 = 0.0;
+#pragma unroll
+    for (int k = N - 1; k >= 1; --k) {
+        const double b = k == N - 1 ? fma(s, b1, c[k]) : fma(s, b1, fma(-q, b2, c[k]));
+        b2 = b1; b1 = b;
+    }
+    v = b1;
+    u = fma(-q, b2, c[0]);
+}
+
+/* Regions III and IV for the FP32 form's core: the rational parts in FP64
+ * (their real part comes out of a mostly imaginary quotient, so FP32
+ * rounding would be amplified), exp(U) cos(Im U) in FP32.  The division by
+ * the quadratic factor loses a few bits more than complex Horner (~2e-13 of
+ * the result), far below the FP32 form's rounding.  In region IV |x| < 5.5
+ * and y < 0.195|x| - 0.176, so Re U >= -30.25 (no underflow), |Im U| < 10,
+ * and Re w = exp-term + a non-negative part: the FP32 error of the exp term
  * (a few 1e-7 of that term) is at most a few 1e-7 of the result. */
+__device__ __forceinline__ double hum_region3_core(double x, double y)
+{
+    /* T = (y, -x) */
+    const double s = 2.0 * y, q = fma(x, x, y * y);
+    const double cn[5] = {16.4955, 20.20933, 11.96482, 3.778987, .5642236};
+    const double cd[6] = {16.4955, 38.82363, 39.27121, 21.69274, 6.699398, 1.0};
+    double nu, nv, du, dv;
+    quad_horner<4>(cn, s, q, nu, nv);
+    quad_horner<5>(cd, s, q, du, dv);
+    const double nr = fma(y, nv, nu), ni = -x * nv, dr = fma(y, dv, du), di = -x * dv;
+    return fma(nr, dr, ni * di) * rcp_f64(fma(dr, dr, di * di));
+}
+
 __device__ __forceinline__ double hum_region4_core(double x, double y)
 {
-    const double ur = y * y - x * x, ui = -2.0 * x * y;
-    const double vr = -ur, vi = -ui;
-    double pr = .56419, pi = 0.0;
-    cmul_add(pr, pi, vr, vi, 1.320522);
-    cmul_add(pr, pi, vr, vi, 35.76683);
-    cmul_add(pr, pi, vr, vi, 219.0313);
-    cmul_add(pr, pi, vr, vi, 1540.787);
-    cmul_add(pr, pi, vr, vi, 3321.9905);
-    cmul_add(pr, pi, vr, vi, 36183.31);
-    double qr = 1.0, qi = 0.0;
-    cmul_add(qr, qi, vr, vi, 1.841439);
-    cmul_add(qr, qi, vr, vi, 61.57037);
-    cmul_add(qr, qi, vr, vi, 364.2191);
-    cmul_add(qr, qi, vr, vi, 2186.181);
-    cmul_add(qr, qi, vr, vi, 9022.228);
-    cmul_add(qr, qi, vr, vi, 24322.84);
-    cmul_add(qr, qi, vr, vi, 32066.6);
-    const double nr = y * pr + x * pi, ni = y * pi - x * pr;
-    return (double)expcos<float>((float)ur, (float)ui) - re_div(nr, ni, qr, qi);
+    /* V = -U = (x^2 - y^2, 2 x y); P, Q polynomials in V */
+    const double vr = fma(x, x, -(y * y)), vi = 2.0 * x * y;
+    const double h = fma(x, x, y * y), s = 2.0 * vr, q = h * h;
+    const double cp[7] = {36183.31, 3321.9905, 1540.787, 219.0313, 35.76683, 1.320522, .56419};
+    const double cq[8] = {32066.6, 24322.84, 9022.228, 2186.181, 364.2191, 61.57037, 1.841439, 1.0};
+    double pu, pv, qu, qv;
+    quad_horner<6>(cp, s, q, pu, pv);
+    quad_horner<7>(cq, s, q, qu, qv);
+    const double pr = fma(vr, pv, pu), pi = vi * pv, qr = fma(vr, qv, qu), qi = vi * qv;
+    const double nr = fma(y, pr, x * pi), ni = fma(y, pi, -(x * pr));
+    return (double)expcos<float>((float)-vr, (float)-vi) -
+           fma(nr, qr, ni * qi) * rcp_f64(fma(qr, qr, qi * qi));
 }
 
 /* region selected by integer bin limits: 1..4 */

@@ -52,7 +52,7 @@ bool slices_apply(int pk, int prec);
 long long slice_lines(const gexs_job* jobs, int njobs, int tile_w, int* max_rows);
 /* the FP32 Voigt core kernel's own slices (its line range per tile is the
  * lines whose core can reach the tile): only when a tile is one core
- * sub-tile (tile_w <= 1024); 8192 lines per slice unless the rows, bounded
+ * sub-tile (tile_w <= 1024); 2048 lines per slice unless the rows, bounded
  * by the core reach 15 nu dop_coef instead of the cutoff, would pass 1 GiB */
 bool core_slices_apply(int pk, int prec, int tile_w);
 long long core_slice_lines(const gexs_job* jobs, int njobs, int tile_w, int* max_rows);

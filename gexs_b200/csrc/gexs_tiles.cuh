@@ -1613,23 +1613,23 @@ voigt_ws_kernel(const KArgs args)
  * most CORE_W bins.  Per sub-tile, the lines whose core can reach it
  * (|f - nu| < 15 / invw = 15 nu dop_coef, inside the cutoff) are found by
  * two warp searches and taken 32 at a time by the warps in turn, one line
- * per lane, derived in FP64 with the region-I kernel's predicates.  A warp
- * then steps through the union of its 32 lines' cores bin by bin: at bin t
- * every lane evaluates its own line in the region t falls in (II in FP32,
- * III and the rational part of IV in FP64, IV's exp term in FP32), a
- * butterfly of shuffles sums the 32 terms in a fixed order, and lane 0
- * adds the sum into the warp's row of doubles.  Lines that
- * are neighbours in nu have overlapping cores, so most lanes work at every
- * step and no lane scans for work.  A bin receives its core terms in a
- * fixed order (groups of 32 lines in ascending order per warp, rows added
- * in warp order), so results are bitwise independent of batching. */
+ * per lane, derived in FP64 with the region-I kernel's predicates.  Each
+ * lane then walks its own line's bins, one region at a time, and adds the
+ * terms into the warp's row of doubles (scatter_phase).  The walk is bound
+ * by the FP64 arithmetic of region IV (about 45 FP64 instructions per bin);
+ * all lanes of a step are in the same region, and neighbouring lines have
+ * nearly equal ranges, so most lanes work.  Stepping the union of the 32
+ * cores bin by bin instead (every lane at the same bin, a butterfly per
+ * bin) ran each region's code at nearly every step: 10.0 against 4.4 ms for
+ * eight (T, P) pairs of a 1e6-line list (sparse, fine grids), 6.0 against
+ * 4.6 ms for a dense 2e7-line list at 1 bar, 33 against 21 us for 3000
+ * lines on 6001 bins.  Two bins per step made the code too long for the
+ * instruction cache (5.4 ms on the dense list). */
 constexpr int CORE_W = 1024;
 constexpr int CORE_WARPS = 4;
 
-struct CoreSmem {
-    static constexpr int NT = CORE_WARPS * 32;
-    static constexpr size_t bytes = (size_t)CORE_WARPS * CORE_W * sizeof(double);
-};
+/* one row of doubles per warp, as wide as a sub-tile */
+__host__ __device__ constexpr int core_row(int tile_w) { return tile_w < CORE_W ? tile_w : CORE_W; }
 
 /* the core of a line as single-region bin ranges, c3 within c2 within c1
  * (an empty inner range collapses to a point):
@@ -1644,20 +1644,86 @@ __device__ __forceinline__ void core_ranges(int c1, int c2, int c3, int& c1a, in
     if (c3a >= c3b) c3a = c3b = c2b;
 }
 
-/* ORDER: the launch's items may be tile-major (its own instantiation: the
- * decode's divisions cost this kernel 8 registers when compiled in) */
+/* Every lane walks its own bins [a, b) of the tile (a >= b: none) and adds
+ * val(t) into row[t].  The ranges are taken in passes of M bins, M the
+ * length of the warp's longest range over the number of passes (M <= 32).
+ * The warp's lanes form groups of M; at step k lane j of a group takes its
+ * bin of residue (k + j) mod M, so the lanes of a group are always at
+ * different bins and add without conflict, and a bin receives its terms in
+ * an order that depends on the 32 ranges alone (the sums are reproducible).
+ * With several groups each adds into a private strip of `scr` (zero on
+ * entry and on return) that covers the ranges' union, and the strips are
+ * added to the row in group order at the end: the groups adding to the row
+ * one after another cost as much as the terms (1.63 against 0.84 ms
+ * without any adds, 4e6 lines at 0.01 cm^-1).  Only a union wider than a
+ * strip (sparse lines) takes that form. */
+constexpr int SCR_D = 544;               /* doubles of a warp's strips */
+
+template <typename F>
+__device__ __forceinline__ void scatter_phase(int a, int b, int lane, double* row, double* scr,
+                                              const F& val)
+{
+    constexpr unsigned ALL = 0xffffffffu;
+    const int longest = __reduce_max_sync(ALL, max(b - a, 0));
+    if (longest == 0) return;
+    const int passes = (longest + 31) / 32;
+    const int M = max((longest + passes - 1) / passes, 4);
+    const int groups = (31 + M) / M, mine = lane / M;
+    int lo = 0, span = 0;
+    const int strip = SCR_D / groups;
+    if (groups > 1) {
+        lo = __reduce_min_sync(ALL, a < b ? a : INT32_MAX);
+        span = __reduce_max_sync(ALL, a < b ? b : INT32_MIN) - lo;
+    }
+    const bool strips = groups > 1 && span <= strip;
+    double* dst = strips ? scr + mine * strip - lo : row;
+    const int rounds = strips ? 1 : groups;
+    int o = (lane - a) % M;
+    if (o < 0) o += M;
+    for (int base = 0; base < longest; base += M) {
+#pragma unroll 1
+        for (int k = 0; k < M; ++k) {
+            const int t = a + base + o;
+            if (++o == M) o = 0;
+            const bool on = t < b;
+            if (!__any_sync(ALL, on)) continue;
+            const double v = val(t);      /* dropped if t is outside */
+            if (rounds == 1) {
+                if (on) dst[t] += v;
+                __syncwarp();
+            } else {
+                for (int g = 0; g < rounds; ++g) {
+                    if (on && mine == g) dst[t] += v;
+                    __syncwarp();
+                }
+            }
+        }
+    }
+    if (strips) {
+        for (int u = lane; u < span; u += 32) {
+            double v = 0.0;
+            for (int g = 0; g < groups; ++g) { v += scr[g * strip + u]; scr[g * strip + u] = 0.0; }
+            row[lo + u] += v;
+        }
+        __syncwarp();
+    }
+}
+
 template <bool PREP, bool ORDER>
-__global__ void __launch_bounds__(CORE_WARPS * 32)
+__global__ void __launch_bounds__(CORE_WARPS * 32, 24 / CORE_WARPS)
 core_kernel(const KArgs args)
 {
-    constexpr int NT = CoreSmem::NT;
+    constexpr int NT = CORE_WARPS * 32;
     extern __shared__ __align__(16) unsigned char smem[];
     double* s_rows = reinterpret_cast<double*>(smem);
     __shared__ int s_item;
     __shared__ long long s_lohi[2];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double* row = s_rows + warp * CORE_W;
+    const int RW = core_row(args.tile_w);      /* doubles per warp row */
+    double* row = s_rows + warp * RW;
+    double* scr = s_rows + CORE_WARPS * RW + warp * SCR_D;
+    for (int z = lane; z < SCR_D; z += 32) scr[z] = 0.0;
     /* sliced (host-enabled only when a tile is one sub-tile of CORE_W) */
     const bool sliced = args.csl.prefix != nullptr;
     const int nitems = sliced ? *(volatile const int*)args.csl.nitems : args.nitems;
@@ -1709,19 +1775,21 @@ core_kernel(const KArgs args)
                     s_lohi[0] = min(a0, thi);
                     s_lohi[1] = min(a0 + per, thi);
                 }
-            } else if (warp == 0) {
-                int64_t v = warp_bound<false>(J.lines.nu, nl, vlo, lane);
-                if (lane == 0) s_lohi[0] = v;
-            } else if (warp == 1) {
-                int64_t v = warp_bound<true>(J.lines.nu, nl, vhi, lane);
-                if (lane == 0) s_lohi[1] = v;
+            } else {
+                if (warp == 0) {
+                    int64_t v = warp_bound<false>(J.lines.nu, nl, vlo, lane);
+                    if (lane == 0) s_lohi[0] = v;
+                }
+                if (warp == CORE_WARPS - 1) {
+                    int64_t v = warp_bound<true>(J.lines.nu, nl, vhi, lane);
+                    if (lane == 0) s_lohi[1] = v;
+                }
             }
-            for (int z = tid; z < CORE_WARPS * CORE_W; z += NT) s_rows[z] = 0.0;
+            for (int z = tid; z < CORE_WARPS * RW; z += NT) s_rows[z] = 0.0;
             __syncthreads();
             const int64_t lo = s_lohi[0], hi = max((int64_t)s_lohi[1], lo);
             for (int64_t g0 = lo + (int64_t)warp * 32; g0 < hi; g0 += NT) {
                 const int64_t i = g0 + lane;
-                bool has = false;
                 int c1a = 0, c1b = 0, c2a = 0, c2b = 0, c3a = 0, c3b = 0;
                 double nu = 0.0, invw = 0.0, y = 0.0, amp = 0.0;
                 float icf = 0.f, fc = 0.f, dx = 0.f, yf = 0.f, ampf = 0.f;
@@ -1740,7 +1808,6 @@ core_kernel(const KArgs args)
                     }
                     Derived<PK_VOIGT> d = derive_line<PK_VOIGT>(T, lq, 10.5);
                     if (lo16(d.c1) < hi16(d.c1)) {
-                        has = true;
                         core_ranges(d.c1, d.c2, d.c3, c1a, c1b, c2a, c2b, c3a, c3b);
                         const double ic = fmin(fmax(floor(d.tc), -8388608.0), 8388607.0);
                         nu = d.nu; invw = d.invw; y = d.y;
@@ -1750,44 +1817,24 @@ core_kernel(const KArgs args)
                         yf = (float)y; ampf = (float)amp;
                     }
                 }
-                /* union of the warp's cores */
-                int ulo = has ? c1a : INT32_MAX, uhi = has ? c1b : INT32_MIN;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    ulo = min(ulo, __shfl_xor_sync(0xffffffffu, ulo, o));
-                    uhi = max(uhi, __shfl_xor_sync(0xffffffffu, uhi, o));
-                }
-                auto term = [&](int t) -> double {
-                    double v = 0.0;
-                    if (has && t >= c1a && t < c1b) {
-                        if (t < c2a || t >= c2b) {
-                            const float x = fabsf(((float)t - icf) - fc) * dx;
-                            v = (double)(ampf * hum_region2<float>(x, yf));
-                        } else {
-                            const double x = dmul(fabs(dsub(grid_f(J.nu_start, J.dnu, T.j0 + t), nu)), invw);
-                            v = amp * ((t >= c3a && t < c3b) ? hum_region3<double>(x, y)
-                                                             : hum_region4_core(x, y));
-                        }
-                    }
-                    return v;
+                __syncwarp();
+                /* II left and right of the inner part, FP32 */
+#pragma unroll 1
+                for (int side = 0; side < 2; ++side)
+                    scatter_phase(side ? c2b : c1a, side ? c1b : c2a, lane, row, scr, [&](int t) {
+                        const float x = fabsf(((float)t - icf) - fc) * dx;
+                        return (double)__fmul_rn(ampf, hum_region2<float>(x, yf));
+                    });
+                auto x_of = [&](int t) {
+                    return dmul(fabs(dsub(grid_f(J.nu_start, J.dnu, T.j0 + t), nu)), invw);
                 };
-                /* two bins per step: their butterflies are independent, so the
-                 * shuffles of one overlap the other's; each bin's terms are
-                 * summed in the same order as one bin per step */
-                for (int t = ulo; t < uhi; t += 2) {
-                    const bool two = t + 1 < uhi;      /* warp-uniform */
-                    double v0 = term(t);
-                    double v1 = two ? term(t + 1) : 0.0;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-                        v1 += __shfl_xor_sync(0xffffffffu, v1, o);
-                    }
-                    if (lane == 0) {
-                        row[t] += v0;
-                        if (two) row[t + 1] += v1;
-                    }
-                }
+                /* IV left and right of III */
+#pragma unroll 1
+                for (int side = 0; side < 2; ++side)
+                    scatter_phase(side ? c3b : c2a, side ? c2b : c3a, lane, row, scr,
+                                  [&](int t) { return amp * hum_region4_core(x_of(t), y); });
+                scatter_phase(c3a, c3b, lane, row, scr,
+                              [&](int t) { return amp * hum_region3_core(x_of(t), y); });
             }
             __syncthreads();
             if (ns == 1) {
@@ -1797,7 +1844,7 @@ core_kernel(const KArgs args)
                     bool any = false;
 #pragma unroll
                     for (int w = 0; w < CORE_WARPS; ++w) {
-                        const double r = s_rows[w * CORE_W + t];
+                        const double r = s_rows[w * RW + t];
                         any |= (r != 0.0);
                         v += r;
                     }
@@ -1813,7 +1860,7 @@ core_kernel(const KArgs args)
                 for (int t = tid; t < T.jn; t += NT) {
                     double v = 0.0;
 #pragma unroll
-                    for (int w = 0; w < CORE_WARPS; ++w) v += s_rows[w * CORE_W + t];
+                    for (int w = 0; w < CORE_WARPS; ++w) v += s_rows[w * RW + t];
                     prow[t] = v;
                 }
                 __threadfence();
@@ -1949,7 +1996,7 @@ template <bool PREP>
 static cudaError_t launch_core(const KArgs& a, int nsm, cudaStream_t st)
 {
     auto kern = a.order ? core_kernel<PREP, true> : core_kernel<PREP, false>;
-    const size_t smem = CoreSmem::bytes;
+    const size_t smem = (size_t)CORE_WARPS * (core_row(a.tile_w) + SCR_D) * sizeof(double);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int occ = 0;
