@@ -114,12 +114,13 @@ constexpr int PK_VOIGT_CLASS = 0;
 
 static gexs_launch_cfg default_cfg(int pk, int prec)
 {
-    /* measured best on B200 for the 1e8-line Voigt workload (FP32: 4 bins x
-     * 4 warps with 256-line stages, FP64: 4 x 8); gexs_autotune replaces it
+    /* measured best on B200 (FP32 Voigt on 1e8 lines: 4 bins x 4 warps with
+     * 256-line stages; FP64 Voigt on 5e6 lines, 0.01 cm^-1: 4 x 4, 20.3
+     * against 21.3 ms at 4 x 8; other FP64 forms 4 x 8); gexs_autotune replaces it
      * per (profile, precision) */
     gexs_launch_cfg c{};
     c.bins_per_lane = 4;
-    c.warps = (prec == GEXS_FP64) ? 8 : 4;
+    c.warps = (prec == GEXS_FP64 && pk != PK_VOIGT_CLASS) ? 8 : 4;
     c.ctas_per_sm = 0;
     c.flags = (pk == PK_VOIGT_CLASS && prec == GEXS_FP32) ? GEXS_LAUNCH_LONG_STAGES : 0;
     return c;
@@ -264,7 +265,7 @@ static Layout group_layout(const Group& g, bool prep, const gexs_launch_cfg& cfg
         const int W = tile_bins(cfg);
         const size_t nt = (size_t)g.nitems;
         L.sliced = true;
-        L.lines_per_slice = slice_lines(g.jobs.data(), (int)g.jobs.size(), W, &L.max_rows);
+        L.lines_per_slice = slice_lines(g.jobs.data(), (int)g.jobs.size(), g.prec, W, &L.max_rows);
         L.os_prefix = up(a); a = L.os_prefix + (nt + 1) * sizeof(int);
         L.os_counts = up(a); a = L.os_counts + nt * sizeof(int);
         L.os_rowbase = up(a); a = L.os_rowbase + nt * sizeof(int);
@@ -274,14 +275,15 @@ static Layout group_layout(const Group& g, bool prep, const gexs_launch_cfg& cfg
         L.os_rows = up(a);   a = L.os_rows + (size_t)L.max_rows * W * sizeof(double);
         if (core_slices_apply(g.pk, g.prec, W)) {
             L.csliced = true;
-            L.clines_per_slice = core_slice_lines(g.jobs.data(), (int)g.jobs.size(), W, &L.cmax_rows);
+            L.clines_per_slice = core_slice_lines(g.jobs.data(), (int)g.jobs.size(), g.prec, W,
+                                                  &L.cmax_rows);
             L.oc_prefix = up(a); a = L.oc_prefix + (nt + 1) * sizeof(int);
             L.oc_counts = up(a); a = L.oc_counts + nt * sizeof(int);
             L.oc_rowbase = up(a); a = L.oc_rowbase + nt * sizeof(int);
             L.oc_ticket = up(a); a = L.oc_ticket + nt * sizeof(int);
             L.oc_lohi = up(a);   a = L.oc_lohi + 2 * nt * sizeof(long long);
             L.oc_nitems = up(a); a = L.oc_nitems + 256;
-            L.oc_rows = up(a);   a = L.oc_rows + (size_t)L.cmax_rows * W * sizeof(double);
+            L.oc_rows = up(a);   a = L.oc_rows + (size_t)L.cmax_rows * core_row_doubles(g.prec, W) * sizeof(double);
         }
     }
     L.bytes = a + 256;

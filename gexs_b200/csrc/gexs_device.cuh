@@ -57,10 +57,24 @@ __device__ __forceinline__ R hum_region1(R x, R y)
     return HC<R>::k(0.5641896) * y * num / den;
 }
 
+/* 1/d in FP64: the hardware's approximate reciprocal refined by one step of
+ * Householder's third-order iteration, r (1 + e + e^2) with e = 1 - d r
+ * (e ~ 2^-20, so the truncation is ~2^-60): three FMAs against the longer
+ * instruction sequence of the IEEE division.  For finite d with 1/d normal
+ * (no special cases); within 1 ulp of the correctly rounded value. */
+__device__ __forceinline__ double rcp_f64(double d)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
 template <typename R>
 __device__ __forceinline__ R re_div(R nr, R ni, R dr, R di)
 {
-    return (nr * dr + ni * di) / (dr * dr + di * di);
+    /* FP64; |d|^2 is between ~1e-1 and ~1e30 in regions II-IV */
+    return fma(nr, dr, ni * di) * rcp_f64(fma(dr, dr, di * di));
 }
 /* FP32: one approximate reciprocal (1 ulp) instead of an IEEE division */
 template <>
@@ -157,19 +171,6 @@ __device__ __forceinline__ R hum_region4(R x, R y)
     return expcos(ur, ui) - re_div(nr, ni, qr, qi);
 }
 
-/* 1/d in FP64: the hardware's approximate reciprocal refined by one step of
- * Householder's third-order iteration, r (1 + e + e^2) with e = 1 - d r
- * (e ~ 2^-20, so the truncation is ~2^-60): three FMAs against the longer
- * instruction sequence of the IEEE division.  For finite d with 1/d normal
- * (no special cases); within 1 ulp of the correctly rounded value. */
-__device__ __forceinline__ double rcp_f64(double d)
-{
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    const double e = fma(-d, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-
 /* p(z) of a polynomial with real coefficients c[0..N] (ascending) at the
  * complex z with s = 2 Re z and q = |z|^2, by division by z's quadratic
  * factor (Knuth, TAOCP 2, 4.6.4): two FMAs per coefficient against four of
@@ -225,14 +226,12 @@ __device__ __forceinline__ double hum_region4_core(double x, double y)
            fma(nr, qr, ni * qi) * rcp_f64(fma(qr, qr, qi * qi));
 }
 
-/* region selected by integer bin limits: 1..4 */
-template <typename R>
-__device__ __forceinline__ R hum_by_region(int reg, R x, R y)
+/* regions II-IV by the tests of compute/CPU/profiles.cpp:24,31 */
+static __device__ __noinline__ double hum_core_f64(double x, double y)
 {
-    if (reg == 1) return hum_region1(x, y);
-    if (reg == 2) return hum_region2(x, y);
-    if (reg == 3) return hum_region3(x, y);
-    return hum_region4(x, y);
+    if (dadd(x, y) >= 5.5) return hum_region2<double>(x, y);
+    if (y >= dsub(dmul(0.195, x), 0.176)) return hum_region3<double>(x, y);
+    return hum_region4<double>(x, y);
 }
 
 /* --------------------------------------------------- Gauss-Hermite Voigt

@@ -291,7 +291,8 @@ bool slices_apply(int, int) { return true; }
 
 bool core_slices_apply(int pk, int prec, int tile_w)
 {
-    return pk == PK_VOIGT && prec == GEXS_FP32 && tile_w <= CORE_W;
+    (void)prec;
+    return pk == PK_VOIGT && tile_w <= CORE_W;
 }
 
 /* A split tile of n lines has ceil(n / per) <= n / per + 1 slices, so for M
@@ -307,7 +308,9 @@ static double tiles_of(const gexs_job& j, int tile_w)
     return std::ceil((double)j.n_points / (double)tile_w);
 }
 
-long long core_slice_lines(const gexs_job* jobs, int njobs, int tile_w, int* max_rows)
+int core_row_doubles(int prec, int tile_w) { return prec == GEXS_FP64 ? 2 * tile_w : tile_w; }
+
+long long core_slice_lines(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows)
 {
     /* as slice_lines, with a line's reach the core's: at most 15 nu
      * dop_coef / (1 - 15 dop_coef) at the job's highest frequency, and at
@@ -326,7 +329,7 @@ long long core_slice_lines(const gexs_job* jobs, int njobs, int tile_w, int* max
             const double tpl = std::floor((2.0 * reach + 8.0 * j.dnu) / ((double)tile_w * j.dnu)) + 3.0;
             rows += row_bound((double)j.lines.count * tpl, tiles_of(j, tile_w), (double)per);
         }
-        if (rows * tile_w * sizeof(double) <= (double)(1ull << 30)) {
+        if (rows * core_row_doubles(prec, tile_w) * sizeof(double) <= (double)(1ull << 30)) {
             *max_rows = (int)rows;
             return per;
         }
@@ -335,7 +338,7 @@ long long core_slice_lines(const gexs_job* jobs, int njobs, int tile_w, int* max
     }
 }
 
-long long slice_lines(const gexs_job* jobs, int njobs, int tile_w, int* max_rows)
+long long slice_lines(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows)
 {
     /* A line lies in at most (2 (cutoff + margin)) / (tile width) + 2 tiles,
      * so the tiles hold at most sum(lines x that) = M line entries.  A split
@@ -346,7 +349,7 @@ long long slice_lines(const gexs_job* jobs, int njobs, int tile_w, int* max_rows
      * is smaller.  16384 lines per slice: measured on one
      * B200, the 1e8-line workload is indifferent to it (16k-128k) and a
      * dense band of 1e6 lines in 80 cm^-1 runs 25% faster than at 65536. */
-    long long per = 16384;
+    long long per = prec == GEXS_FP32 ? 16384 : 2048;
     for (;;) {
         double rows = 0.0, need = 0.0;
         for (int i = 0; i < njobs; ++i) {

@@ -68,8 +68,8 @@ constexpr int GH_PAIR_BIT = 1 << 25;
 struct __align__(16) RecF64 {   /* 64 bytes */
     double nu;             /* centre after the nu==0 rule                   */
     double invw;
-    double y;              /* Voigt/GH: y ; Doppler: unused                 */
-    double amp;            /* Voigt/GH: S*invw ; Doppler: S                 */
+    double y;              /* GH: y ; Doppler: unused                       */
+    double amp;            /* GH: S*invw ; Doppler: S                       */
     int    win, c1, c2, c3;
     int    mask, pad0, pad1, pad2;
 };
@@ -93,10 +93,26 @@ struct __align__(16) RecV {
 };
 
 
+/* FP64 Voigt record (64 bytes): a full-tier line takes the first 48 */
+struct __align__(16) RecV64 {
+    double nu, invw;
+    double c;              /* y^2 - 1/2                                      */
+    double y2;             /* 2 y^2                                          */
+    double a;              /* amp * 0.5641896 * y; tier 3: amp (= S * invw *
+                              out_scale)                                     */
+    int    tiers;          /* 2 bits per warp, as RecV.tiers; 3 is per bin,
+                              with IEEE divisions: |x| or y may exceed 1e60,
+                              or y < 0 (the line's core included)            */
+    int    win;
+    int    c1, pad;
+    double y;
+};
+
 /* record type of a (profile class, precision) */
 template <int PK, int PREC> struct RecOf;
 template <int PK> struct RecOf<PK, GEXS_FP32> { typedef RecF32 T; };
 template <int PK> struct RecOf<PK, GEXS_FP64> { typedef RecF64 T; };
+template <> struct RecOf<PK_VOIGT, GEXS_FP64> { typedef RecV64 T; };
 
 __device__ __forceinline__ int pack2(int a, int b) { return a | (b << 16); }
 __device__ __forceinline__ int lo16(int v) { return v & 0xffff; }
@@ -497,6 +513,23 @@ __device__ __forceinline__ void make_rec(RecF64& q, const Derived<PK>& d, const 
 }
 
 
+template <int PK, int B, int WARPS>
+__device__ __forceinline__ void make_rec(RecV64& q, const Derived<PK>& d, const gexs_job& J,
+                                         const Tile& T)
+{
+    const double amp = dmul(dmul(d.S, d.invw), J.out_scale);
+    const double dfar = fmax(fabs(d.nu - T.f0), fabs(d.nu - T.fl));
+    /* beyond: x^4 or y^4 could overflow, or (y < 0) the core kernel's line
+     * search, which assumes y >= 0, could miss the line */
+    const bool general = !(dfar * d.invw < 1e60) || !(d.y < 1e60) || d.y < 0.0;
+    q.nu = d.nu; q.invw = d.invw; q.y = d.y;
+    q.c = d.y * d.y - 0.5;
+    q.y2 = 2.0 * d.y * d.y;
+    q.a = general ? amp : amp * 0.5641896 * d.y;
+    q.win = d.win; q.c1 = d.c1; q.pad = 0;
+    q.tiers = (d.win == 0) ? 0 : voigt_tiers<B, WARPS>(d, general);
+}
+
 /* accumulator of bin k of a lane: pairs (2j, 2j+1) share one float2 so the
  * Voigt loop runs on packed f32x2 instructions; k is a compile-time
  * constant after unrolling */
@@ -842,8 +875,9 @@ __device__ __forceinline__ void lines_voigt_f32(const RecV* __restrict__ rec, in
     }
 }
 
-/* FP64 form: per-bin window and region tests, FP64 arithmetic, bins sum
- * their lines in line order (the order of the FP64 oracle). */
+/* FP64 form of the Doppler/Gaussian and Gauss-Hermite profiles: per-bin
+ * window tests, FP64 arithmetic, bins sum their lines in line order (the
+ * order of the FP64 oracle). */
 template <int PK, int B>
 __device__ __forceinline__ void lines_f64(const RecF64* __restrict__ rec, int nrec, int warp,
                                           int lane, const double (&fbin)[B], double (&acc)[B],
@@ -856,21 +890,7 @@ __device__ __forceinline__ void lines_f64(const RecF64* __restrict__ rec, int nr
         const RecF64& q = rec[i];
         if (!(q.mask & bit)) continue;
         const int a = lo16(q.win), b = hi16(q.win);
-        if constexpr (PK == PK_VOIGT) {
-            const int c1 = q.c1, c2 = q.c2, c3 = q.c3;
-#pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const int t = wb + lane + 32 * k;
-                if (t < a || t >= b) continue;
-                double x = dmul(fabs(dsub(fbin[k], q.nu)), q.invw);
-                int reg;
-                if (t < lo16(c1) || t >= hi16(c1)) reg = 1;
-                else if (t < lo16(c2) || t >= hi16(c2)) reg = 2;
-                else reg = (t >= lo16(c3) && t < hi16(c3)) ? 3 : 4;
-                double kv = hum_by_region<double>(reg, x, q.y);
-                acc[k] = dadd(acc[k], dmul(dmul(q.amp, kv), out_scale));
-            }
-        } else if constexpr (PK == PK_ERF) {
+        if constexpr (PK == PK_ERF) {
             const int c1a = lo16(q.c1), c1b = hi16(q.c1);
             const int form = J.erf_form;
             const double h = 0.5 * J.dnu;
@@ -895,6 +915,70 @@ __device__ __forceinline__ void lines_f64(const RecF64* __restrict__ rec, int nr
                 double kv = dmul(gh_sum_f64<NODES>(x, y2), yk);
                 acc[k] = dadd(acc[k], dmul(dmul(q.amp, kv), out_scale));
             }
+        }
+    }
+}
+
+/* FP64 Voigt, region I: K = c y (m + 1) / (m^2 + 2 y^2), m = x^2 + y^2 -
+ * 1/2 (the rational of hum_region1 without its cancellation), with 1/d from
+ * rcp_f64: nine FP64 instructions per evaluation (x two, m, d, three of the
+ * reciprocal, two of the sum), so the FP64 pipe bounds the loop at 64 / 9
+ * evaluations per SM-clock.  Per-bin region tests and IEEE divisions took
+ * about 45 issue slots per evaluation.  The core is core_kernel's, as in
+ * the FP32 form. */
+template <int B>
+__device__ __forceinline__ void lines_voigt_f64(const RecV64* __restrict__ rec, int nrec, int warp,
+                                                int lane, const double (&fbin)[B], double (&acc)[B])
+{
+    const int sh = 2 * warp, tl = warp * 32 * B + lane;
+    for (int i = 0; i < nrec; ++i) {
+        const RecV64& q = rec[i];
+        const double a = q.a;
+        const int tier = (q.tiers >> sh) & 3;
+        if (tier == 0) continue;
+        if (tier == 3) {
+            const int wa = lo16(q.win), wb = hi16(q.win), ca = lo16(q.c1), cb = hi16(q.c1);
+            const double y = q.y;
+#pragma unroll 1
+            for (int k = 0; k < B; ++k) {
+                const int t = tl + 32 * k;
+                const bool core = t >= ca && t < cb;
+                if (t < wa || t >= wb || (core && !(y < 0.0))) continue;
+                double f = fbin[0];
+#pragma unroll
+                for (int j = 1; j < B; ++j) if (j == k) f = fbin[j];
+                const double x = dmul(fabs(dsub(f, q.nu)), q.invw);
+                const double v = a * (core ? hum_core_f64(x, y) : hum_region1<double>(x, y));
+#pragma unroll
+                for (int j = 0; j < B; ++j) if (j == k) acc[j] += v;
+            }
+            continue;
+        }
+        const double nu = q.nu, invw = q.invw, c = q.c, y2 = q.y2;
+        if (tier == 1) {
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const double x = (fbin[k] - nu) * invw;
+                const double m = fma(x, x, c);
+                const double r = rcp_f64(fma(m, m, y2));
+                acc[k] = fma(a, fma(m, r, r), acc[k]);
+            }
+            continue;
+        }
+        /* partial: bins outside the window or inside the core are evaluated
+         * and dropped */
+        const int wa = lo16(q.win), ca = lo16(q.c1);
+        const unsigned wn = (unsigned)(hi16(q.win) - wa);
+        const unsigned cn = (unsigned)max(hi16(q.c1) - ca, 0);
+#pragma unroll
+        for (int k = 0; k < B; ++k) {
+            const int t = tl + 32 * k;
+            const double x = (fbin[k] - nu) * invw;
+            const double m = fma(x, x, c);
+            const double r = rcp_f64(fma(m, m, y2));
+            const double v = fma(m, r, r);
+            const bool in = (unsigned)(t - wa) < wn && !((unsigned)(t - ca) < cn);
+            acc[k] = fma(a, in ? v : 0.0, acc[k]);
         }
     }
 }
@@ -1097,8 +1181,12 @@ tile_kernel(const KArgs args)
                     for (int j = 0; j < B / 2; ++j) part[j] = make_float2(0.f, 0.f);
                 }
             } else {
-                lines_f64<PK, B>(reinterpret_cast<const RecF64*>(s_rec), nrec, warp, lane, fbin,
-                                 acc, J);
+                if constexpr (PK == PK_VOIGT)
+                    lines_voigt_f64<B>(reinterpret_cast<const RecV64*>(s_rec), nrec, warp, lane,
+                                       fbin, acc);
+                else
+                    lines_f64<PK, B>(reinterpret_cast<const RecF64*>(s_rec), nrec, warp, lane, fbin,
+                                     acc, J);
             }
             __syncthreads();
         }
@@ -1603,7 +1691,7 @@ voigt_ws_kernel(const KArgs args)
     }
 }
 
-/* ------------------------------------------------- FP32 Voigt core kernel
+/* ------------------------------------------------------ Voigt core kernel
  * The core of a line (its bins outside Humlicek region I: regions II, III,
  * IV) is evaluated here, after the region-I kernel, and added into the
  * output.  Kept out of that kernel so it carries no FP64 Humlicek code and
@@ -1659,9 +1747,22 @@ __device__ __forceinline__ void core_ranges(int c1, int c2, int c3, int& c1a, in
  * strip (sparse lines) takes that form. */
 constexpr int SCR_D = 544;               /* doubles of a warp's strips */
 
-template <typename F>
-__device__ __forceinline__ void scatter_phase(int a, int b, int lane, double* row, double* scr,
-                                              const F& val)
+/* (hi, lo) += v with the rounding error kept (Knuth's TwoSum): sums of the
+ * same terms in another order round to the same double */
+__device__ __forceinline__ void dd_add(double& hi, double& lo, double v)
+{
+    const double s = dadd(hi, v), bb = dsub(s, hi);
+    lo = dadd(lo, dadd(dsub(hi, dsub(s, bb)), dsub(v, bb)));
+    hi = s;
+}
+
+/* LO = 0: plain sums.  LO > 0 (the FP64 form): row[t] and row[LO + t] are a
+ * (hi, lo) sum, because that form's results are the same for every tile
+ * shape and the order of the terms here is not; no strips, the groups add
+ * one after another. */
+template <bool DD, typename F>
+__device__ __forceinline__ void scatter_phase(int a, int b, int lane, double* row, int LO,
+                                              double* scr, const F& val)
 {
     constexpr unsigned ALL = 0xffffffffu;
     const int longest = __reduce_max_sync(ALL, max(b - a, 0));
@@ -1671,11 +1772,11 @@ __device__ __forceinline__ void scatter_phase(int a, int b, int lane, double* ro
     const int groups = (31 + M) / M, mine = lane / M;
     int lo = 0, span = 0;
     const int strip = SCR_D / groups;
-    if (groups > 1) {
+    if (!DD && groups > 1) {
         lo = __reduce_min_sync(ALL, a < b ? a : INT32_MAX);
         span = __reduce_max_sync(ALL, a < b ? b : INT32_MIN) - lo;
     }
-    const bool strips = groups > 1 && span <= strip;
+    const bool strips = !DD && groups > 1 && span <= strip;
     double* dst = strips ? scr + mine * strip - lo : row;
     const int rounds = strips ? 1 : groups;
     int o = (lane - a) % M;
@@ -1688,7 +1789,12 @@ __device__ __forceinline__ void scatter_phase(int a, int b, int lane, double* ro
             const bool on = t < b;
             if (!__any_sync(ALL, on)) continue;
             const double v = val(t);      /* dropped if t is outside */
-            if (rounds == 1) {
+            if (DD) {
+                for (int g = 0; g < rounds; ++g) {
+                    if (on && mine == g) dd_add(row[t], row[LO + t], v);
+                    __syncwarp();
+                }
+            } else if (rounds == 1) {
                 if (on) dst[t] += v;
                 __syncwarp();
             } else {
@@ -1709,7 +1815,7 @@ __device__ __forceinline__ void scatter_phase(int a, int b, int lane, double* ro
     }
 }
 
-template <bool PREP, bool ORDER>
+template <int PREC, bool PREP, bool ORDER>
 __global__ void __launch_bounds__(CORE_WARPS * 32, 24 / CORE_WARPS)
 core_kernel(const KArgs args)
 {
@@ -1722,8 +1828,10 @@ core_kernel(const KArgs args)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int RW = core_row(args.tile_w);      /* doubles per warp row */
     double* row = s_rows + warp * RW;
+    constexpr bool DD = PREC == GEXS_FP64;
+    const int LO = DD ? CORE_WARPS * RW : 0;   /* the low parts' rows */
     double* scr = s_rows + CORE_WARPS * RW + warp * SCR_D;
-    for (int z = lane; z < SCR_D; z += 32) scr[z] = 0.0;
+    if (!DD) for (int z = lane; z < SCR_D; z += 32) scr[z] = 0.0;
     /* sliced (host-enabled only when a tile is one sub-tile of CORE_W) */
     const bool sliced = args.csl.prefix != nullptr;
     const int nitems = sliced ? *(volatile const int*)args.csl.nitems : args.nitems;
@@ -1785,7 +1893,7 @@ core_kernel(const KArgs args)
                     if (lane == 0) s_lohi[1] = v;
                 }
             }
-            for (int z = tid; z < CORE_WARPS * RW; z += NT) s_rows[z] = 0.0;
+            for (int z = tid; z < CORE_WARPS * RW + LO; z += NT) s_rows[z] = 0.0;
             __syncthreads();
             const int64_t lo = s_lohi[0], hi = max((int64_t)s_lohi[1], lo);
             for (int64_t g0 = lo + (int64_t)warp * 32; g0 < hi; g0 += NT) {
@@ -1807,7 +1915,8 @@ core_kernel(const KArgs args)
                         lq = line_quantities<true>(J, Lr);
                     }
                     Derived<PK_VOIGT> d = derive_line<PK_VOIGT>(T, lq, 10.5);
-                    if (lo16(d.c1) < hi16(d.c1)) {
+                    /* FP64: the tile kernel keeps lines of y < 0 whole */
+                    if (lo16(d.c1) < hi16(d.c1) && !(PREC == GEXS_FP64 && d.y < 0.0)) {
                         core_ranges(d.c1, d.c2, d.c3, c1a, c1b, c2a, c2b, c3a, c3b);
                         const double ic = fmin(fmax(floor(d.tc), -8388608.0), 8388607.0);
                         nu = d.nu; invw = d.invw; y = d.y;
@@ -1818,50 +1927,64 @@ core_kernel(const KArgs args)
                     }
                 }
                 __syncwarp();
-                /* II left and right of the inner part, FP32 */
-#pragma unroll 1
-                for (int side = 0; side < 2; ++side)
-                    scatter_phase(side ? c2b : c1a, side ? c1b : c2a, lane, row, scr, [&](int t) {
-                        const float x = fabsf(((float)t - icf) - fc) * dx;
-                        return (double)__fmul_rn(ampf, hum_region2<float>(x, yf));
-                    });
                 auto x_of = [&](int t) {
                     return dmul(fabs(dsub(grid_f(J.nu_start, J.dnu, T.j0 + t), nu)), invw);
                 };
+                /* II left and right of the inner part */
+#pragma unroll 1
+                for (int side = 0; side < 2; ++side)
+                    scatter_phase<DD>(side ? c2b : c1a, side ? c1b : c2a, lane, row, LO, scr, [&](int t) {
+                        if constexpr (PREC == GEXS_FP64) return amp * hum_region2<double>(x_of(t), y);
+                        const float x = fabsf(((float)t - icf) - fc) * dx;
+                        return (double)__fmul_rn(ampf, hum_region2<float>(x, yf));
+                    });
                 /* IV left and right of III */
 #pragma unroll 1
                 for (int side = 0; side < 2; ++side)
-                    scatter_phase(side ? c3b : c2a, side ? c2b : c3a, lane, row, scr,
-                                  [&](int t) { return amp * hum_region4_core(x_of(t), y); });
-                scatter_phase(c3a, c3b, lane, row, scr,
-                              [&](int t) { return amp * hum_region3_core(x_of(t), y); });
+                    scatter_phase<DD>(side ? c3b : c2a, side ? c2b : c3a, lane, row, LO, scr, [&](int t) {
+                        const double x = x_of(t);
+                        return amp * (PREC == GEXS_FP64 ? hum_region4<double>(x, y)
+                                                        : hum_region4_core(x, y));
+                    });
+                scatter_phase<DD>(c3a, c3b, lane, row, LO, scr, [&](int t) {
+                    const double x = x_of(t);
+                    return amp * (PREC == GEXS_FP64 ? hum_region3<double>(x, y)
+                                                    : hum_region3_core(x, y));
+                });
             }
             __syncthreads();
-            if (ns == 1) {
-                /* rows in warp order, added to the region-I result */
-                for (int t = tid; t < T.jn; t += NT) {
-                    double v = 0.0;
-                    bool any = false;
+            /* rows in warp order: a bin's total (hi, lo) */
+            auto total = [&](int t, double& hi, double& lo) {
+                hi = lo = 0.0;
 #pragma unroll
-                    for (int w = 0; w < CORE_WARPS; ++w) {
-                        const double r = s_rows[w * RW + t];
-                        any |= (r != 0.0);
-                        v += r;
+                for (int w = 0; w < CORE_WARPS; ++w) {
+                    if (DD) {
+                        dd_add(hi, lo, s_rows[w * RW + t]);
+                        lo = dadd(lo, s_rows[LO + w * RW + t]);
+                    } else {
+                        hi += s_rows[w * RW + t];
                     }
-                    if (any) J.out[T.j0 + t] += v;
+                }
+            };
+            if (ns == 1) {
+                /* added to the region-I result */
+                for (int t = tid; t < T.jn; t += NT) {
+                    double hi, lo;
+                    total(t, hi, lo);
+                    if (hi != 0.0) J.out[T.j0 + t] += hi + lo;
                 }
             } else {
-                /* a slice of a split tile: rows in warp order into its partial
-                 * row, a ticket, and the last slice adds the partial rows in
-                 * slice order (a zero total adds nothing, as above) */
+                /* a slice of a split tile: its totals into its partial row, a
+                 * ticket, and the last slice adds the partial rows in slice
+                 * order (a zero total adds nothing, as above) */
                 const int rb = args.csl.rowbase[ti];
-                const int W = args.tile_w;
-                double* prow = args.csl.rows + (size_t)(rb + sidx) * W;
+                const int W = args.tile_w, RS = DD ? 2 * W : W;
+                double* prow = args.csl.rows + (size_t)(rb + sidx) * RS;
                 for (int t = tid; t < T.jn; t += NT) {
-                    double v = 0.0;
-#pragma unroll
-                    for (int w = 0; w < CORE_WARPS; ++w) v += s_rows[w * RW + t];
-                    prow[t] = v;
+                    double hi, lo;
+                    total(t, hi, lo);
+                    prow[t] = hi;
+                    if (DD) prow[W + t] = lo;
                 }
                 __threadfence();
                 __syncthreads();
@@ -1870,9 +1993,13 @@ core_kernel(const KArgs args)
                 if (s_last) {
                     __threadfence();
                     for (int t = tid; t < T.jn; t += NT) {
-                        double v = 0.0;
-                        for (int q = 0; q < ns; ++q) v += __ldcg(args.csl.rows + (size_t)(rb + q) * W + t);
-                        if (v != 0.0) J.out[T.j0 + t] += v;
+                        double hi = 0.0, lo = 0.0;
+                        for (int q = 0; q < ns; ++q) {
+                            const double* r = args.csl.rows + (size_t)(rb + q) * RS + t;
+                            if (DD) { dd_add(hi, lo, __ldcg(r)); lo = dadd(lo, __ldcg(r + W)); }
+                            else hi += __ldcg(r);
+                        }
+                        if (hi != 0.0) J.out[T.j0 + t] += hi + lo;
                     }
                 }
             }
@@ -1992,11 +2119,12 @@ static cudaError_t launch_cfg(const KArgs& a, const gexs_launch_cfg& c, int nsm,
  * tables reserve 256 bytes for counters) */
 constexpr int CORE_COUNTER_OFFSET = 32;
 
-template <bool PREP>
+template <int PREC, bool PREP>
 static cudaError_t launch_core(const KArgs& a, int nsm, cudaStream_t st)
 {
-    auto kern = a.order ? core_kernel<PREP, true> : core_kernel<PREP, false>;
-    const size_t smem = (size_t)CORE_WARPS * (core_row(a.tile_w) + SCR_D) * sizeof(double);
+    auto kern = a.order ? core_kernel<PREC, PREP, true> : core_kernel<PREC, PREP, false>;
+    const size_t smem = (size_t)CORE_WARPS * sizeof(double) *
+                        (PREC == GEXS_FP64 ? 2 * core_row(a.tile_w) : core_row(a.tile_w) + SCR_D);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int occ = 0;
@@ -2023,14 +2151,19 @@ static cudaError_t launch_pk(int prec, const KArgs& a, const gexs_launch_cfg& cf
                              cudaStream_t st)
 {
     const bool prep = a.prep != nullptr;
-    if (prec == GEXS_FP32) {
-        cudaError_t e = prep ? launch_cfg<PK, GEXS_FP32, true>(a, cfg, nsm, st)
-                             : launch_cfg<PK, GEXS_FP32, false>(a, cfg, nsm, st);
-        if (PK != PK_VOIGT || e != cudaSuccess) return e;
-        return prep ? launch_core<true>(a, nsm, st) : launch_core<false>(a, nsm, st);
+    const bool f32 = prec == GEXS_FP32;
+    cudaError_t e = f32 ? (prep ? launch_cfg<PK, GEXS_FP32, true>(a, cfg, nsm, st)
+                                : launch_cfg<PK, GEXS_FP32, false>(a, cfg, nsm, st))
+                        : (prep ? launch_cfg<PK, GEXS_FP64, true>(a, cfg, nsm, st)
+                                : launch_cfg<PK, GEXS_FP64, false>(a, cfg, nsm, st));
+    if constexpr (PK == PK_VOIGT) {
+        if (e != cudaSuccess) return e;
+        return f32 ? (prep ? launch_core<GEXS_FP32, true>(a, nsm, st)
+                           : launch_core<GEXS_FP32, false>(a, nsm, st))
+                   : (prep ? launch_core<GEXS_FP64, true>(a, nsm, st)
+                           : launch_core<GEXS_FP64, false>(a, nsm, st));
     }
-    return prep ? launch_cfg<PK, GEXS_FP64, true>(a, cfg, nsm, st)
-                : launch_cfg<PK, GEXS_FP64, false>(a, cfg, nsm, st);
+    return e;
 }
 
 /* defined one per translation unit */

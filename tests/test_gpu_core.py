@@ -54,3 +54,26 @@ def test_core_ranges_match_oracle(gpu_ctx, case):
         else:
             rel, band = H.fp32_errors(got, want)
             assert rel <= H.FP32_REL and band <= H.FP32_BAND, (rel, band)
+
+
+@pytest.mark.parametrize("dop,gamma", [(None, -0.02), (1e-58, 0.05), (1e-70, 0.05), (1e-70, 0.0)])
+def test_fp64_general_tier(gpu_ctx, dop, gamma):
+    """FP64 lines outside the fast tiers: y < 0 (the whole line per bin), |x|
+    or y near and beyond 1e60 (IEEE divisions, no x^4 overflow)."""
+    rng = np.random.Generator(np.random.PCG64(5))
+    n, g = 70, 1500
+    L = {"nu": np.sort(rng.uniform(1000.0, 1012.0, n)), "elow": rng.uniform(0.0, 2000.0, n),
+         "aif": 10.0 ** rng.uniform(-2, 1, n), "gns": np.full(n, 3, dtype=np.int32),
+         "gamma": np.where(np.arange(n) % 3 == 0, gamma, 0.04), "n": np.full(n, 0.5)}
+    out = torch.zeros(g, dtype=torch.float64, device="cuda")
+    job = Job(LineList.from_dict(L), out, convention=capi.CONV_PHYSICAL, profile=capi.VOIGT,
+              temperature=900.0, pressure=0.2, partition=100.0, mass=18.0, nu_start=998.0,
+              dnu=0.01, grid_points=g, precision=capi.FP64, cutoff=25.0)
+    if dop is not None:
+        job.c.dop_coef = dop
+    gpu_ctx.run([job])
+    gpu_ctx.check()
+    want = H.oracle_of(job, L)
+    assert np.isfinite(want).all()
+    worst, nbad = H.fp64_mismatch(out.cpu().numpy(), want, abs_floor=1e-13 * np.max(np.abs(want)))
+    assert nbad == 0, worst
