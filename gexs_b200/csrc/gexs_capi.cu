@@ -109,18 +109,18 @@ cudaError_t pool_alloc(cudaMemPool_t pool, void** p, size_t bytes, cudaStream_t 
 }
 }  // namespace gexs
 
-/* profile_class() of GEXS_VOIGT */
-constexpr int PK_VOIGT_CLASS = 0;
+/* profile_class() of GEXS_VOIGT, and of GEXS_DOPPLER and GEXS_GAUSSIAN */
+constexpr int PK_VOIGT_CLASS = 0, PK_ERF_CLASS = 1;
 
 static gexs_launch_cfg default_cfg(int pk, int prec)
 {
     /* measured best on B200 (FP32 Voigt on 1e8 lines: 4 bins x 4 warps with
      * 256-line stages; FP64 Voigt on 5e6 lines, 0.01 cm^-1: 4 x 4, 20.3
-     * against 21.3 ms at 4 x 8; other FP64 forms 4 x 8); gexs_autotune replaces it
+     * against 21.3 ms at 4 x 8; FP64 quadrature 4 x 8); gexs_autotune replaces it
      * per (profile, precision) */
     gexs_launch_cfg c{};
     c.bins_per_lane = 4;
-    c.warps = (prec == GEXS_FP64 && pk != PK_VOIGT_CLASS) ? 8 : 4;
+    c.warps = (prec == GEXS_FP64 && pk > PK_ERF_CLASS) ? 8 : 4;
     c.ctas_per_sm = 0;
     c.flags = (pk == PK_VOIGT_CLASS && prec == GEXS_FP32) ? GEXS_LAUNCH_LONG_STAGES : 0;
     return c;
@@ -231,18 +231,17 @@ static int build_groups(const gexs_job* jobs, int njobs, const gexs_launch_cfg* 
 struct Layout {
     size_t op, oc, opp, oprep, bytes;
     std::vector<size_t> job_prep;   /* byte offset of each job's prep arrays */
-    /* line-slice tables (FP32 Voigt groups): offsets, item bound, lines per slice */
+    /* line-slice tables: offsets, row bound, lines per slice */
     bool sliced = false;
     size_t os_prefix = 0, os_counts = 0, os_rowbase = 0, os_ticket = 0, os_lohi = 0, os_nitems = 0,
            os_rows = 0;
     int max_rows = 0;
     long long lines_per_slice = 0;
-    /* the FP32 Voigt core kernel's slice tables */
+    /* the core kernel's slice tables */
     bool csliced = false;
     size_t oc_prefix = 0, oc_counts = 0, oc_rowbase = 0, oc_ticket = 0, oc_lohi = 0, oc_nitems = 0,
            oc_rows = 0;
-    int cmax_rows = 0;
-    long long clines_per_slice = 0;
+    int cmax_rows = 0, ccut_shift = 0;
 };
 
 static Layout group_layout(const Group& g, bool prep, const gexs_launch_cfg& cfg)
@@ -261,9 +260,9 @@ static Layout group_layout(const Group& g, bool prep, const gexs_launch_cfg& cfg
         L.job_prep.push_back(a);
         if (prep) a = up(a + (size_t)j.lines.count * 3 * sizeof(double));
     }
-    if (slices_apply(g.pk, g.prec) && g.nitems > 0) {
-        const int W = tile_bins(cfg);
-        const size_t nt = (size_t)g.nitems;
+    const int W = tile_bins(cfg);
+    const size_t nt = (size_t)g.nitems;
+    if (slices_apply(g.pk, g.prec) && nt > 0) {
         L.sliced = true;
         L.lines_per_slice = slice_lines(g.jobs.data(), (int)g.jobs.size(), g.prec, W, &L.max_rows);
         L.os_prefix = up(a); a = L.os_prefix + (nt + 1) * sizeof(int);
@@ -272,19 +271,18 @@ static Layout group_layout(const Group& g, bool prep, const gexs_launch_cfg& cfg
         L.os_ticket = up(a); a = L.os_ticket + nt * sizeof(int);
         L.os_lohi = up(a);   a = L.os_lohi + 2 * nt * sizeof(long long);
         L.os_nitems = up(a); a = L.os_nitems + 256;
-        L.os_rows = up(a);   a = L.os_rows + (size_t)L.max_rows * W * sizeof(double);
-        if (core_slices_apply(g.pk, g.prec, W)) {
-            L.csliced = true;
-            L.clines_per_slice = core_slice_lines(g.jobs.data(), (int)g.jobs.size(), g.prec, W,
-                                                  &L.cmax_rows);
-            L.oc_prefix = up(a); a = L.oc_prefix + (nt + 1) * sizeof(int);
-            L.oc_counts = up(a); a = L.oc_counts + nt * sizeof(int);
-            L.oc_rowbase = up(a); a = L.oc_rowbase + nt * sizeof(int);
-            L.oc_ticket = up(a); a = L.oc_ticket + nt * sizeof(int);
-            L.oc_lohi = up(a);   a = L.oc_lohi + 2 * nt * sizeof(long long);
-            L.oc_nitems = up(a); a = L.oc_nitems + 256;
-            L.oc_rows = up(a);   a = L.oc_rows + (size_t)L.cmax_rows * core_row_doubles(g.prec, W) * sizeof(double);
-        }
+        L.os_rows = up(a);   a = L.os_rows + (size_t)L.max_rows * row_doubles(g.prec, W) * sizeof(double);
+    }
+    if (core_slices_apply(g.pk, g.prec, W) && nt > 0) {
+        L.csliced = true;
+        L.ccut_shift = core_cut_shift(g.jobs.data(), (int)g.jobs.size(), g.prec, W, &L.cmax_rows);
+        L.oc_prefix = up(a); a = L.oc_prefix + (nt + 1) * sizeof(int);
+        L.oc_counts = up(a); a = L.oc_counts + nt * sizeof(int);
+        L.oc_rowbase = up(a); a = L.oc_rowbase + nt * sizeof(int);
+        L.oc_ticket = up(a); a = L.oc_ticket + nt * sizeof(int);
+        L.oc_lohi = up(a);   a = L.oc_lohi + 2 * nt * sizeof(long long);
+        L.oc_nitems = up(a); a = L.oc_nitems + 256;
+        L.oc_rows = up(a);   a = L.oc_rows + (size_t)L.cmax_rows * row_doubles(g.prec, W) * sizeof(double);
     }
     L.bytes = a + 256;
     return L;
@@ -351,7 +349,7 @@ static cudaError_t enqueue_group(const Group& g, const Layout& L, unsigned char*
         csl.nitems = (int*)(d + L.oc_nitems);
         csl.rows = (double*)(d + L.oc_rows);
         csl.max_rows = L.cmax_rows;
-        csl.lines_per_slice = L.clines_per_slice;
+        csl.cut_shift = L.ccut_shift;
     }
     return launch_tiles(g.pk, g.prec, (const gexs_job*)d, (const int*)(d + L.op),
                         (int)g.jobs.size(), g.nitems, (int*)(d + L.oc), d_err,

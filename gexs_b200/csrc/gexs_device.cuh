@@ -344,7 +344,9 @@ __device__ __forceinline__ float erf_bin_f32(float xm, float xp, int form)
     if (form == GEXS_ERF_LITERAL || xm < 0.f) return erff(xp) - erff(xm);
     return erfcf(xm) - erfcf(xp);
 }
-__device__ __forceinline__ double erf_bin_f64(double xm, double xp, int form)
+/* a call: four inlined functions at two places would not fit the
+ * instruction cache */
+static __device__ __noinline__ double erf_bin_f64(double xm, double xp, int form)
 {
     if (form == GEXS_ERF_LITERAL || xm < 0.0) return dsub(erf(xp), erf(xm));
     return dsub(erfc(xm), erfc(xp));

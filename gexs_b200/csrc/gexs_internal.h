@@ -11,15 +11,14 @@ namespace gexs {
 int profile_class(const gexs_job& j);
 int tile_bins(const gexs_launch_cfg& c);
 /* Line slices of the tile kernels (the FP32 Voigt region-I kernel and
- * tile_kernel; the FP32 Voigt core kernel has its own, below): a tile
- * whose line range
- * holds more than `lines_per_slice` lines (16384 unless the partial rows
- * would pass 1 GiB) is cut into ceil(n / lines_per_slice) work items (the
- * count depends on the tile alone, so the same tile is cut the same way
- * in every launch).  A split tile's slices write
+ * tile_kernel; the core kernel has its own, below): a tile whose line range
+ * holds more than `lines_per_slice` lines is cut into
+ * ceil(n / lines_per_slice) work items.  FP32 sums depend on the cut, which
+ * therefore depends on the tile alone (unless the partial rows would pass
+ * 1 GiB); FP64 sums do not (SUM_BLOCK).  A split tile's slices write
  * partial rows; the last one to finish sums them in slice order into the
  * output.  All arrays live in the launch table; slice_plan_kernel fills
- * them (and zeroes the tickets) before the region-I kernel runs. */
+ * them (and zeroes the tickets) before the kernel runs. */
 struct SliceTables {
     int*       prefix;      /* ntiles + 1: first item of each tile       */
     int*       counts;      /* ntiles: slices per tile                   */
@@ -30,6 +29,7 @@ struct SliceTables {
     double*    rows;        /* max_rows x tile bins: partial rows        */
     int        max_rows;
     long long  lines_per_slice;
+    int        cut_shift;   /* core kernel: see core_cut                    */
 };
 
 /* d_prep: device array of per-job prep arrays (S | invw | y, 3 N doubles
@@ -45,19 +45,35 @@ cudaError_t launch_tiles(int pk, int prec, const gexs_job* d_jobs, const int* d_
                          double* const* d_prep, const gexs_launch_cfg& cfg, int nsm,
                          cudaStream_t st, const SliceTables* sl = nullptr,
                          const SliceTables* csl = nullptr, const int* d_order = nullptr);
-/* which groups are sliced (all); lines_per_slice for a group (grows only
- * when the partial rows of its split tiles could pass 1 GiB) and the bound
- * on those rows */
+/* The FP64 tile kernel sums a bin's lines in order within blocks of this
+ * many lines of the list (by index, so that a tile of any shape or cut has
+ * the same block sums) and the blocks' sums as (hi, lo) pairs, whose
+ * rounded total does not depend on their order: a result is the same for
+ * every tile shape, slice length and batch.  Sub-lists of one list start
+ * at multiples of it. */
+constexpr int SUM_BLOCK = 512;
+
+/* doubles of a partial row: a value per bin, (hi, lo) in the FP64 forms */
+inline int row_doubles(int prec, int tile_w) { return prec == GEXS_FP64 ? 2 * tile_w : tile_w; }
+
+/* which groups are sliced; lines_per_slice for a group and the bound on the
+ * rows of its split tiles */
 bool slices_apply(int pk, int prec);
 long long slice_lines(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows);
-/* the Voigt core kernel's own slices (its line range per tile is the
- * lines whose core can reach the tile): only when a tile is one core
- * sub-tile (tile_w <= 1024); 2048 lines per slice unless the rows, bounded
- * by the core reach 15 nu dop_coef instead of the cutoff, would pass 1 GiB;
- * a partial row's doubles (the FP64 form keeps (hi, lo) sums) */
+
+/* the core kernel's own slices (its line range per tile is reach_range's):
+ * only when a tile is one core sub-tile (tile_w <= 1024).  Lines per slice
+ * by the tiles of the job's whole grid, so that a sub-range of it and a
+ * batch are cut alike: a job of few tiles has only its lines to fill the
+ * chip with.  The shift grows when the rows would pass 1 GiB. */
+__host__ __device__ inline long long core_cut(long long grid_points, int tile_w, int shift)
+{
+    const long long tiles = (grid_points + tile_w - 1) / tile_w;
+    if (shift >= 40) return 1ll << 62;
+    return (tiles < 148 ? 256ll : tiles < 296 ? 512ll : 2048ll) << shift;
+}
 bool core_slices_apply(int pk, int prec, int tile_w);
-long long core_slice_lines(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows);
-int core_row_doubles(int prec, int tile_w);
+int core_cut_shift(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows);
 cudaError_t launch_prep(const gexs_job* d_jobs, double* const* d_prep, int njobs,
                         int64_t max_lines, int nsm, cudaStream_t st);
 cudaError_t launch_count(const gexs_job* d_jobs, int njobs, unsigned long long* d_counts,

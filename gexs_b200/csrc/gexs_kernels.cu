@@ -191,9 +191,7 @@ __global__ void slice_plan_kernel(const KArgs a)
     }
 }
 
-/* the same for the FP32 Voigt core kernel: its line range per tile is the
- * core kernel's own search (lines whose core, |f - nu| < 15 nu dop_coef,
- * can reach the tile), computed with the same expressions */
+/* the same for the core kernel, with its own search (reach_range) */
 __global__ void core_slice_plan_kernel(const KArgs a)
 {
     const int lane = threadIdx.x & 31;
@@ -208,17 +206,13 @@ __global__ void core_slice_plan_kernel(const KArgs a)
     const double f0 = grid_f(J.nu_start, J.dnu, t0);
     const double fl = grid_f(J.nu_start, J.dnu, t0 + jn - 1);
     const int64_t nl = J.lines.count;
-    const double margin = 2.0 * J.dnu + 1e-9 * (fabs(fl) + J.cutoff);
-    const double k15 = 15.0 * J.dop_coef;
-    double vlo = f0 - J.cutoff, vhi = fl + J.cutoff;
-    vlo = fmax(vlo, f0 / (1.0 + k15));
-    if (k15 < 1.0) vhi = fmin(vhi, fl / (1.0 - k15));
-    vlo -= margin; vhi += margin;
-    if (vlo < 1e-6 + margin) vlo = -1.0;
+    double vlo, vhi;
+    reach_range(J, f0, fl, vlo, vhi);
     const int64_t lo = warp_bound<false>(J.lines.nu, nl, vlo, lane);
     const int64_t hi = max(warp_bound<true>(J.lines.nu, nl, vhi, lane), lo);
     if (lane == 0) {
-        const long long n = hi - lo, per = a.csl.lines_per_slice;
+        const long long n = hi - lo;
+        const long long per = core_cut(J.grid_points, a.tile_w, a.csl.cut_shift);
         a.csl.lohi[2 * ti] = lo;
         a.csl.lohi[2 * ti + 1] = hi;
         a.csl.counts[ti] = n > per ? (int)((n + per - 1) / per) : 1;
@@ -287,84 +281,81 @@ cudaError_t launch_core_slice_plan(const KArgs& a, cudaStream_t st)
     return cudaGetLastError();
 }
 
-bool slices_apply(int, int) { return true; }
+bool slices_apply(int pk, int prec) { return !(pk == PK_ERF && prec == GEXS_FP64); }
 
 bool core_slices_apply(int pk, int prec, int tile_w)
 {
-    (void)prec;
-    return pk == PK_VOIGT && tile_w <= CORE_W;
+    return (pk == PK_VOIGT || (pk == PK_ERF && prec == GEXS_FP64)) && tile_w <= CORE_W;
 }
 
-/* A split tile of n lines has ceil(n / per) <= n / per + 1 slices, so for M
- * line entries in all tiles the slices of split tiles number at most
- * M / per + (split tiles), and a split tile holds more than per entries. */
-static double row_bound(double m, double tiles, double per)
+/* A split tile of n lines has ceil(n / per) <= n / per + 1 slices, so for m
+ * line entries in all of a job's tiles the slices of split tiles number at
+ * most m / per + (split tiles), and a split tile holds more than per. */
+static double row_bound(const gexs_job& j, double m, int tile_w, double per)
 {
+    const double tiles = std::ceil((double)j.n_points / (double)tile_w);
     return std::ceil(m / per) + std::min(tiles, std::floor(m / per));
 }
 
-static double tiles_of(const gexs_job& j, int tile_w)
+/* a line lies in at most (2 (reach + margin)) / (tile width) + 2 tiles */
+static double tile_entries(const gexs_job& j, double reach, int tile_w)
 {
-    return std::ceil((double)j.n_points / (double)tile_w);
+    const double tpl = std::floor((2.0 * reach + 8.0 * j.dnu) / ((double)tile_w * j.dnu)) + 3.0;
+    return (double)j.lines.count * tpl;
 }
 
-int core_row_doubles(int prec, int tile_w) { return prec == GEXS_FP64 ? 2 * tile_w : tile_w; }
+static const double kMaxRowBytes = (double)(1ull << 30);
 
-long long core_slice_lines(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows)
+int core_cut_shift(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows)
 {
-    /* as slice_lines, with a line's reach the core's: at most 15 nu
-     * dop_coef / (1 - 15 dop_coef) at the job's highest frequency, and at
-     * most the cutoff.  2048 lines per slice: a launch of few tiles fills
-     * more of the chip than at 8192 (12 tiles of 256 lines each: 21 against
-     * 33 us) and large launches end more evenly. */
-    long long per = 2048;
-    for (;;) {
+    /* a line's reach is reach_range's at the job's highest frequency */
+    for (int shift = 0; shift < 40; ++shift) {
         double rows = 0.0;
         for (int i = 0; i < njobs; ++i) {
             const gexs_job& j = jobs[i];
-            const double k15 = 15.0 * j.dop_coef;
+            const double z = j.profile == GEXS_VOIGT ? 15.0 : ERF_Z64, k = z * j.dop_coef;
             const double nu_hi = j.nu_start + (double)(j.start_idx + j.n_points) * j.dnu + j.cutoff;
             double reach = j.cutoff;
-            if (k15 < 1.0) reach = std::min(reach, nu_hi * k15 / (1.0 - k15));
-            const double tpl = std::floor((2.0 * reach + 8.0 * j.dnu) / ((double)tile_w * j.dnu)) + 3.0;
-            rows += row_bound((double)j.lines.count * tpl, tiles_of(j, tile_w), (double)per);
+            if (j.profile == GEXS_GAUSSIAN) reach = std::min(reach, z / j.inv_width);
+            else if (k < 1.0) reach = std::min(reach, (nu_hi + j.dnu) * k / (1.0 - k));
+            rows += row_bound(j, tile_entries(j, reach, tile_w), tile_w,
+                              (double)core_cut(j.grid_points, tile_w, shift));
         }
-        if (rows * core_row_doubles(prec, tile_w) * sizeof(double) <= (double)(1ull << 30)) {
+        if (rows * row_doubles(prec, tile_w) * sizeof(double) <= kMaxRowBytes) {
             *max_rows = (int)rows;
-            return per;
+            return shift;
         }
-        if (per >= (1ll << 40)) { *max_rows = 0; return 1ll << 62; }
-        per *= 2;
     }
+    *max_rows = 0;
+    return 40;
 }
 
 long long slice_lines(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows)
 {
-    /* A line lies in at most (2 (cutoff + margin)) / (tile width) + 2 tiles,
-     * so the tiles hold at most sum(lines x that) = M line entries.  A split
-     * tile (n > per lines) has ceil(n / per) < 2 n / per slices, so the
-     * slices of split tiles, which alone need partial rows, are fewer than
-     * 2 M / per.  per doubles until those rows fit in 1 GiB; past 2^40 no
-     * tile can be split at all.  The rows reserved are row_bound's, which
-     * is smaller.  16384 lines per slice: measured on one
-     * B200, the 1e8-line workload is indifferent to it (16k-128k) and a
-     * dense band of 1e6 lines in 80 cm^-1 runs 25% faster than at 65536. */
-    long long per = prec == GEXS_FP32 ? 16384 : 2048;
-    for (;;) {
+    /* FP32: slices of 16384 lines, more when the rows of split tiles, fewer
+     * than 2 m / per, could pass 1 GiB.  Measured on one B200: the 1e8-line
+     * workload is indifferent to 16k-128k, a dense band of 1e6 lines in 80
+     * cm^-1 runs 25% faster than at 65536.
+     * FP64 (any cut gives the same sums): about eight items for each of the
+     * 888 CTAs that fit, of 512 to 4096 lines.  2e5 lines on 194 tiles
+     * (GH32): 8.2 ms against 34 ms uncut. */
+    double m = 0.0;
+    for (int i = 0; i < njobs; ++i) m += tile_entries(jobs[i], jobs[i].cutoff, tile_w);
+    long long per = 16384;
+    if (prec == GEXS_FP64)
+        for (per = 512; per < 4096 && (double)per * (8 * 888) < m; ) per *= 2;
+    for (;; per *= 2) {
         double rows = 0.0, need = 0.0;
         for (int i = 0; i < njobs; ++i) {
-            const gexs_job& j = jobs[i];
-            const double tpl = std::floor((2.0 * j.cutoff + 8.0 * j.dnu) / ((double)tile_w * j.dnu)) + 3.0;
-            const double m = (double)j.lines.count * tpl;
-            rows += 2.0 * std::ceil(m / (double)per);
-            need += row_bound(m, tiles_of(j, tile_w), (double)per);
+            const double mi = tile_entries(jobs[i], jobs[i].cutoff, tile_w);
+            rows += 2.0 * std::ceil(mi / (double)per);
+            need += row_bound(jobs[i], mi, tile_w, (double)per);
         }
-        if (rows * tile_w * sizeof(double) <= (double)(1ull << 30)) {
+        if ((prec == GEXS_FP64 ? need : rows) * row_doubles(prec, tile_w) * sizeof(double) <= kMaxRowBytes) {
             *max_rows = (int)std::min(rows, need);
             return per;
         }
         if (per >= (1ll << 40)) { *max_rows = 0; return 1ll << 62; }
-        per *= 2;
     }
 }
 

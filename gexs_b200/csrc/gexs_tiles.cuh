@@ -65,11 +65,11 @@ struct __align__(16) RecF32 {   /* 48 bytes; Doppler/Gaussian and GH */
  * part of mfcdx (their high parts are dx and mfcdx), see make_rec */
 constexpr int GH_PAIR_BIT = 1 << 25;
 
-struct __align__(16) RecF64 {   /* 64 bytes */
+struct __align__(16) RecF64 {   /* 64 bytes; GH */
     double nu;             /* centre after the nu==0 rule                   */
     double invw;
-    double y;              /* GH: y ; Doppler: unused                       */
-    double amp;            /* GH: S*invw ; Doppler: S                       */
+    double y;
+    double amp;            /* S*invw                                        */
     int    win, c1, c2, c3;
     int    mask, pad0, pad1, pad2;
 };
@@ -169,6 +169,32 @@ struct Tile {
                             guesses and FP32 offsets; every window and
                             region decision uses exact predicates)   */
 };
+
+/* the lines a scattered part of a profile can reach bins [f0, fl] from, as
+ * the interval [vlo, vhi] of centres: the Voigt core reaches |f - nu| < 15 /
+ * invw, the erf profiles' non-zero bins zthr / invw + dnu / 2, both within
+ * the cutoff; 1 / invw = nu dop_coef, or a constant for GAUSSIAN.  The
+ * margin (2 bins and rounding) covers dnu / 2. */
+constexpr double ERF_Z32 = 10.5, ERF_Z64 = 27.5;   /* erfc underflows to zero beyond */
+__device__ __forceinline__ void reach_range(const gexs_job& J, double f0, double fl,
+                                            double& vlo, double& vhi)
+{
+    const double margin = 2.0 * J.dnu + 1e-9 * (fabs(fl) + J.cutoff);
+    const double z = J.profile == GEXS_VOIGT ? 15.0 : J.precision == GEXS_FP32 ? ERF_Z32 : ERF_Z64;
+    vlo = f0 - J.cutoff; vhi = fl + J.cutoff;
+    if (J.profile == GEXS_GAUSSIAN) {
+        const double w = z / J.inv_width;
+        vlo = fmax(vlo, f0 - w); vhi = fmin(vhi, fl + w);
+    } else {
+        /* with h = dnu / 2 (inside the margin) taken before the division:
+         * nu > (f0 - h) / (1 + k), nu < (fl + h) / (1 - k) */
+        const double k = z * J.dop_coef, h = 0.5 * J.dnu;
+        vlo = fmax(vlo, (f0 - h) / (1.0 + k));
+        if (k < 1.0) vhi = fmin(vhi, (fl + h) / (1.0 - k));
+    }
+    vlo -= margin; vhi += margin;
+    if (vlo < 1e-6 + margin) vlo = -1.0;       /* nu == 0 lines count as 1e-6 */
+}
 
 /* window of a line inside the tile as [a, b) (tile-relative) */
 __device__ __forceinline__ void tile_window(const Tile& T, double nu, double tc,
@@ -383,6 +409,15 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float v)
     s = t;
 }
 
+/* (hi, lo) += v with the rounding error kept (Knuth's TwoSum): sums of the
+ * same terms in another order round to the same double */
+__device__ __forceinline__ void dd_add(double& hi, double& lo, double v)
+{
+    const double s = dadd(hi, v), bb = dsub(s, hi);
+    lo = dadd(lo, dadd(dsub(hi, dsub(s, bb)), dsub(v, bb)));
+    hi = s;
+}
+
 /* per-warp tiers of a line (bits of RecF*.mask).  Warp w owns bins
  * [32*B*w, 32*B*(w+1)) of the tile. */
 template <int PK, int B, int WARPS>
@@ -506,7 +541,7 @@ __device__ __forceinline__ void make_rec(RecF64& q, const Derived<PK>& d, const 
                                          const Tile&)
 {
     q.nu = d.nu; q.invw = d.invw; q.y = d.y;
-    q.amp = (PK == PK_ERF) ? d.S : dmul(d.S, d.invw);
+    q.amp = dmul(d.S, d.invw);
     q.win = d.win; q.c1 = d.c1; q.c2 = d.c2; q.c3 = d.c3;
     q.mask = (d.win == 0) ? 0 : warp_mask<PK, B, WARPS>(d, 1);
     q.pad0 = q.pad1 = q.pad2 = 0;
@@ -553,28 +588,41 @@ __device__ __forceinline__ void lines_f32(const RecF32* __restrict__ rec, int nr
     const int wb = warp * 32 * B;
     const float wbf = (float)wb, lanef = (float)lane;
     const int bit = 1 << warp;
-    for (int i = 0; i < nrec; ++i) {
-        const int4 qi = *reinterpret_cast<const int4*>(&rec[i].win);   /* win c1 mask pad */
-        const int mask = qi.z;
-        if (!(mask & bit)) continue;
-        const float4 q0 = *reinterpret_cast<const float4*>(&rec[i].icf);   /* icf dx mfcdx a1 */
-        const float4 q1 = *reinterpret_cast<const float4*>(&rec[i].p);     /* p y amp fc */
-        const float ncf = wbf - q0.x;
-        if constexpr (PK == PK_ERF) {
-            const int a = lo16(qi.x), b = hi16(qi.x);
-            const int c1a = lo16(qi.y), c1b = hi16(qi.y);
-            const float t0 = lanef + ncf;
+    if constexpr (PK == PK_ERF) {
+        /* a line touches few warps of its tile: the records that touch this
+         * one, 32 at a time, in order */
+        for (int i0 = 0; i0 < nrec; i0 += 32) {
+            unsigned todo = __ballot_sync(0xffffffffu,
+                                          i0 + lane < nrec && (rec[min(i0 + lane, nrec - 1)].mask & bit));
+            while (todo) {
+                const int i = i0 + __ffs(todo) - 1;
+                todo &= todo - 1;
+                const int4 qi = *reinterpret_cast<const int4*>(&rec[i].win);   /* win c1 mask pad */
+                const float4 q0 = *reinterpret_cast<const float4*>(&rec[i].icf);   /* icf dx mfcdx a1 */
+                const float4 q1 = *reinterpret_cast<const float4*>(&rec[i].p);     /* p y amp fc */
+                const int a = lo16(qi.x), b = hi16(qi.x);
+                const int c1a = lo16(qi.y), c1b = hi16(qi.y);
+                const float t0 = lanef + (wbf - q0.x);
 #pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const int t = wb + lane + 32 * k;
-                if (t < a || t >= b || t < c1a || t >= c1b) continue;
-                const float xd = fabsf(((t0 + (float)(32 * k)) - q1.w) * q0.y);
-                /* FP32 always takes the cancellation-free form: the literal
-                 * erf difference loses ~1e-7 absolute in FP32 far wings */
-                float& acc = bin_acc<B>(part, k);
-                acc = fmaf(q1.z, erf_bin_f32(xd - q1.y, xd + q1.y, GEXS_ERF_STABLE), acc);
+                for (int k = 0; k < B; ++k) {
+                    const int t = wb + lane + 32 * k;
+                    if (t < a || t >= b || t < c1a || t >= c1b) continue;
+                    const float xd = fabsf(((t0 + (float)(32 * k)) - q1.w) * q0.y);
+                    /* FP32 always takes the cancellation-free form: the literal
+                     * erf difference loses ~1e-7 absolute in FP32 far wings */
+                    float& acc = bin_acc<B>(part, k);
+                    acc = fmaf(q1.z, erf_bin_f32(xd - q1.y, xd + q1.y, GEXS_ERF_STABLE), acc);
+                }
             }
-        } else {
+        }
+    } else {
+        for (int i = 0; i < nrec; ++i) {
+            const int4 qi = *reinterpret_cast<const int4*>(&rec[i].win);   /* win c1 mask pad */
+            const int mask = qi.z;
+            if (!(mask & bit)) continue;
+            const float4 q0 = *reinterpret_cast<const float4*>(&rec[i].icf);   /* icf dx mfcdx a1 */
+            const float4 q1 = *reinterpret_cast<const float4*>(&rec[i].p);     /* p y amp fc */
+            const float ncf = wbf - q0.x;
             constexpr int NODES = (PK == PK_GH16) ? 16 : 32;
             if (mask & GH_PAIR_BIT) {
                 /* narrow line: x as a float pair, per-bin window test */
@@ -875,7 +923,7 @@ __device__ __forceinline__ void lines_voigt_f32(const RecV* __restrict__ rec, in
     }
 }
 
-/* FP64 form of the Doppler/Gaussian and Gauss-Hermite profiles: per-bin
+/* FP64 form of the Gauss-Hermite profiles: per-bin
  * window tests, FP64 arithmetic, bins sum their lines in line order (the
  * order of the FP64 oracle). */
 template <int PK, int B>
@@ -890,21 +938,7 @@ __device__ __forceinline__ void lines_f64(const RecF64* __restrict__ rec, int nr
         const RecF64& q = rec[i];
         if (!(q.mask & bit)) continue;
         const int a = lo16(q.win), b = hi16(q.win);
-        if constexpr (PK == PK_ERF) {
-            const int c1a = lo16(q.c1), c1b = hi16(q.c1);
-            const int form = J.erf_form;
-            const double h = 0.5 * J.dnu;
-#pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const int t = wb + lane + 32 * k;
-                if (t < a || t >= b || t < c1a || t >= c1b) continue;
-                double dist = fabs(dsub(fbin[k], q.nu));
-                double xp = dmul(q.invw, dadd(dist, h));
-                double xm = dmul(q.invw, dsub(dist, h));
-                double de = erf_bin_f64(xm, xp, form);
-                acc[k] = dadd(acc[k], dmul(dmul(q.amp, de), out_scale));
-            }
-        } else {
+        {
             constexpr int NODES = (PK == PK_GH16) ? 16 : 32;
             const double y2 = dmul(q.y, q.y), yk = dmul(q.y, GEXS_INV_PI);
 #pragma unroll
@@ -996,9 +1030,10 @@ struct Smem {
     static constexpr size_t off_gn = NF64 * raw_d;
     static constexpr size_t off_rec = (off_gn + (PREP ? 0 : (size_t)2 * NT * sizeof(int)) + 15) & ~size_t(15);
     static constexpr size_t rec_sz = sizeof(typename RecOf<PK, PREC>::T);
-    /* FP32: Kahan (sum, compensation) per bin; each lane owns its bins */
+    /* FP32: Kahan (sum, compensation) per bin; FP64: (hi, lo) sum of the
+     * line blocks; each lane owns its bins */
     static constexpr size_t off_kahan = (off_rec + (size_t)R * rec_sz + 15) & ~size_t(15);
-    static constexpr size_t bytes = off_kahan + (PREC == GEXS_FP32 ? (size_t)2 * W * sizeof(float) : 0);
+    static constexpr size_t bytes = off_kahan + (size_t)2 * W * (PREC == GEXS_FP32 ? sizeof(float) : sizeof(double));
 };
 
 /* ---------------------------------------------------------------- kernel */
@@ -1028,11 +1063,13 @@ tile_kernel(const KArgs args)
     Rec*    s_rec = reinterpret_cast<Rec*>(smem + L::off_rec);
     float*  s_ks = reinterpret_cast<float*>(smem + L::off_kahan);
     float*  s_kc = s_ks + W;
+    double* s_hi = reinterpret_cast<double*>(smem + L::off_kahan);
+    double* s_lo = s_hi + W;
     __shared__ int s_item;
-    __shared__ long long s_lohi[2];
+    __shared__ long long s_lohi[2], s_near[2];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const double zthr = (PREC == GEXS_FP32) ? 10.5 : 27.5;
+    const double zthr = ERF_Z32;              /* the erf profiles are FP32 here */
 
     const bool sliced = args.sl.prefix != nullptr;
     const int nitems = sliced ? *(volatile const int*)args.sl.nitems : args.nitems;
@@ -1071,9 +1108,15 @@ tile_kernel(const KArgs args)
             if (tid == 0) {
                 const long long tlo = __ldg(args.sl.lohi + 2 * ti), thi = __ldg(args.sl.lohi + 2 * ti + 1);
                 const long long per = (thi - tlo + ns - 1) / ns;
-                const long long a0 = tlo + (long long)sidx * per;
+                long long a0 = tlo + (long long)sidx * per, a1 = a0 + per;
+                if (PREC == GEXS_FP64) {
+                    /* inner cuts at the next line block */
+                    if (sidx > 0) a0 = (a0 + SUM_BLOCK - 1) & ~(long long)(SUM_BLOCK - 1);
+                    a1 = (a1 + SUM_BLOCK - 1) & ~(long long)(SUM_BLOCK - 1);
+                    if (sidx == ns - 1) a1 = thi;
+                }
                 s_lohi[0] = min(a0, thi);
-                s_lohi[1] = min(a0 + per, thi);
+                s_lohi[1] = min(a1, thi);
             }
         } else if (warp == 0) {
             int64_t v = warp_bound<false>(J.lines.nu, nl, T.f0 - J.cutoff - margin, lane);
@@ -1082,15 +1125,51 @@ tile_kernel(const KArgs args)
             int64_t v = warp_bound<true>(J.lines.nu, nl, T.fl + J.cutoff + margin, lane);
             if (lane == 0) s_lohi[1] = v;
         }
+        if constexpr (PK == PK_ERF) {
+            if (warp >= 2 && warp < 4) {
+                double vlo, vhi;
+                reach_range(J, T.f0, T.fl, vlo, vhi);
+                const int64_t v = warp == 2 ? warp_bound<false>(J.lines.nu, nl, vlo, lane)
+                                            : warp_bound<true>(J.lines.nu, nl, vhi, lane);
+                if (lane == 0) s_near[warp - 2] = v;
+            }
+        }
         __syncthreads();
         const int64_t lo = s_lohi[0];
         const int64_t hi = max((int64_t)s_lohi[1], lo);
         const int nph = (int)((hi - lo + R - 1) / R);
+        /* phases to run: all, or for the erf profiles those that hold a line
+         * whose non-zero bins can reach the tile (of the lines within the
+         * cutoff about a tenth at 0.01 cm^-1 and 1500 K).  Phases stay those
+         * of the whole range: a skipped one would add zeros, so the FP32
+         * sums are the same bits. */
+        int ph0 = 0, ph1 = nph;
+        if constexpr (PK == PK_ERF) {
+            const int64_t nlo = min(max((int64_t)s_near[0], lo), hi);
+            const int64_t nhi = min(max((int64_t)s_near[1], nlo), hi);
+            ph0 = (int)((nlo - lo) / R);
+            ph1 = nhi > nlo ? (int)((nhi - lo + R - 1) / R) : ph0;
+        }
         if constexpr (PREC == GEXS_FP32) {
             /* Kahan pairs: touched only by the lane that owns the bin */
             for (int z = tid; z < W; z += NT) { s_ks[z] = 0.f; s_kc[z] = 0.f; }
             __syncthreads();
+        } else {
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const int t = warp * 32 * B + lane + 32 * k;
+                s_hi[t] = 0.0; s_lo[t] = 0.0;
+            }
         }
+        /* the end of a line block: its sums into the (hi, lo) pairs */
+        auto end_block = [&](double (&acc)[B]) {
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const int t = warp * 32 * B + lane + 32 * k;
+                dd_add(s_hi[t], s_lo[t], acc[k]);
+                acc[k] = 0.0;
+            }
+        };
 
         float2 part[B / 2];
         double acc[B], fbin[B];
@@ -1105,7 +1184,7 @@ tile_kernel(const KArgs args)
         /* thread tid stages and derives lines lo + u*NT + tid, u = 0, 1, ...;
          * every thread only ever reads the staging slots it filled itself,
          * so the double-buffered cp.async pipeline needs no barrier */
-        const int nsub = nph * PH;
+        const int nsub = ph1 * PH;
         const double* pb = nullptr;
         if constexpr (PREP) pb = args.prep[jl];
         auto issue = [&](int u) {
@@ -1129,10 +1208,10 @@ tile_kernel(const KArgs args)
             }
             cp_async_commit();
         };
-        issue(0);
-        issue(1);
+        issue(ph0 * PH);
+        issue(ph0 * PH + 1);
 
-        for (int ph = 0; ph < nph; ++ph) {
+        for (int ph = ph0; ph < ph1; ++ph) {
             const int64_t pbase = lo + (int64_t)ph * R;
             const int nrec = (int)min((int64_t)R, hi - pbase);
 #pragma unroll
@@ -1181,26 +1260,35 @@ tile_kernel(const KArgs args)
                     for (int j = 0; j < B / 2; ++j) part[j] = make_float2(0.f, 0.f);
                 }
             } else {
-                if constexpr (PK == PK_VOIGT)
-                    lines_voigt_f64<B>(reinterpret_cast<const RecV64*>(s_rec), nrec, warp, lane,
-                                       fbin, acc);
-                else
-                    lines_f64<PK, B>(reinterpret_cast<const RecF64*>(s_rec), nrec, warp, lane, fbin,
-                                     acc, J);
+                for (int c0 = 0; c0 < nrec;) {
+                    const int left = SUM_BLOCK - (int)((pbase + c0) & (SUM_BLOCK - 1));
+                    const int cn = min(left, nrec - c0);
+                    if constexpr (PK == PK_VOIGT)
+                        lines_voigt_f64<B>(reinterpret_cast<const RecV64*>(s_rec) + c0, cn, warp, lane,
+                                           fbin, acc);
+                    else
+                        lines_f64<PK, B>(reinterpret_cast<const RecF64*>(s_rec) + c0, cn, warp, lane,
+                                         fbin, acc, J);
+                    if (cn == left) end_block(acc);
+                    c0 += cn;
+                }
             }
             __syncthreads();
         }
         cp_async_wait<0>();
 
         /* ------------------------------------------------------- write out */
+        constexpr bool DD = PREC == GEXS_FP64;
+        if constexpr (DD) end_block(acc);
         double* out = J.out;
         const int acc_mode = J.accumulate;
+        auto hi_of = [&](int t) { return DD ? s_hi[t] : (double)s_ks[t] - (double)s_kc[t]; };
         if (ns == 1) {
 #pragma unroll
             for (int k = 0; k < B; ++k) {
                 const int t = warp * 32 * B + lane + 32 * k;
                 if (t < T.jn) {
-                    const double v = (PREC == GEXS_FP32) ? ((double)s_ks[t] - (double)s_kc[t]) : acc[k];
+                    const double v = DD ? s_hi[t] + s_lo[t] : hi_of(t);
                     int64_t j = T.j0 + t;
                     out[j] = acc_mode ? out[j] + v : v;
                 }
@@ -1208,13 +1296,16 @@ tile_kernel(const KArgs args)
         } else {
             /* one slice of a split tile: its partial row, then a ticket; the
              * last slice to finish adds the rows in slice order */
-            const int base = args.sl.prefix[ti];
+            constexpr int RS = DD ? 2 * W : W;
             const int rb = args.sl.rowbase[ti];
-            double* row = args.sl.rows + (size_t)(rb + sidx) * W;
+            double* row = args.sl.rows + (size_t)(rb + sidx) * RS;
 #pragma unroll
             for (int k = 0; k < B; ++k) {
                 const int t = warp * 32 * B + lane + 32 * k;
-                if (t < T.jn) row[t] = (PREC == GEXS_FP32) ? ((double)s_ks[t] - (double)s_kc[t]) : acc[k];
+                if (t < T.jn) {
+                    row[t] = hi_of(t);
+                    if (DD) row[W + t] = s_lo[t];
+                }
             }
             __threadfence();
             __syncthreads();
@@ -1226,14 +1317,18 @@ tile_kernel(const KArgs args)
                 for (int k = 0; k < B; ++k) {
                     const int t = warp * 32 * B + lane + 32 * k;
                     if (t < T.jn) {
-                        double v = 0.0;
-                        for (int q = 0; q < ns; ++q) v += __ldcg(args.sl.rows + (size_t)(rb + q) * W + t);
+                        double hi = 0.0, lo = 0.0;
+                        for (int q = 0; q < ns; ++q) {
+                            const double* r = args.sl.rows + (size_t)(rb + q) * RS + t;
+                            if (DD) { dd_add(hi, lo, __ldcg(r)); lo = dadd(lo, __ldcg(r + W)); }
+                            else hi += __ldcg(r);
+                        }
+                        const double v = DD ? hi + lo : hi;
                         int64_t j = T.j0 + t;
                         out[j] = acc_mode ? out[j] + v : v;
                     }
                 }
             }
-            (void)base;
         }
         __syncthreads();
     }
@@ -1416,7 +1511,7 @@ voigt_ws_kernel(const KArgs args)
             const int64_t nl = J.lines.count;
             const double margin = 2.0 * J.dnu + 1e-9 * (fabs(T.fl) + J.cutoff);
             if (sliced) {
-                /* the tile's range from slice_plan_kernel, cut into ns equal parts */
+                /* the item's lines: the tile's range from slice_plan_kernel, cut */
                 if (ptid == 0) {
                     const long long tlo = __ldg(args.sl.lohi + 2 * ti), thi = __ldg(args.sl.lohi + 2 * ti + 1);
                     const long long per = (thi - tlo + ns - 1) / ns;
@@ -1691,7 +1786,13 @@ voigt_ws_kernel(const KArgs args)
     }
 }
 
-/* ------------------------------------------------------ Voigt core kernel
+/* ---------------------------------- Voigt core kernel, FP64 erf profiles
+ * (below "core": for the FP64 Doppler/Gaussian form the bins of a line that
+ * are not exactly zero, its whole profile; their launch has no tile kernel.
+ * A line reaches ~11 bins of a 0.1 cm^-1 grid at 1500 K, so tiles of bins
+ * that scan all lines within the cutoff idled through most records and
+ * lanes: 11.0 against 0.3 ms for 1e6 lines on 99,001 bins.)
+ *
  * The core of a line (its bins outside Humlicek region I: regions II, III,
  * IV) is evaluated here, after the region-I kernel, and added into the
  * output.  Kept out of that kernel so it carries no FP64 Humlicek code and
@@ -1747,26 +1848,78 @@ __device__ __forceinline__ void core_ranges(int c1, int c2, int c3, int& c1a, in
  * strip (sparse lines) takes that form. */
 constexpr int SCR_D = 544;               /* doubles of a warp's strips */
 
-/* (hi, lo) += v with the rounding error kept (Knuth's TwoSum): sums of the
- * same terms in another order round to the same double */
-__device__ __forceinline__ void dd_add(double& hi, double& lo, double v)
+/* what a lane's terms need of its line */
+struct CoreLine {
+    double nu, invw, y, amp;
+    float icf, fc, dx, yf, ampf;      /* FP32 form */
+};
+template <int PREC>
+__device__ __forceinline__ CoreLine core_line_of(const CoreLine& c, int src)
 {
-    const double s = dadd(hi, v), bb = dsub(s, hi);
-    lo = dadd(lo, dadd(dsub(hi, dsub(s, bb)), dsub(v, bb)));
-    hi = s;
+    constexpr unsigned ALL = 0xffffffffu;
+    CoreLine r;
+    r.nu = __shfl_sync(ALL, c.nu, src); r.invw = __shfl_sync(ALL, c.invw, src);
+    r.y = __shfl_sync(ALL, c.y, src);   r.amp = __shfl_sync(ALL, c.amp, src);
+    if (PREC == GEXS_FP32) {
+        r.icf = __shfl_sync(ALL, c.icf, src); r.fc = __shfl_sync(ALL, c.fc, src);
+        r.dx = __shfl_sync(ALL, c.dx, src);   r.yf = __shfl_sync(ALL, c.yf, src);
+        r.ampf = __shfl_sync(ALL, c.ampf, src);
+    } else {
+        r.icf = r.fc = r.dx = r.yf = r.ampf = 0.f;
+    }
+    return r;
+}
+
+/* a core term out of line, for scatter_phase's sparse form: a second inline
+ * copy of every region cost the dense form 13% in instruction fetches */
+template <int PREC, int REGION>
+__device__ __noinline__ double core_term(double x, double y, double amp)
+{
+    if (REGION == 2) return amp * hum_region2<double>(x, y);
+    if (REGION == 3) return amp * (PREC == GEXS_FP64 ? hum_region3<double>(x, y) : hum_region3_core(x, y));
+    return amp * (PREC == GEXS_FP64 ? hum_region4<double>(x, y) : hum_region4_core(x, y));
+}
+__device__ __forceinline__ double core_term2_f32(const CoreLine& l, int t)
+{
+    const float x = fabsf(((float)t - l.icf) - l.fc) * l.dx;
+    return (double)__fmul_rn(l.ampf, hum_region2<float>(x, l.yf));
 }
 
 /* LO = 0: plain sums.  LO > 0 (the FP64 form): row[t] and row[LO + t] are a
  * (hi, lo) sum, because that form's results are the same for every tile
- * shape and the order of the terms here is not; no strips, the groups add
- * one after another. */
-template <bool DD, typename F>
-__device__ __forceinline__ void scatter_phase(int a, int b, int lane, double* row, int LO,
-                                              double* scr, const F& val)
+ * shape and cut (SUM_BLOCK) and the order of the terms here is not; no
+ * strips, the groups add one after another. */
+template <int PREC, typename F, typename C>
+__device__ __forceinline__ void scatter_phase(int a, int b, int lane, const CoreLine& line,
+                                              double* row, int LO, double* scr, const F& val,
+                                              const C& call)
 {
     constexpr unsigned ALL = 0xffffffffu;
+    constexpr bool DD = PREC == GEXS_FP64;
     const int longest = __reduce_max_sync(ALL, max(b - a, 0));
     if (longest == 0) return;
+    /* few lines with long ranges (sparse lists on fine grids): one line
+     * after another, a bin per lane; a step of this form costs about a third
+     * more (the line's values travel by shuffles, the term is a call).
+     * 564 lines on 2.7e5 bins: 20 against 66 us for the bin-by-bin form. */
+    const int steps = (int)__reduce_add_sync(ALL, (unsigned)(max(b - a, 0) + 31) / 32);
+    if (steps * 4 < longest * 3) {
+        unsigned todo = __ballot_sync(ALL, a < b);
+        while (todo) {
+            const int src = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int sa = __shfl_sync(ALL, a, src), sb = __shfl_sync(ALL, b, src);
+            const CoreLine l = core_line_of<PREC>(line, src);
+#pragma unroll 1
+            for (int t = sa + lane; t < sb; t += 32) {
+                const double v = call(l, t);
+                if (DD) dd_add(row[t], row[LO + t], v);
+                else row[t] += v;
+            }
+            __syncwarp();
+        }
+        return;
+    }
     const int passes = (longest + 31) / 32;
     const int M = max((longest + passes - 1) / passes, 4);
     const int groups = (31 + M) / M, mine = lane / M;
@@ -1788,7 +1941,7 @@ __device__ __forceinline__ void scatter_phase(int a, int b, int lane, double* ro
             if (++o == M) o = 0;
             const bool on = t < b;
             if (!__any_sync(ALL, on)) continue;
-            const double v = val(t);      /* dropped if t is outside */
+            const double v = val(line, t);      /* dropped if t is outside */
             if (DD) {
                 for (int g = 0; g < rounds; ++g) {
                     if (on && mine == g) dd_add(row[t], row[LO + t], v);
@@ -1815,7 +1968,7 @@ __device__ __forceinline__ void scatter_phase(int a, int b, int lane, double* ro
     }
 }
 
-template <int PREC, bool PREP, bool ORDER>
+template <int PK, int PREC, bool PREP, bool ORDER>
 __global__ void __launch_bounds__(CORE_WARPS * 32, 24 / CORE_WARPS)
 core_kernel(const KArgs args)
 {
@@ -1858,7 +2011,6 @@ core_kernel(const KArgs args)
         const int64_t tend = min((int64_t)(t0 + args.tile_w), J.start_idx + J.n_points);
         const int64_t nl = J.lines.count;
         const double* pb = PREP ? args.prep[jl] : nullptr;
-        const double k15 = 15.0 * J.dop_coef;
         for (int64_t s0 = t0; s0 < tend; s0 += CORE_W) {
             Tile T;
             T.J = Jp;
@@ -1867,13 +2019,8 @@ core_kernel(const KArgs args)
             T.f0 = grid_f(J.nu_start, J.dnu, T.j0);
             T.fl = grid_f(J.nu_start, J.dnu, T.j0 + T.jn - 1);
             T.inv_dnu = 1.0 / J.dnu;
-            const double margin = 2.0 * J.dnu + 1e-9 * (fabs(T.fl) + J.cutoff);
-            /* a core reaches f only if |f - nu| < 15 nu dop_coef */
-            double vlo = T.f0 - J.cutoff, vhi = T.fl + J.cutoff;
-            vlo = fmax(vlo, T.f0 / (1.0 + k15));
-            if (k15 < 1.0) vhi = fmin(vhi, T.fl / (1.0 - k15));
-            vlo -= margin; vhi += margin;
-            if (vlo < 1e-6 + margin) vlo = -1.0;   /* nu == 0 lines count as 1e-6 */
+            double vlo, vhi;
+            reach_range(J, T.f0, T.fl, vlo, vhi);
             if (sliced) {
                 /* the range from core_slice_plan_kernel, cut into ns parts */
                 if (tid == 0) {
@@ -1899,8 +2046,7 @@ core_kernel(const KArgs args)
             for (int64_t g0 = lo + (int64_t)warp * 32; g0 < hi; g0 += NT) {
                 const int64_t i = g0 + lane;
                 int c1a = 0, c1b = 0, c2a = 0, c2b = 0, c3a = 0, c3b = 0;
-                double nu = 0.0, invw = 0.0, y = 0.0, amp = 0.0;
-                float icf = 0.f, fc = 0.f, dx = 0.f, yf = 0.f, ampf = 0.f;
+                CoreLine L = {0.0, 0.0, 0.0, 0.0, 0.f, 0.f, 0.f, 0.f, 0.f};
                 if (i < hi) {
                     LineQ lq;
                     if constexpr (PREP) {
@@ -1911,46 +2057,73 @@ core_kernel(const KArgs args)
                         RawLine Lr;
                         Lr.nu = __ldg(J.lines.nu + i); Lr.elow = __ldg(J.lines.elow + i);
                         Lr.aif = __ldg(J.lines.aif + i); Lr.g = __ldg(J.lines.gns + i);
-                        Lr.gam = __ldg(J.lines.gamma + i); Lr.nexp = __ldg(J.lines.n + i);
-                        lq = line_quantities<true>(J, Lr);
+                        if (PK == PK_VOIGT) { Lr.gam = __ldg(J.lines.gamma + i); Lr.nexp = __ldg(J.lines.n + i); }
+                        else { Lr.gam = 0.0; Lr.nexp = 0.0; }
+                        lq = line_quantities<PK == PK_VOIGT>(J, Lr);
                     }
-                    Derived<PK_VOIGT> d = derive_line<PK_VOIGT>(T, lq, 10.5);
-                    /* FP64: the tile kernel keeps lines of y < 0 whole */
-                    if (lo16(d.c1) < hi16(d.c1) && !(PREC == GEXS_FP64 && d.y < 0.0)) {
+                    Derived<PK> d = derive_line<PK>(T, lq, ERF_Z64);
+                    if constexpr (PK == PK_ERF) {
+                        c1a = lo16(d.c1); c1b = hi16(d.c1);
+                        L.nu = d.nu; L.invw = d.invw; L.amp = dmul(d.S, J.out_scale);
+                    } else if (lo16(d.c1) < hi16(d.c1) && !(PREC == GEXS_FP64 && d.y < 0.0)) {
+                        /* FP64: the tile kernel keeps lines of y < 0 whole */
                         core_ranges(d.c1, d.c2, d.c3, c1a, c1b, c2a, c2b, c3a, c3b);
                         const double ic = fmin(fmax(floor(d.tc), -8388608.0), 8388607.0);
-                        nu = d.nu; invw = d.invw; y = d.y;
-                        amp = dmul(dmul(d.S, d.invw), J.out_scale);
-                        icf = (float)ic; fc = (float)(d.tc - ic);
-                        dx = (float)dmul(J.dnu, d.invw);
-                        yf = (float)y; ampf = (float)amp;
+                        L.nu = d.nu; L.invw = d.invw; L.y = d.y;
+                        L.amp = dmul(dmul(d.S, d.invw), J.out_scale);
+                        L.icf = (float)ic; L.fc = (float)(d.tc - ic);
+                        L.dx = (float)dmul(J.dnu, d.invw);
+                        L.yf = (float)d.y; L.ampf = (float)L.amp;
                     }
                 }
                 __syncwarp();
-                auto x_of = [&](int t) {
-                    return dmul(fabs(dsub(grid_f(J.nu_start, J.dnu, T.j0 + t), nu)), invw);
+                if constexpr (PK == PK_ERF) {
+                    const double h = 0.5 * J.dnu;
+                    const int form = J.erf_form;
+                    auto term = [&](const CoreLine& l, int t) {
+                        const double dist = fabs(dsub(grid_f(J.nu_start, J.dnu, T.j0 + t), l.nu));
+                        return dmul(l.amp, erf_bin_f64(dmul(l.invw, dsub(dist, h)),
+                                                       dmul(l.invw, dadd(dist, h)), form));
+                    };
+                    scatter_phase<PREC>(c1a, c1b, lane, L, row, LO, scr, term, term);
+                } else {
+                auto x_of = [&](const CoreLine& l, int t) {
+                    return dmul(fabs(dsub(grid_f(J.nu_start, J.dnu, T.j0 + t), l.nu)), l.invw);
                 };
                 /* II left and right of the inner part */
 #pragma unroll 1
                 for (int side = 0; side < 2; ++side)
-                    scatter_phase<DD>(side ? c2b : c1a, side ? c1b : c2a, lane, row, LO, scr, [&](int t) {
-                        if constexpr (PREC == GEXS_FP64) return amp * hum_region2<double>(x_of(t), y);
-                        const float x = fabsf(((float)t - icf) - fc) * dx;
-                        return (double)__fmul_rn(ampf, hum_region2<float>(x, yf));
-                    });
+                    scatter_phase<PREC>(side ? c2b : c1a, side ? c1b : c2a, lane, L, row, LO, scr,
+                        [&](const CoreLine& l, int t) {
+                            if constexpr (PREC == GEXS_FP32) return core_term2_f32(l, t);
+                            return l.amp * hum_region2<double>(x_of(l, t), l.y);
+                        },
+                        [&](const CoreLine& l, int t) {
+                            if constexpr (PREC == GEXS_FP32) return core_term2_f32(l, t);
+                            return core_term<PREC, 2>(x_of(l, t), l.y, l.amp);
+                        });
                 /* IV left and right of III */
 #pragma unroll 1
                 for (int side = 0; side < 2; ++side)
-                    scatter_phase<DD>(side ? c3b : c2a, side ? c2b : c3a, lane, row, LO, scr, [&](int t) {
-                        const double x = x_of(t);
-                        return amp * (PREC == GEXS_FP64 ? hum_region4<double>(x, y)
-                                                        : hum_region4_core(x, y));
+                    scatter_phase<PREC>(side ? c3b : c2a, side ? c2b : c3a, lane, L, row, LO, scr,
+                        [&](const CoreLine& l, int t) {
+                            const double x = x_of(l, t);
+                            return l.amp * (PREC == GEXS_FP64 ? hum_region4<double>(x, l.y)
+                                                              : hum_region4_core(x, l.y));
+                        },
+                        [&](const CoreLine& l, int t) {
+                            return core_term<PREC, 4>(x_of(l, t), l.y, l.amp);
+                        });
+                scatter_phase<PREC>(c3a, c3b, lane, L, row, LO, scr,
+                    [&](const CoreLine& l, int t) {
+                        const double x = x_of(l, t);
+                        return l.amp * (PREC == GEXS_FP64 ? hum_region3<double>(x, l.y)
+                                                          : hum_region3_core(x, l.y));
+                    },
+                    [&](const CoreLine& l, int t) {
+                        return core_term<PREC, 3>(x_of(l, t), l.y, l.amp);
                     });
-                scatter_phase<DD>(c3a, c3b, lane, row, LO, scr, [&](int t) {
-                    const double x = x_of(t);
-                    return amp * (PREC == GEXS_FP64 ? hum_region3<double>(x, y)
-                                                    : hum_region3_core(x, y));
-                });
+                }
             }
             __syncthreads();
             /* rows in warp order: a bin's total (hi, lo) */
@@ -1966,12 +2139,18 @@ core_kernel(const KArgs args)
                     }
                 }
             };
+            /* the Voigt core is added to the region-I result, the erf
+             * profiles are the result */
+            auto put = [&](int t, double v) {
+                double* o = J.out + T.j0 + t;
+                if (PK == PK_ERF) *o = J.accumulate ? *o + v : v;
+                else if (v != 0.0) *o += v;
+            };
             if (ns == 1) {
-                /* added to the region-I result */
                 for (int t = tid; t < T.jn; t += NT) {
                     double hi, lo;
                     total(t, hi, lo);
-                    if (hi != 0.0) J.out[T.j0 + t] += hi + lo;
+                    put(t, hi + lo);
                 }
             } else {
                 /* a slice of a split tile: its totals into its partial row, a
@@ -1999,7 +2178,7 @@ core_kernel(const KArgs args)
                             if (DD) { dd_add(hi, lo, __ldcg(r)); lo = dadd(lo, __ldcg(r + W)); }
                             else hi += __ldcg(r);
                         }
-                        if (hi != 0.0) J.out[T.j0 + t] += hi + lo;
+                        put(t, hi + lo);
                     }
                 }
             }
@@ -2119,10 +2298,10 @@ static cudaError_t launch_cfg(const KArgs& a, const gexs_launch_cfg& c, int nsm,
  * tables reserve 256 bytes for counters) */
 constexpr int CORE_COUNTER_OFFSET = 32;
 
-template <int PREC, bool PREP>
+template <int PK, int PREC, bool PREP>
 static cudaError_t launch_core(const KArgs& a, int nsm, cudaStream_t st)
 {
-    auto kern = a.order ? core_kernel<PREC, PREP, true> : core_kernel<PREC, PREP, false>;
+    auto kern = a.order ? core_kernel<PK, PREC, PREP, true> : core_kernel<PK, PREC, PREP, false>;
     const size_t smem = (size_t)CORE_WARPS * sizeof(double) *
                         (PREC == GEXS_FP64 ? 2 * core_row(a.tile_w) : core_row(a.tile_w) + SCR_D);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -2151,19 +2330,25 @@ static cudaError_t launch_pk(int prec, const KArgs& a, const gexs_launch_cfg& cf
                              cudaStream_t st)
 {
     const bool prep = a.prep != nullptr;
-    const bool f32 = prec == GEXS_FP32;
-    cudaError_t e = f32 ? (prep ? launch_cfg<PK, GEXS_FP32, true>(a, cfg, nsm, st)
-                                : launch_cfg<PK, GEXS_FP32, false>(a, cfg, nsm, st))
-                        : (prep ? launch_cfg<PK, GEXS_FP64, true>(a, cfg, nsm, st)
-                                : launch_cfg<PK, GEXS_FP64, false>(a, cfg, nsm, st));
-    if constexpr (PK == PK_VOIGT) {
-        if (e != cudaSuccess) return e;
-        return f32 ? (prep ? launch_core<GEXS_FP32, true>(a, nsm, st)
-                           : launch_core<GEXS_FP32, false>(a, nsm, st))
-                   : (prep ? launch_core<GEXS_FP64, true>(a, nsm, st)
-                           : launch_core<GEXS_FP64, false>(a, nsm, st));
+    if (prec == GEXS_FP32) {
+        cudaError_t e = prep ? launch_cfg<PK, GEXS_FP32, true>(a, cfg, nsm, st)
+                             : launch_cfg<PK, GEXS_FP32, false>(a, cfg, nsm, st);
+        if constexpr (PK == PK_VOIGT) {
+            if (e != cudaSuccess) return e;
+            return prep ? launch_core<PK, GEXS_FP32, true>(a, nsm, st)
+                        : launch_core<PK, GEXS_FP32, false>(a, nsm, st);
+        }
+        return e;
     }
-    return e;
+    if constexpr (PK != PK_ERF) {
+        cudaError_t e = prep ? launch_cfg<PK, GEXS_FP64, true>(a, cfg, nsm, st)
+                             : launch_cfg<PK, GEXS_FP64, false>(a, cfg, nsm, st);
+        if (PK != PK_VOIGT || e != cudaSuccess) return e;
+    }
+    if constexpr (PK == PK_VOIGT || PK == PK_ERF)
+        return prep ? launch_core<PK, GEXS_FP64, true>(a, nsm, st)
+                    : launch_core<PK, GEXS_FP64, false>(a, nsm, st);
+    return cudaErrorInvalidValue;
 }
 
 /* defined one per translation unit */
