@@ -242,14 +242,14 @@ template <> struct GH<16> { static constexpr int NP = 8; };
 template <> struct GH<32> { static constexpr int NP = 16; };
 
 template <int NODES>
-__device__ __forceinline__ double gh_t(int k)
+__host__ __device__ __forceinline__ constexpr double gh_t(int k)
 {
     constexpr double t16[8] = {GEXS_GH16_T_LIST};
     constexpr double t32[16] = {GEXS_GH32_T_LIST};
     return NODES == 16 ? t16[k] : t32[k];
 }
 template <int NODES>
-__device__ __forceinline__ double gh_w(int k)
+__host__ __device__ __forceinline__ constexpr double gh_w(int k)
 {
     constexpr double w16[8] = {GEXS_GH16_W_LIST};
     constexpr double w32[16] = {GEXS_GH32_W_LIST};
@@ -325,17 +325,65 @@ __device__ __forceinline__ float gh_sum_f32_wide(float x, float y2)
     return acc;
 }
 
+/* the sum as the reference writes it, any x and y */
 template <int NODES>
-__device__ __forceinline__ double gh_sum_f64(double x, double y2)
+__device__ __noinline__ double gh_sum_f64(double x, double y2)
 {
     double acc = 0.0;
-#pragma unroll
+#pragma unroll 1
     for (int k = 0; k < GH<NODES>::NP; ++k) {
         double d1 = dsub(x, gh_t<NODES>(k)), d2 = dadd(x, gh_t<NODES>(k));
         double A = dadd(y2, dmul(d1, d1)), B = dadd(y2, dmul(d2, d2));
         acc = dadd(acc, dmul(gh_w<NODES>(k), ddiv(dadd(A, B), dmul(A, B))));
     }
     return acc;
+}
+
+/* the same with refined reciprocals, for 1e-100 <= y and |x|, y <= 1e60: 11
+ * FP64 instructions per node pair */
+template <int NODES>
+__device__ __forceinline__ double gh_sum_f64_near(double x, double y2)
+{
+    double acc = 0.0;
+#pragma unroll
+    for (int k = 0; k < GH<NODES>::NP; ++k) {
+        const double d1 = x - gh_t<NODES>(k), d2 = x + gh_t<NODES>(k);
+        const double A = fma(d1, d1, y2), B = fma(d2, d2, y2);
+        acc = fma(gh_w<NODES>(k) * (A + B), rcp_f64(A * B), acc);
+    }
+    return acc;
+}
+
+/* sum_k w_k t_k^(2 m) over all nodes */
+template <int NODES>
+__host__ __device__ constexpr double gh_moment(int m)
+{
+    double s = 0.0;
+    for (int k = 0; k < GH<NODES>::NP; ++k) {
+        double v = 2.0 * gh_w<NODES>(k);
+        for (int i = 0; i < 2 * m; ++i) v *= gh_t<NODES>(k);
+        s += v;
+    }
+    return s;
+}
+
+/* Far from the nodes (|x| >= GH_FAR) the quadrature's own asymptotic
+ * series: sum_k w_k / (z - t_k) = (1/z) p(1/z^2) with p's coefficients the
+ * moments above, whose real part over y is (A + B (3 x^2 - y^2) / |z|^4) /
+ * |z|^2 for p(zeta) = A + B zeta (quad_horner).  Seven terms: the first one
+ * left out is below 2e-17 of the sum.  27 FP64 instructions whatever the
+ * number of nodes, against 90 (16 nodes) or 180 (32). */
+constexpr double GH_FAR = 32.0;
+template <int NODES>
+__device__ __forceinline__ double gh_sum_f64_far(double x, double y2)
+{
+    constexpr double c[7] = {gh_moment<NODES>(0), gh_moment<NODES>(1), gh_moment<NODES>(2),
+                             gh_moment<NODES>(3), gh_moment<NODES>(4), gh_moment<NODES>(5),
+                             gh_moment<NODES>(6)};
+    const double x2 = x * x, inv = rcp_f64(x2 + y2), i2 = inv * inv;
+    double a, b;
+    quad_horner<6>(c, 2.0 * (x2 - y2) * i2, i2, a, b);
+    return fma(b, fma(3.0, x2, -y2) * i2, a) * inv;
 }
 
 /* ------------------------------------------------ bin-averaged erf difference */

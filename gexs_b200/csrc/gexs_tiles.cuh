@@ -65,13 +65,17 @@ struct __align__(16) RecF32 {   /* 48 bytes; Doppler/Gaussian and GH */
  * part of mfcdx (their high parts are dx and mfcdx), see make_rec */
 constexpr int GH_PAIR_BIT = 1 << 25;
 
-struct __align__(16) RecF64 {   /* 64 bytes; GH */
+struct __align__(16) RecF64 {   /* 48 bytes; GH */
     double nu;             /* centre after the nu==0 rule                   */
     double invw;
-    double y;
-    double amp;            /* S*invw                                        */
-    int    win, c1, c2, c3;
-    int    mask, pad0, pad1, pad2;
+    double y2;             /* y^2                                            */
+    double a;              /* S * invw * out_scale * y / pi                  */
+    int    win;
+    int    mask;           /* bit w: touches warp w; 8 + w: its bins all at
+                              |x| >= GH_FAR; 16 + w: all in the window;
+                              bit 24: IEEE form (y < 1e-100, or |x| or y may
+                              exceed 1e60)                                   */
+    int    pad0, pad1;
 };
 
 /* FP32 Voigt record (64 bytes): the main-loop constants of a line in a
@@ -537,16 +541,29 @@ __device__ __forceinline__ void make_rec(RecV& q, const Derived<PK>& d, const ge
 }
 
 template <int PK, int B, int WARPS>
-__device__ __forceinline__ void make_rec(RecF64& q, const Derived<PK>& d, const gexs_job&,
-                                         const Tile&)
+__device__ __forceinline__ void make_rec(RecF64& q, const Derived<PK>& d, const gexs_job& J,
+                                         const Tile& T)
 {
-    q.nu = d.nu; q.invw = d.invw; q.y = d.y;
-    q.amp = dmul(d.S, d.invw);
-    q.win = d.win; q.c1 = d.c1; q.c2 = d.c2; q.c3 = d.c3;
-    q.mask = (d.win == 0) ? 0 : warp_mask<PK, B, WARPS>(d, 1);
-    q.pad0 = q.pad1 = q.pad2 = 0;
+    q.nu = d.nu; q.invw = d.invw; q.y2 = d.y * d.y;
+    q.a = dmul(dmul(d.S, d.invw), J.out_scale) * dmul(d.y, GEXS_INV_PI);
+    q.win = d.win;
+    q.pad0 = q.pad1 = 0;
+    const int a = lo16(d.win), b = hi16(d.win);
+    const double dfar = fmax(fabs(d.nu - T.f0), fabs(d.nu - T.fl));
+    const bool general = !(d.y >= 1e-100) || !(d.y < 1e60) || !(dfar * d.invw < 1e60);
+    /* distance of GH_FAR in bins */
+    const double reach = GH_FAR / d.invw * T.inv_dnu + 1.0;
+    int m = general ? 1 << 24 : 0;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+        const int r0 = 32 * B * w, r1 = r0 + 32 * B;
+        if (!(a < r1 && b > r0)) continue;
+        m |= 1 << w;
+        if (d.tc + reach < (double)r0 || d.tc - reach > (double)r1) m |= 1 << (8 + w);
+        if (a <= r0 && b >= r1) m |= 1 << (16 + w);
+    }
+    q.mask = d.win == 0 ? 0 : m;
 }
-
 
 template <int PK, int B, int WARPS>
 __device__ __forceinline__ void make_rec(RecV64& q, const Derived<PK>& d, const gexs_job& J,
@@ -923,31 +940,44 @@ __device__ __forceinline__ void lines_voigt_f32(const RecV* __restrict__ rec, in
     }
 }
 
-/* FP64 form of the Gauss-Hermite profiles: per-bin
- * window tests, FP64 arithmetic, bins sum their lines in line order (the
- * order of the FP64 oracle). */
+/* FP64 form of the Gauss-Hermite profiles: bins sum their lines in line
+ * order.  Bound by the FP64 pipe: 30 instructions per evaluation at |x| >=
+ * GH_FAR, which is most of a 25 cm^-1 window, and 11 per node pair nearer
+ * the centre.  2e5 lines, 32 nodes, 198,001 bins: 10.0 ms with the node sum
+ * everywhere and IEEE divisions, 1.4 ms so. */
 template <int PK, int B>
 __device__ __forceinline__ void lines_f64(const RecF64* __restrict__ rec, int nrec, int warp,
-                                          int lane, const double (&fbin)[B], double (&acc)[B],
-                                          const gexs_job& J)
+                                          int lane, const double (&fbin)[B], double (&acc)[B])
 {
-    const int wb = warp * 32 * B;
-    const int bit = 1 << warp;
-    const double out_scale = J.out_scale;
+    constexpr int NODES = (PK == PK_GH16) ? 16 : 32;
+    const int tl = warp * 32 * B + lane;
     for (int i = 0; i < nrec; ++i) {
         const RecF64& q = rec[i];
-        if (!(q.mask & bit)) continue;
-        const int a = lo16(q.win), b = hi16(q.win);
-        {
-            constexpr int NODES = (PK == PK_GH16) ? 16 : 32;
-            const double y2 = dmul(q.y, q.y), yk = dmul(q.y, GEXS_INV_PI);
+        const int mask = q.mask >> warp;
+        if (!(mask & 1)) continue;
+        const int wa = lo16(q.win);
+        const unsigned wn = (unsigned)(hi16(q.win) - wa);
+        const double nu = q.nu, invw = q.invw, y2 = q.y2, a = q.a;
+        if (q.mask >> 24) {
 #pragma unroll
             for (int k = 0; k < B; ++k) {
-                const int t = wb + lane + 32 * k;
-                if (t < a || t >= b) continue;
-                double x = dmul(fabs(dsub(fbin[k], q.nu)), q.invw);
-                double kv = dmul(gh_sum_f64<NODES>(x, y2), yk);
-                acc[k] = dadd(acc[k], dmul(dmul(q.amp, kv), out_scale));
+                if ((unsigned)(tl + 32 * k - wa) >= wn) continue;
+                const double x = dmul(fabs(dsub(fbin[k], nu)), invw);
+                acc[k] = fma(a, gh_sum_f64<NODES>(x, y2), acc[k]);
+            }
+        } else if (mask & (1 << 8)) {
+            const bool full = mask & (1 << 16);
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const double v = gh_sum_f64_far<NODES>((fbin[k] - nu) * invw, y2);
+                const bool in = full || (unsigned)(tl + 32 * k - wa) < wn;
+                acc[k] = fma(a, in ? v : 0.0, acc[k]);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                if ((unsigned)(tl + 32 * k - wa) >= wn) continue;
+                acc[k] = fma(a, gh_sum_f64_near<NODES>((fbin[k] - nu) * invw, y2), acc[k]);
             }
         }
     }
@@ -1268,7 +1298,7 @@ tile_kernel(const KArgs args)
                                            fbin, acc);
                     else
                         lines_f64<PK, B>(reinterpret_cast<const RecF64*>(s_rec) + c0, cn, warp, lane,
-                                         fbin, acc, J);
+                                         fbin, acc);
                     if (cn == left) end_block(acc);
                     c0 += cn;
                 }
