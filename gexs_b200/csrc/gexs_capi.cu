@@ -317,14 +317,11 @@ static int64_t max_lines(const Group& g)
     return m;
 }
 
-/* prep kernel then tile kernel for one group whose image is at d */
+/* the kernels of one group whose image is at d */
 static cudaError_t enqueue_group(const Group& g, const Layout& L, unsigned char* d, bool prep,
                                  const gexs_launch_cfg& cfg, int* d_err, int nsm, cudaStream_t s)
 {
     double* const* pp = reinterpret_cast<double* const*>(d + L.opp);
-    cudaError_t e = cudaSuccess;
-    if (prep) e = launch_prep((const gexs_job*)d, pp, (int)g.jobs.size(), max_lines(g), nsm, s);
-    if (e != cudaSuccess) return e;
     SliceTables sl;
     std::memset(&sl, 0, sizeof(sl));
     if (L.sliced) {
@@ -355,7 +352,8 @@ static cudaError_t enqueue_group(const Group& g, const Layout& L, unsigned char*
                         (int)g.jobs.size(), g.nitems, (int*)(d + L.oc), d_err,
                         prep ? pp : nullptr, cfg, nsm, s, L.sliced ? &sl : nullptr,
                         L.csliced ? &csl : nullptr,
-                        g.order.empty() ? nullptr : (const int*)(d + L.op) + g.prefix.size());
+                        g.order.empty() ? nullptr : (const int*)(d + L.op) + g.prefix.size(),
+                        prep ? max_lines(g) : 0);
 }
 
 extern "C" {
@@ -644,8 +642,8 @@ static int batch_enqueue(gexs_batch* b, cudaStream_t s)
         const Group& g = b->groups[gi];
         if (g.nitems == 0) continue;
         unsigned char* d = (unsigned char*)b->dmem[gi];
-        cudaError_t e = zero_ints((int*)(d + b->layouts[gi].oc), 1, s);
-        if (e != cudaSuccess) return cuda_error(e, "reset work counter");
+        cudaError_t e = zero_ints((int*)(d + b->layouts[gi].oc), 64, s);
+        if (e != cudaSuccess) return cuda_error(e, "reset work counters");
         e = enqueue_group(g, b->layouts[gi], d, b->prep[gi], b->cfgs[gi], b->ctx->d_err,
                           b->ctx->nsm, s);
         if (e != cudaSuccess) return cuda_error(e, "tile kernel launch");

@@ -17,7 +17,7 @@ int tile_bins(const gexs_launch_cfg& c);
  * therefore depends on the tile alone (unless the partial rows would pass
  * 1 GiB); FP64 sums do not (SUM_BLOCK).  A split tile's slices write
  * partial rows; the last one to finish sums them in slice order into the
- * output.  All arrays live in the launch table; slice_plan_kernel fills
+ * output.  All arrays live in the launch table; the set-up kernel fills
  * them (and zeroes the tickets) before the kernel runs. */
 struct SliceTables {
     int*       prefix;      /* ntiles + 1: first item of each tile       */
@@ -32,19 +32,22 @@ struct SliceTables {
     int        cut_shift;   /* core kernel: see core_cut                    */
 };
 
-/* d_prep: device array of per-job prep arrays (S | invw | y, 3 N doubles
- * each, from launch_prep), or NULL to derive every line on load.
+/* One set-up launch (prep arrays, slice tables) where there is any to do,
+ * then the kernels of one (profile class, precision).
+ * d_prep: device array of per-job prep arrays (S | invw | y, 3 N doubles
+ * each), filled here for lists of up to prep_lines lines, or NULL to derive
+ * every line on load.
  * d_order: tile-major order tables of a launch with several jobs (F | R | P,
  * 3 njobs + 1 ints, see tile_order in gexs_capi.cu), or NULL for job-major
  * items.
- * d_counter: a 256-byte block of work counters; the caller zeroes the
- * first int, the FP32 Voigt core kernel's counter (int 32) is zeroed here
- * (by zero_ints). */
+ * d_counter: a 256-byte block of work counters, zeroed by the caller: int 0
+ * the tile kernel's, 16 the set-up kernel's, 32 the core kernel's. */
 cudaError_t launch_tiles(int pk, int prec, const gexs_job* d_jobs, const int* d_prefix,
                          int njobs, int nitems, int* d_counter, int* d_err,
                          double* const* d_prep, const gexs_launch_cfg& cfg, int nsm,
                          cudaStream_t st, const SliceTables* sl = nullptr,
-                         const SliceTables* csl = nullptr, const int* d_order = nullptr);
+                         const SliceTables* csl = nullptr, const int* d_order = nullptr,
+                         int64_t prep_lines = 0);
 /* The FP64 tile kernel sums a bin's lines in order within blocks of this
  * many lines of the list (by index, so that a tile of any shape or cut has
  * the same block sums) and the blocks' sums as (hi, lo) pairs, whose
@@ -74,8 +77,6 @@ __host__ __device__ inline long long core_cut(long long grid_points, int tile_w,
 }
 bool core_slices_apply(int pk, int prec, int tile_w);
 int core_cut_shift(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows);
-cudaError_t launch_prep(const gexs_job* d_jobs, double* const* d_prep, int njobs,
-                        int64_t max_lines, int nsm, cudaStream_t st);
 cudaError_t launch_count(const gexs_job* d_jobs, int njobs, unsigned long long* d_counts,
                          int nsm, cudaStream_t st);
 cudaError_t launch_partition(const double* d_e, const int32_t* d_g, int64_t n,

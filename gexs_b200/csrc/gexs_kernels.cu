@@ -1,7 +1,7 @@
 /*
- * gexs_kernels.cu — the per-job prep kernel, exact evaluation counting,
- * Q(T), and the front of the tile-kernel dispatch (the tile kernel itself
- * is in gexs_tiles.cuh).
+ * gexs_kernels.cu — the set-up kernel (per-line prep arrays, slice tables),
+ * exact evaluation counting, Q(T), and the front of the tile-kernel
+ * dispatch (the tile kernels themselves are in gexs_tiles.cuh).
  */
 #include <cmath>
 #include <cstring>
@@ -10,20 +10,19 @@
 
 namespace gexs {
 
-/* ------------------------------------------------------------ prep kernel
+/* ------------------------------------------------------------ prep
  * Per job, the FP64 per-line quantities once: S at base[i], invw at
  * base[N + i], y at base[2N + i] (N = line count).  The tile kernel then
  * reads 32 bytes per line instead of recomputing two exponentials, a power
- * and two divisions for every tile the line reaches. */
-__global__ void prep_kernel(const gexs_job* __restrict__ jobs, double* const* __restrict__ prep)
+ * and two divisions for every tile the line reaches.  Lines first + k
+ * stride. */
+__device__ __forceinline__ void prep_lines(const gexs_job& J, double* base, int64_t first,
+                                           int64_t stride)
 {
-    const gexs_job& J = jobs[blockIdx.y];
-    double* base = prep[blockIdx.y];
     const int64_t N = J.lines.count;
     const bool press = J.profile == GEXS_VOIGT || J.profile == GEXS_VOIGT_QUAD;
     const bool compact = J.lines.format == GEXS_LINES_COMPACT;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N;
-         i += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t i = first; i < N; i += stride) {
         RawLine L;
         L.nu = J.lines.nu[i];
         if (compact) {
@@ -125,55 +124,21 @@ int profile_class(const gexs_job& j)
     return -1;
 }
 
-cudaError_t launch_tiles(int pk, int prec, const gexs_job* d_jobs, const int* d_prefix,
-                         int njobs, int nitems, int* d_counter, int* d_err,
-                         double* const* d_prep, const gexs_launch_cfg& cfg, int nsm,
-                         cudaStream_t st, const SliceTables* sl, const SliceTables* csl,
-                         const int* d_order)
-{
-    KArgs a;
-    a.jobs = d_jobs; a.prefix = d_prefix; a.njobs = njobs; a.nitems = nitems;
-    a.order = njobs > 1 ? d_order : nullptr;
-    a.counter = d_counter; a.err = d_err; a.prep = d_prep;
-    a.tile_w = tile_bins(cfg);
-    a.spin = cfg.wait_spins > 0 ? cfg.wait_spins : WS_SPIN;
-    std::memset(&a.sl, 0, sizeof(a.sl));
-    std::memset(&a.csl, 0, sizeof(a.csl));
-    if (sl && slices_apply(pk, prec)) a.sl = *sl;
-    if (csl && core_slices_apply(pk, prec, a.tile_w)) a.csl = *csl;
-    switch (pk) {
-    case PK_VOIGT: return launch_tiles_voigt(prec, a, cfg, nsm, st);
-    case PK_ERF:   return launch_tiles_erf(prec, a, cfg, nsm, st);
-    case PK_GH16:  return launch_tiles_gh16(prec, a, cfg, nsm, st);
-    case PK_GH32:  return launch_tiles_gh32(prec, a, cfg, nsm, st);
-    }
-    return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_prep(const gexs_job* d_jobs, double* const* d_prep, int njobs,
-                        int64_t max_lines, int nsm, cudaStream_t st)
-{
-    if (max_lines <= 0) return cudaSuccess;
-    int bx = (int)std::min<int64_t>((max_lines + 255) / 256, (int64_t)nsm * 8);
-    dim3 grid(bx, njobs);
-    prep_kernel<<<grid, 256, 0, st>>>(d_jobs, d_prep);
-    return cudaGetLastError();
-}
-
 int tile_bins(const gexs_launch_cfg& c) { return 32 * c.bins_per_lane * c.warps; }
 
-/* ------------------------------------------------------------ line slices */
+/* ------------------------------------------------------------ set-up
+ * One launch before the tile kernels: the line ranges and slice counts of
+ * every tile (a warp per tile), their scans (the last of those blocks to
+ * finish) and the prep arrays (the other blocks).  Its work is short and
+ * bound by launch latency for small jobs: separate kernels for prep, two
+ * plans, two one-CTA scans and a counter reset cost 26 us of a 170 us pass
+ * with 3000 lines, this one 11. */
 namespace {
-/* one warp per tile: the tile's line range, searched exactly as the
- * region-I kernel's producers search it, and its slice count */
-__global__ void slice_plan_kernel(const KArgs a)
+
+/* a tile's line range, searched exactly as the region-I kernel's producers
+ * search it, and its slice count */
+__device__ __forceinline__ void plan_tile(const KArgs& a, const gexs_job& J, int ti, int tj, int lane)
 {
-    const int lane = threadIdx.x & 31;
-    const int ti = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (ti >= a.nitems) return;
-    int tj = 0;
-    const int jl = tile_job(a, ti, &tj);
-    const gexs_job& J = a.jobs[jl];
     const int64_t j0 = J.start_idx + (int64_t)tj * a.tile_w;
     const int jn = (int)min((int64_t)a.tile_w, J.start_idx + J.n_points - j0);
     const double f0 = grid_f(J.nu_start, J.dnu, j0);
@@ -192,14 +157,8 @@ __global__ void slice_plan_kernel(const KArgs a)
 }
 
 /* the same for the core kernel, with its own search (reach_range) */
-__global__ void core_slice_plan_kernel(const KArgs a)
+__device__ __forceinline__ void plan_core_tile(const KArgs& a, const gexs_job& J, int ti, int tj, int lane)
 {
-    const int lane = threadIdx.x & 31;
-    const int ti = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (ti >= a.nitems) return;
-    int tj = 0;
-    const int jl = tile_job(a, ti, &tj);
-    const gexs_job& J = a.jobs[jl];
     const int64_t t0 = J.start_idx + (int64_t)tj * a.tile_w;
     const int64_t tend = min((int64_t)(t0 + a.tile_w), J.start_idx + J.n_points);
     const int jn = (int)min((int64_t)CORE_W, tend - t0);
@@ -220,65 +179,124 @@ __global__ void core_slice_plan_kernel(const KArgs a)
     }
 }
 
-/* one CTA: exclusive prefixes of the slice counts (items) and of the
- * slices of split tiles (partial rows), and the item count */
-__global__ void __launch_bounds__(1024) slice_scan_kernel(const KArgs a)
+constexpr int SETUP_NT = 256, SCAN_ITEMS = 8;
+typedef cub::BlockScan<unsigned long long, SETUP_NT> SetupScan;
+
+/* exclusive prefixes of the slice counts (items, upper word) and of the
+ * slices of split tiles (partial rows, lower word), and the item count */
+__device__ void scan_slices(const SliceTables& sl, int ntiles, int* err,
+                            SetupScan::TempStorage& tmp)
 {
-    typedef cub::BlockScan<int, 1024> Scan;
-    __shared__ typename Scan::TempStorage tmp;
-    __shared__ long long carry, rcarry;
-    if (threadIdx.x == 0) { carry = 0; rcarry = 0; }
-    __syncthreads();
-    for (int base = 0; base < a.nitems; base += 1024) {
-        const int i = base + (int)threadIdx.x;
-        const int v = i < a.nitems ? a.sl.counts[i] : 0;
-        const int r = v > 1 ? v : 0;
-        int ex = 0, tot = 0, rex = 0, rtot = 0;
-        Scan(tmp).ExclusiveSum(v, ex, tot);
-        __syncthreads();
-        Scan(tmp).ExclusiveSum(r, rex, rtot);
-        if (i < a.nitems) {
-            a.sl.prefix[i] = (int)min(carry + ex, (long long)INT32_MAX);
-            a.sl.rowbase[i] = (int)min(rcarry + rex, (long long)INT32_MAX);
+    unsigned long long carry = 0;
+    for (int base = 0; base < ntiles; base += SETUP_NT * SCAN_ITEMS) {
+        unsigned long long v[SCAN_ITEMS], tot;
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; ++k) {
+            const int i = base + (int)threadIdx.x * SCAN_ITEMS + k;
+            const unsigned c = i < ntiles ? (unsigned)__ldcg(sl.counts + i) : 0u;
+            v[k] = ((unsigned long long)c << 32) | (c > 1 ? c : 0u);
         }
-        __syncthreads();
-        if (threadIdx.x == 0) { carry += tot; rcarry += rtot; }
+        SetupScan(tmp).ExclusiveSum(v, v, tot);
+#pragma unroll
+        for (int k = 0; k < SCAN_ITEMS; ++k) {
+            const int i = base + (int)threadIdx.x * SCAN_ITEMS + k;
+            if (i >= ntiles) break;
+            const unsigned long long e = carry + v[k];
+            sl.prefix[i] = (int)(e >> 32);
+            sl.rowbase[i] = (int)(unsigned)e;
+        }
+        carry += tot;
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        if (rcarry > a.sl.max_rows || carry > INT32_MAX) {
+        const unsigned items = (unsigned)(carry >> 32), rows = (unsigned)carry;
+        if (rows > (unsigned)sl.max_rows || items > (unsigned)INT32_MAX) {
             /* cannot happen with the host's bound; run no item rather than
              * write past the partial rows */
-            atomicOr(a.err, GEXS_KERR_SLICES);
-            *a.sl.nitems = 0;
+            atomicOr(err, GEXS_KERR_SLICES);
+            *sl.nitems = 0;
         } else {
-            a.sl.prefix[a.nitems] = (int)carry;
-            *a.sl.nitems = (int)carry;
+            sl.prefix[ntiles] = (int)items;
+            *sl.nitems = (int)items;
         }
     }
 }
+
+/* int of the counter block that the set-up kernel's plan blocks count in */
+constexpr int SETUP_COUNTER = 16;
+
+/* blocks [0, nplan): eight tiles each; then per_job blocks a job for prep */
+__global__ void __launch_bounds__(SETUP_NT) setup_kernel(const KArgs a, int nplan, int per_job)
+{
+    __shared__ SetupScan::TempStorage tmp;
+    __shared__ int s_last;
+    if ((int)blockIdx.x >= nplan) {
+        const int b = (int)blockIdx.x - nplan, j = b / per_job;
+        prep_lines(a.jobs[j], a.prep[j], (int64_t)(b % per_job) * SETUP_NT + threadIdx.x,
+                   (int64_t)per_job * SETUP_NT);
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    const int ti = blockIdx.x * (SETUP_NT / 32) + (threadIdx.x >> 5);
+    if (ti < a.nitems) {
+        int tj = 0;
+        const gexs_job& J = a.jobs[tile_job(a, ti, &tj)];
+        if (a.sl.prefix) plan_tile(a, J, ti, tj, lane);
+        if (a.csl.prefix) plan_core_tile(a, J, ti, tj, lane);
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(a.counter + SETUP_COUNTER, 1) == nplan - 1;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    if (a.sl.prefix) scan_slices(a.sl, a.nitems, a.err, tmp);
+    __syncthreads();
+    if (a.csl.prefix) scan_slices(a.csl, a.nitems, a.err, tmp);
+}
 }  // namespace
 
-cudaError_t launch_slice_plan(const KArgs& a, cudaStream_t st)
+/* max_lines: the longest list of the launch's jobs when they have prep
+ * arrays, else 0 */
+static cudaError_t launch_setup(const KArgs& a, int64_t max_lines, int nsm, cudaStream_t st)
 {
-    if (a.nitems <= 0) return cudaSuccess;
-    slice_plan_kernel<<<(a.nitems + 7) / 8, 256, 0, st>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    slice_scan_kernel<<<1, 1024, 0, st>>>(a);
+    const bool plan = (a.sl.prefix || a.csl.prefix) && a.nitems > 0;
+    const int nplan = plan ? (a.nitems + SETUP_NT / 32 - 1) / (SETUP_NT / 32) : 0;
+    const int per_job = a.prep && max_lines > 0
+                            ? (int)std::min<int64_t>((max_lines + SETUP_NT - 1) / SETUP_NT, (int64_t)nsm * 8)
+                            : 0;
+    const int64_t blocks = nplan + (int64_t)per_job * a.njobs;
+    if (blocks == 0) return cudaSuccess;
+    if (blocks > INT32_MAX) return cudaErrorInvalidValue;
+    setup_kernel<<<(unsigned)blocks, SETUP_NT, 0, st>>>(a, nplan, per_job > 0 ? per_job : 1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_core_slice_plan(const KArgs& a, cudaStream_t st)
+cudaError_t launch_tiles(int pk, int prec, const gexs_job* d_jobs, const int* d_prefix,
+                         int njobs, int nitems, int* d_counter, int* d_err,
+                         double* const* d_prep, const gexs_launch_cfg& cfg, int nsm,
+                         cudaStream_t st, const SliceTables* sl, const SliceTables* csl,
+                         const int* d_order, int64_t prep_lines)
 {
-    if (a.nitems <= 0) return cudaSuccess;
-    core_slice_plan_kernel<<<(a.nitems + 7) / 8, 256, 0, st>>>(a);
-    cudaError_t e = cudaGetLastError();
+    KArgs a;
+    a.jobs = d_jobs; a.prefix = d_prefix; a.njobs = njobs; a.nitems = nitems;
+    a.order = njobs > 1 ? d_order : nullptr;
+    a.counter = d_counter; a.err = d_err; a.prep = d_prep;
+    a.tile_w = tile_bins(cfg);
+    a.spin = cfg.wait_spins > 0 ? cfg.wait_spins : WS_SPIN;
+    std::memset(&a.sl, 0, sizeof(a.sl));
+    std::memset(&a.csl, 0, sizeof(a.csl));
+    if (sl && slices_apply(pk, prec)) a.sl = *sl;
+    if (csl && core_slices_apply(pk, prec, a.tile_w)) a.csl = *csl;
+    const cudaError_t e = launch_setup(a, prep_lines, nsm, st);
     if (e != cudaSuccess) return e;
-    KArgs c = a;
-    c.sl = a.csl;
-    slice_scan_kernel<<<1, 1024, 0, st>>>(c);
-    return cudaGetLastError();
+    switch (pk) {
+    case PK_VOIGT: return launch_tiles_voigt(prec, a, cfg, nsm, st);
+    case PK_ERF:   return launch_tiles_erf(prec, a, cfg, nsm, st);
+    case PK_GH16:  return launch_tiles_gh16(prec, a, cfg, nsm, st);
+    case PK_GH32:  return launch_tiles_gh32(prec, a, cfg, nsm, st);
+    }
+    return cudaErrorInvalidValue;
 }
 
 bool slices_apply(int pk, int prec) { return !(pk == PK_ERF && prec == GEXS_FP64); }

@@ -273,7 +273,7 @@ struct RawLine { double nu, elow, aif, gam, nexp; int g; };
 
 /* FP64 per-line quantities of a job: centre (after the nu==0 rule), S(T),
  * 1/width and y = gammaL/width.  Either computed on load or read from the
- * job's prep arrays (prep_kernel). */
+ * job's prep arrays (set-up kernel). */
 struct LineQ { double nu, S, invw, y; };
 
 template <int PK>
@@ -399,11 +399,6 @@ __device__ __forceinline__ int tile_job(const KArgs& a, int ti, int* tile)
     *tile = ti - __ldg(a.prefix + jl);
     return jl;
 }
-
-/* slice_plan_kernel + slice_scan_kernel (gexs_kernels.cu): every tile's
- * line range and slice count, then the item prefix and count */
-cudaError_t launch_slice_plan(const KArgs& a, cudaStream_t st);
-cudaError_t launch_core_slice_plan(const KArgs& a, cudaStream_t st);
 
 __device__ __forceinline__ void kahan_add(float& s, float& c, float v)
 {
@@ -1541,7 +1536,7 @@ voigt_ws_kernel(const KArgs args)
             const int64_t nl = J.lines.count;
             const double margin = 2.0 * J.dnu + 1e-9 * (fabs(T.fl) + J.cutoff);
             if (sliced) {
-                /* the item's lines: the tile's range from slice_plan_kernel, cut */
+                /* the item's lines: the tile's range from the set-up kernel, cut */
                 if (ptid == 0) {
                     const long long tlo = __ldg(args.sl.lohi + 2 * ti), thi = __ldg(args.sl.lohi + 2 * ti + 1);
                     const long long per = (thi - tlo + ns - 1) / ns;
@@ -2052,7 +2047,7 @@ core_kernel(const KArgs args)
             double vlo, vhi;
             reach_range(J, T.f0, T.fl, vlo, vhi);
             if (sliced) {
-                /* the range from core_slice_plan_kernel, cut into ns parts */
+                /* the range from the set-up kernel, cut into ns parts */
                 if (tid == 0) {
                     const long long tlo = __ldg(args.csl.lohi + 2 * ti), thi = __ldg(args.csl.lohi + 2 * ti + 1);
                     const long long per = (thi - tlo + ns - 1) / ns;
@@ -2295,10 +2290,6 @@ static cudaError_t launch_ws(const KArgs& a, const gexs_launch_cfg& c, int nsm, 
 template <int PK, int PREC, bool PREP>
 static cudaError_t launch_cfg(const KArgs& a, const gexs_launch_cfg& c, int nsm, cudaStream_t st)
 {
-    if (a.sl.prefix) {
-        cudaError_t e = launch_slice_plan(a, st);
-        if (e != cudaSuccess) return e;
-    }
     if constexpr (PK == PK_VOIGT && PREC == GEXS_FP32) {
         return launch_ws<PREP>(a, c, nsm, st);
     } else {
@@ -2343,12 +2334,6 @@ static cudaError_t launch_core(const KArgs& a, int nsm, cudaStream_t st)
     const int grid = a.csl.prefix ? max(occ, 1) * nsm : max(1, min(a.nitems, max(occ, 1) * nsm));
     KArgs c = a;
     c.counter = a.counter + CORE_COUNTER_OFFSET;
-    e = zero_ints(c.counter, 1, st);
-    if (e != cudaSuccess) return e;
-    if (c.csl.prefix) {
-        e = launch_core_slice_plan(c, st);
-        if (e != cudaSuccess) return e;
-    }
     kern<<<grid, CORE_WARPS * 32, smem, st>>>(c);
     return cudaGetLastError();
 }
