@@ -28,6 +28,7 @@ SOURCES = [
     "csrc/gexs_noalloc.cu",
     "csrc/gexs_ingest.cu",
     "host/B200Manager.cpp",
+    "host/gexs_upload.cpp",
     "host/gexs_server.cpp",
     "host/B200ExomolReader.cpp",
     "host/gexs_output.cpp",

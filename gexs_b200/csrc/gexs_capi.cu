@@ -79,6 +79,7 @@ struct gexs_ctx {
      * release threshold) and never made to wait on a free from another
      * stream (no internal dependencies), so calls on two streams overlap */
     cudaMemPool_t pool = nullptr;
+    gexs::Uploader* up = nullptr;    /* pinned staging, allocated on first use */
     std::mutex mu;
     std::map<int, gexs_launch_cfg> tuned;   /* key: pk*4 + prec */
 };
@@ -87,6 +88,7 @@ namespace gexs {
 int ctx_device(gexs_ctx* c) { return c->device; }
 int ctx_sm_count(gexs_ctx* c) { return c->nsm; }
 cudaMemPool_t ctx_pool(gexs_ctx* c) { return c->pool; }
+Uploader* ctx_uploader(gexs_ctx* c) { return c->up; }
 
 /* gexs_debug_fail_allocs: allocations still to refuse (host-side fault
  * injection for the out-of-memory paths; nothing reaches the device) */
@@ -505,6 +507,7 @@ int gexs_ctx_create(int device, gexs_ctx** out)
         c->pool = nullptr;
     }
     cudaGetLastError();
+    c->up = gexs::uploader_create(device);
     *out = c;
     return GEXS_OK;
 }
@@ -513,6 +516,7 @@ int gexs_ctx_destroy(gexs_ctx* ctx)
 {
     if (!ctx) return GEXS_OK;
     cudaSetDevice(ctx->device);
+    gexs::uploader_destroy(ctx->up);
     cudaFree(ctx->d_err);
     if (ctx->pool) cudaMemPoolDestroy(ctx->pool);
     delete ctx;
@@ -816,17 +820,18 @@ int gexs_partition(gexs_ctx* ctx, const double* d_energy, const int32_t* d_g, in
         betas[i] = planck * vellgt / (boltz * h_temps[i]);
     }
     int nchunk = (int)std::min<int64_t>(ctx->nsm * 2, (nstates + 255) / 256);
-    double *db = nullptr, *dp = nullptr, *dq = nullptr;
-    if (cudaMalloc(&db, sizeof(double) * nt) != cudaSuccess ||
-        cudaMalloc(&dp, sizeof(double) * (size_t)nt * nchunk) != cudaSuccess ||
-        cudaMalloc(&dq, sizeof(double) * nt) != cudaSuccess) {
-        cudaFree(db); cudaFree(dp); cudaFree(dq);
+    /* one block of the context's pool: temperatures' betas, chunk sums, Q */
+    void* d = nullptr;
+    cudaStream_t s = 0;
+    if (pool_alloc(ctx->pool, &d, sizeof(double) * ((size_t)nt * nchunk + 2 * (size_t)nt), s) != cudaSuccess)
         return set_error(GEXS_ERR_OOM, "partition buffers");
-    }
-    cudaMemcpy(db, betas.data(), sizeof(double) * nt, cudaMemcpyHostToDevice);
-    cudaError_t e = launch_partition(d_energy, d_g, nstates, db, nt, dp, nchunk, dq, 0);
-    if (e == cudaSuccess) e = cudaMemcpy(h_q, dq, sizeof(double) * nt, cudaMemcpyDeviceToHost);
-    cudaFree(db); cudaFree(dp); cudaFree(dq);
+    double *db = (double*)d, *dq = db + nt, *dp = dq + nt;
+    cudaError_t e = put_bytes(db, betas.data(), sizeof(double) * nt, s);
+    if (e == cudaSuccess) e = launch_partition(d_energy, d_g, nstates, db, nt, dp, nchunk, dq, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_q, dq, sizeof(double) * nt, cudaMemcpyDeviceToHost, s);
+    cudaFreeAsync(d, s);
+    const cudaError_t es = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) return cuda_error(e, "partition kernel");
     return GEXS_OK;
 }

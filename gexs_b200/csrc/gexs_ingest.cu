@@ -467,10 +467,27 @@ __global__ void iota_kernel(int64_t* __restrict__ v, int64_t n)
 }
 
 /* ------------------------------------------------------------ host helpers */
+/* alloc: memory that a returned table may own (cudaMalloc).  scratch: from
+ * the context's pool, freed in stream order; a parse's scratch came to some
+ * twenty cudaMalloc/cudaFree pairs, each of which waits for the device. */
 struct DevBuf {
     void* p = nullptr;
-    ~DevBuf() { if (p) cudaFree(p); }
+    bool pooled = false;
+    cudaStream_t stream = 0;
+    ~DevBuf()
+    {
+        if (!p) return;
+        if (pooled) cudaFreeAsync(p, stream);
+        else cudaFree(p);
+    }
     cudaError_t alloc(size_t n) { return cudaMalloc(&p, n ? n : 1); }
+    cudaError_t scratch(gexs_ctx* ctx, size_t n, cudaStream_t s)
+    {
+        pooled = true; stream = s;
+        const cudaError_t e = pool_alloc(ctx_pool(ctx), &p, n ? n : 1, s);
+        if (e != cudaSuccess) p = nullptr;
+        return e;
+    }
     template <typename T> T* as() const { return reinterpret_cast<T*>(p); }
     void* release() { void* q = p; p = nullptr; return q; }
 };
@@ -488,21 +505,23 @@ int index_text(gexs_ctx* ctx, const char* h_text, int64_t nbytes, DevBuf& d_text
 {
     *nlines = 0;
     if (nbytes == 0) return GEXS_OK;
-    if (d_text.alloc((size_t)nbytes + 16) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: text buffer");
-    cudaError_t e = cudaMemcpyAsync(d_text.p, h_text, (size_t)nbytes, cudaMemcpyHostToDevice, s);
-    if (e != cudaSuccess) return cuda_error(e, "ingest: copy text");
+    if (d_text.scratch(ctx, (size_t)nbytes + 16, s) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: text buffer");
+    const gexs_upload_piece piece = {d_text.p, h_text, (size_t)nbytes, nullptr};
+    const int up = gexs_ctx_upload(ctx, &piece, 1, s);
+    if (up) return up;
+    cudaError_t e;
     const int64_t nchunk = (nbytes + CHUNK - 1) / CHUNK;
     /* counts[nchunk] stays 0 so the exclusive scan's last entry is the total */
     DevBuf d_cnt, d_off, d_tmp;
-    if (d_cnt.alloc(sizeof(int64_t) * (nchunk + 1)) != cudaSuccess ||
-        d_off.alloc(sizeof(int64_t) * (nchunk + 1)) != cudaSuccess)
+    if (d_cnt.scratch(ctx, sizeof(int64_t) * (nchunk + 1), s) != cudaSuccess ||
+        d_off.scratch(ctx, sizeof(int64_t) * (nchunk + 1), s) != cudaSuccess)
         return set_error(GEXS_ERR_OOM, "ingest: line index");
     cudaMemsetAsync(d_cnt.p, 0, sizeof(int64_t) * (nchunk + 1), s);
     const int wgrid = grid_for(ctx, nchunk * 32, 256);
     nl_count_kernel<<<wgrid, 256, 0, s>>>(d_text.as<uint8_t>(), nbytes, nchunk, d_cnt.as<int64_t>());
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, d_cnt.as<int64_t>(), d_off.as<int64_t>(), (int)(nchunk + 1), s);
-    if (d_tmp.alloc(tb) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: scan");
+    if (d_tmp.scratch(ctx, tb, s) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: scan");
     cub::DeviceScan::ExclusiveSum(d_tmp.p, tb, d_cnt.as<int64_t>(), d_off.as<int64_t>(), (int)(nchunk + 1), s);
     int64_t nnl = 0;
     e = cudaMemcpyAsync(&nnl, d_off.as<int64_t>() + nchunk, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
@@ -512,7 +531,7 @@ int index_text(gexs_ctx* ctx, const char* h_text, int64_t nbytes, DevBuf& d_text
     e = cudaMemcpy(&last, d_text.as<char>() + nbytes - 1, 1, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_error(e, "ingest: last byte");
     const int64_t nl = nnl + (last != '\n' ? 1 : 0);
-    if (d_end.alloc(sizeof(int64_t) * (nl + 1)) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: line index");
+    if (d_end.scratch(ctx, sizeof(int64_t) * (nl + 1), s) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: line index");
     nl_index_kernel<<<wgrid, 256, 0, s>>>(d_text.as<uint8_t>(), nbytes, nchunk, d_off.as<int64_t>(),
                                           d_end.as<int64_t>());
     if (last != '\n') {
@@ -531,14 +550,14 @@ int sort_lines(gexs_ctx* ctx, int64_t nrec, DevBuf& nu, DevBuf& el, DevBuf& A, D
 {
     const size_t n8 = sizeof(double) * nrec;
     DevBuf k2, i1, i2, t2;
-    if (k2.alloc(n8) != cudaSuccess || i1.alloc(sizeof(int64_t) * nrec) != cudaSuccess ||
-        i2.alloc(sizeof(int64_t) * nrec) != cudaSuccess)
+    if (k2.alloc(n8) != cudaSuccess || i1.scratch(ctx, sizeof(int64_t) * nrec, s) != cudaSuccess ||
+        i2.scratch(ctx, sizeof(int64_t) * nrec, s) != cudaSuccess)
         return set_error(GEXS_ERR_OOM, "ingest: sort buffers");
     iota_kernel<<<grid_for(ctx, nrec, 256), 256, 0, s>>>(i1.as<int64_t>(), nrec);
     size_t sb = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, sb, nu.as<double>(), k2.as<double>(), i1.as<int64_t>(),
                                     i2.as<int64_t>(), nrec, 0, 64, s);
-    if (t2.alloc(sb) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: sort");
+    if (t2.scratch(ctx, sb, s) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: sort");
     cub::DeviceRadixSort::SortPairs(t2.p, sb, nu.as<double>(), k2.as<double>(), i1.as<int64_t>(),
                                     i2.as<int64_t>(), nrec, 0, 64, s);
     const int gg = grid_for(ctx, nrec, 256);
@@ -556,12 +575,18 @@ int sort_lines(gexs_ctx* ctx, int64_t nrec, DevBuf& nu, DevBuf& el, DevBuf& A, D
     return e == cudaSuccess ? GEXS_OK : cuda_error(e, "ingest: sort");
 }
 
+/* scratch beyond 1 GiB goes back to the device after a parse */
+struct TrimPool {
+    gexs_ctx* ctx;
+    ~TrimPool() { if (ctx_pool(ctx)) cudaMemPoolTrimTo(ctx_pool(ctx), (size_t)1 << 30); }
+};
+
 /* records = non-empty lines, numbered in order: rec[i] for line i, *nrec */
 int number_records(gexs_ctx* ctx, const DevBuf& d_text, int64_t nbytes, const DevBuf& d_end,
                    int64_t nl, DevBuf& d_rec, int64_t* nrec, cudaStream_t s)
 {
     DevBuf d_flag, d_tmp;
-    if (d_flag.alloc(sizeof(int64_t) * (nl + 1)) != cudaSuccess || d_rec.alloc(sizeof(int64_t) * (nl + 1)) != cudaSuccess)
+    if (d_flag.scratch(ctx, sizeof(int64_t) * (nl + 1), s) != cudaSuccess || d_rec.scratch(ctx, sizeof(int64_t) * (nl + 1), s) != cudaSuccess)
         return set_error(GEXS_ERR_OOM, "ingest: record index");
     cudaMemsetAsync(d_flag.p, 0, sizeof(int64_t) * (nl + 1), s);
     if (nl > 0)
@@ -569,7 +594,7 @@ int number_records(gexs_ctx* ctx, const DevBuf& d_text, int64_t nbytes, const De
                                                                  d_end.as<int64_t>(), nl, d_flag.as<int64_t>());
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, d_flag.as<int64_t>(), d_rec.as<int64_t>(), (int)(nl + 1), s);
-    if (d_tmp.alloc(tb) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: scan");
+    if (d_tmp.scratch(ctx, tb, s) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: scan");
     cub::DeviceScan::ExclusiveSum(d_tmp.p, tb, d_flag.as<int64_t>(), d_rec.as<int64_t>(), (int)(nl + 1), s);
     cudaError_t e = cudaMemcpyAsync(nrec, d_rec.as<int64_t>() + nl, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -648,13 +673,14 @@ int gexs_exomol_parse_states(gexs_ctx* ctx, const char* h_text, int64_t nbytes,
     std::memset(out, 0, sizeof(*out));
     cudaSetDevice(ctx_device(ctx));
     cudaStream_t s = 0;
+    const TrimPool trim = {ctx};
     DevBuf d_text, d_end;
     int64_t nl = 0;
     int st = index_text(ctx, h_text, nbytes, d_text, d_end, &nl, s);
     if (st) return st;
     DevBuf dE, dg, dJ, derr;
     if (dE.alloc(sizeof(double) * nl) != cudaSuccess || dg.alloc(sizeof(int32_t) * nl) != cudaSuccess ||
-        dJ.alloc(sizeof(int32_t) * nl) != cudaSuccess || derr.alloc(sizeof(int)) != cudaSuccess)
+        dJ.alloc(sizeof(int32_t) * nl) != cudaSuccess || derr.scratch(ctx, sizeof(int), s) != cudaSuccess)
         return set_error(GEXS_ERR_OOM, "gexs_exomol_parse_states: tables");
     cudaMemsetAsync(derr.p, 0, sizeof(int), s);
     if (nl > 0)
@@ -686,13 +712,14 @@ int gexs_exomol_parse_trans(gexs_ctx* ctx, const gexs_state_table* states, const
     std::memset(out, 0, sizeof(*out));
     cudaSetDevice(ctx_device(ctx));
     cudaStream_t s = 0;
+    const TrimPool trim = {ctx};
     DevBuf d_text, d_end;
     int64_t nl = 0;
     int st = index_text(ctx, h_text, nbytes, d_text, d_end, &nl, s);
     if (st) return st;
     /* records: non-empty lines, numbered in order */
     DevBuf d_flag, d_rec, d_tmp;
-    if (d_flag.alloc(sizeof(int64_t) * (nl + 1)) != cudaSuccess || d_rec.alloc(sizeof(int64_t) * (nl + 1)) != cudaSuccess)
+    if (d_flag.scratch(ctx, sizeof(int64_t) * (nl + 1), s) != cudaSuccess || d_rec.scratch(ctx, sizeof(int64_t) * (nl + 1), s) != cudaSuccess)
         return set_error(GEXS_ERR_OOM, "gexs_exomol_parse_trans: record index");
     cudaMemsetAsync(d_flag.p, 0, sizeof(int64_t) * (nl + 1), s);
     if (nl > 0)
@@ -700,7 +727,7 @@ int gexs_exomol_parse_trans(gexs_ctx* ctx, const gexs_state_table* states, const
                                                                  d_end.as<int64_t>(), nl, d_flag.as<int64_t>());
     size_t tb = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tb, d_flag.as<int64_t>(), d_rec.as<int64_t>(), (int)(nl + 1), s);
-    if (d_tmp.alloc(tb) != cudaSuccess) return set_error(GEXS_ERR_OOM, "gexs_exomol_parse_trans: scan");
+    if (d_tmp.scratch(ctx, tb, s) != cudaSuccess) return set_error(GEXS_ERR_OOM, "gexs_exomol_parse_trans: scan");
     cub::DeviceScan::ExclusiveSum(d_tmp.p, tb, d_flag.as<int64_t>(), d_rec.as<int64_t>(), (int)(nl + 1), s);
     int64_t nrec = 0;
     cudaError_t e = cudaMemcpyAsync(&nrec, d_rec.as<int64_t>() + nl, sizeof(int64_t), cudaMemcpyDeviceToHost, s);
@@ -712,7 +739,7 @@ int gexs_exomol_parse_trans(gexs_ctx* ctx, const gexs_state_table* states, const
     if (broad_mode == GEXS_BROAD_BY_J && broad_nbytes > 0) parse_broadener(h_broad, broad_nbytes, bh);
     DevBuf dj0, dg0, dx0, dk1, dg1, dx1;
     auto up = [&](DevBuf& d, const void* h, size_t n) -> bool {
-        if (d.alloc(n) != cudaSuccess) return false;
+        if (d.scratch(ctx, n, s) != cudaSuccess) return false;
         return n == 0 || cudaMemcpyAsync(d.p, h, n, cudaMemcpyHostToDevice, s) == cudaSuccess;
     };
     if (!up(dj0, bh.j0.data(), bh.j0.size() * 4) || !up(dg0, bh.g0.data(), bh.g0.size() * 8) ||
@@ -728,7 +755,7 @@ int gexs_exomol_parse_trans(gexs_ctx* ctx, const gexs_state_table* states, const
     const size_t n8 = sizeof(double) * nrec, n4 = sizeof(int32_t) * nrec;
     if (nu.alloc(n8) != cudaSuccess || el.alloc(n8) != cudaSuccess || A.alloc(n8) != cudaSuccess ||
         g.alloc(n4) != cudaSuccess || gm.alloc(n8) != cudaSuccess || nx.alloc(n8) != cudaSuccess ||
-        derr.alloc(sizeof(int)) != cudaSuccess)
+        derr.scratch(ctx, sizeof(int), s) != cudaSuccess)
         return set_error(GEXS_ERR_OOM, "gexs_exomol_parse_trans: line arrays");
     cudaMemsetAsync(derr.p, 0, sizeof(int), s);
     if (nl > 0)

@@ -112,6 +112,13 @@ cudaMemPool_t ctx_pool(gexs_ctx* c);
  * out-of-memory the pool's unused pages are released and the call retried */
 cudaError_t pool_alloc(cudaMemPool_t pool, void** p, size_t bytes, cudaStream_t s);
 
+/* gexs_ctx_upload's worker (gexs_upload.cpp) */
+struct Uploader;
+Uploader* uploader_create(int device);
+void uploader_destroy(Uploader* u);
+cudaError_t upload(Uploader* u, const gexs_upload_piece* pieces, int n, cudaStream_t s);
+Uploader* ctx_uploader(gexs_ctx* c);
+
 /* error reporting (gexs_capi.cu): thread-local message, returns status */
 int set_error(int status, const std::string& msg);
 int cuda_error(cudaError_t e, const char* where);

@@ -167,22 +167,23 @@ void B200Manager::TransferVectors(size_t Nener, double* h_energies, double* h_nu
     const bool press = h_gamma && h_n && d_gam_ && d_n_;
     nchunks_ = Nener == 0 ? 0 : (Nener >= kSegmentMinLines ? kCopyChunks : 1);
     chunk_lines_ = nchunks_ ? (Nener + nchunks_ - 1) / nchunks_ : 0;
-    bool ok = true;
-    for (int c = 0; c < nchunks_ && ok; ++c) {
+    std::vector<gexs_upload_piece> pieces;
+    for (int c = 0; c < nchunks_; ++c) {
         const size_t i0 = std::min(Nener, (size_t)c * chunk_lines_);
         const size_t n = std::min(chunk_lines_, Nener - i0);
         const size_t d8 = sizeof(double) * n, d4 = sizeof(int) * n;
-        if (n) {
-            ok = cudaMemcpyAsync(d_nu_ + i0, h_nu + i0, d8, cudaMemcpyHostToDevice, cs) == cudaSuccess &&
-                 cudaMemcpyAsync(d_e_ + i0, h_energies + i0, d8, cudaMemcpyHostToDevice, cs) == cudaSuccess &&
-                 cudaMemcpyAsync(d_a_ + i0, h_aif + i0, d8, cudaMemcpyHostToDevice, cs) == cudaSuccess &&
-                 cudaMemcpyAsync(d_g_ + i0, h_gns + i0, d4, cudaMemcpyHostToDevice, cs) == cudaSuccess;
-            if (ok && press)
-                ok = cudaMemcpyAsync(d_gam_ + i0, h_gamma + i0, d8, cudaMemcpyHostToDevice, cs) == cudaSuccess &&
-                     cudaMemcpyAsync(d_n_ + i0, h_n + i0, d8, cudaMemcpyHostToDevice, cs) == cudaSuccess;
+        pieces.push_back({d_nu_ + i0, h_nu + i0, d8, nullptr});
+        pieces.push_back({d_e_ + i0, h_energies + i0, d8, nullptr});
+        pieces.push_back({d_a_ + i0, h_aif + i0, d8, nullptr});
+        pieces.push_back({d_g_ + i0, h_gns + i0, d4, nullptr});
+        if (press) {
+            pieces.push_back({d_gam_ + i0, h_gamma + i0, d8, nullptr});
+            pieces.push_back({d_n_ + i0, h_n + i0, d8, nullptr});
         }
-        if (ok) ok = cudaEventRecord((cudaEvent_t)chunk_ev_[c], cs) == cudaSuccess;
+        pieces.back().event = chunk_ev_[c];
     }
+    const bool ok = pieces.empty() ||
+                    gexs_ctx_upload(ctx_, pieces.data(), (int)pieces.size(), copy_stream_) == GEXS_OK;
     if (!ok) { fail(GEXS_ERR_CUDA); return; }
     /* nu at every stride-th line and at the last: conservative line bounds later */
     samp_idx_.clear(); samp_nu_.clear();

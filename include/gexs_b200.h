@@ -230,6 +230,20 @@ int gexs_run(gexs_ctx* ctx, const gexs_job* jobs, int njobs,
  * exchange on the device, so no flag raised meanwhile is lost. */
 int gexs_ctx_check(gexs_ctx* ctx, void* stream);
 
+/* Copy host arrays to the device, in order, on `stream`; after a piece its
+ * `event` (a cudaEvent_t, or NULL) is recorded there.  Pageable sources go
+ * through a ring of pinned buffers that several host threads fill (8 MiB
+ * per process, allocated by the first call of 4 MiB or more, freed with the
+ * last context) and have been read when the call returns; pinned sources are copied directly and must
+ * stay valid until the stream has passed the copy. */
+typedef struct gexs_upload_piece {
+    void*       dst;      /* device */
+    const void* src;      /* host   */
+    size_t      bytes;
+    void*       event;
+} gexs_upload_piece;
+int gexs_ctx_upload(gexs_ctx* ctx, const gexs_upload_piece* pieces, int n, void* stream);
+
 /* Exact number of (line, bin) profile evaluations of each job (the window
  * rule applied to every line): counts[i] for jobs[i]. Synchronous. */
 int gexs_count_evals(gexs_ctx* ctx, const gexs_job* jobs, int njobs,

@@ -1,0 +1,72 @@
+"""gexs_ctx_upload: bytes arrive unchanged from pageable and pinned sources, at
+sizes around a slot (0.5 MiB), the staging threshold (4 MiB) and the ring (8
+MiB), with empty and odd pieces; a pageable source may be overwritten as soon
+as the call returns; calls from several threads on one context."""
+import ctypes as C
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+from gexs_b200._capi import check, lib
+
+pytestmark = pytest.mark.gpu
+
+MIB = 1 << 20
+
+
+class Piece(C.Structure):
+    _fields_ = [("dst", C.c_void_p), ("src", C.c_void_p), ("bytes", C.c_size_t),
+                ("event", C.c_void_p)]
+
+
+def _upload(ctx, arrays, stream):
+    dev = [torch.zeros(max(a.size, 1), dtype=torch.uint8, device="cuda") for a in arrays]
+    p = (Piece * len(arrays))()
+    for i, (d, a) in enumerate(zip(dev, arrays)):
+        p[i] = Piece(d.data_ptr(), a.ctypes.data, a.size, None)
+    torch.cuda.synchronize()
+    check(lib().gexs_ctx_upload(ctx.h, p, len(arrays), C.c_void_p(stream.cuda_stream)), "upload")
+    return dev
+
+
+@pytest.mark.parametrize("sizes", [
+    [0, 1, 7], [4 * MIB - 1], [4 * MIB], [MIB, MIB + 1, 3 * MIB - 1], [16 * MIB + 5, 0, 3],
+    [53 * MIB + 11, 1, 17 * MIB]])
+def test_bytes_arrive(gpu_ctx, sizes):
+    rng = np.random.Generator(np.random.PCG64(len(sizes)))
+    want = [rng.integers(0, 256, n, dtype=np.uint8) for n in sizes]
+    stream = torch.cuda.Stream()
+    src = [w.copy() for w in want]
+    dev = _upload(gpu_ctx, src, stream)
+    for s in src:
+        s[:] = 0                      # pageable: already read
+    stream.synchronize()
+    pinned = [torch.from_numpy(w).pin_memory() if w.size else torch.empty(0, dtype=torch.uint8)
+              for w in want]
+    half = [p.numpy() if i % 2 == 0 else w for i, (p, w) in enumerate(zip(pinned, want))]
+    dev2 = _upload(gpu_ctx, half, stream)
+    stream.synchronize()
+    for d, d2, w in zip(dev, dev2, want):
+        assert np.array_equal(d.cpu().numpy()[:w.size], w)
+        assert np.array_equal(d2.cpu().numpy()[:w.size], w)
+
+
+def test_threads_share_a_context(gpu_ctx):
+    rng = np.random.Generator(np.random.PCG64(9))
+    want = [rng.integers(0, 256, 9 * MIB + k, dtype=np.uint8) for k in range(4)]
+    got = [None] * 4
+
+    def one(k):
+        s = torch.cuda.Stream()
+        got[k] = _upload(gpu_ctx, [want[k]], s)[0]
+        s.synchronize()
+
+    th = [threading.Thread(target=one, args=(k,)) for k in range(4)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    for g, w in zip(got, want):
+        assert np.array_equal(g.cpu().numpy()[:w.size], w)
