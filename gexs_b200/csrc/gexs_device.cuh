@@ -256,18 +256,31 @@ __host__ __device__ __forceinline__ constexpr double gh_w(int k)
     return NODES == 16 ? w16[k] : w32[k];
 }
 
-template <int NODES>
-__device__ __forceinline__ float gh_sum_f32(float x, float y2)
+/* FP32, NP pairs of bins on packed f32x2 instructions, nodes outermost so
+ * that a node's constants serve every pair: eight packed instructions and
+ * two MUFU reciprocals per pair and node pair.  Both pipes then need 16
+ * cycles of a scheduler per warp; one bin at a time took 16 + 2 issues.
+ * Every rounding is that of the scalar sum w (A + B) * rcp(A B). */
+template <int NODES, int NP>
+__device__ __forceinline__ void gh_sum2_f32(const float2 (&x)[NP], float y2, float2 (&acc)[NP])
 {
-    float acc = 0.f;
+    const float2 yy = make_float2(y2, y2);
+#pragma unroll
+    for (int j = 0; j < NP; ++j) acc[j] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < GH<NODES>::NP; ++k) {
-        float t = (float)gh_t<NODES>(k), w = (float)gh_w<NODES>(k);
-        float d1 = x - t, d2 = x + t;
-        float A = fmaf(d1, d1, y2), B = fmaf(d2, d2, y2);
-        acc = fmaf(w * (A + B), rcp_approx(A * B), acc);
+        const float t = (float)gh_t<NODES>(k), w = (float)gh_w<NODES>(k);
+        const float2 tp = make_float2(t, t), tm = make_float2(-t, -t), ww = make_float2(w, w);
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            const float2 d1 = __fadd2_rn(x[j], tm), d2 = __fadd2_rn(x[j], tp);
+            const float2 A = __ffma2_rn(d1, d1, yy), B = __ffma2_rn(d2, d2, yy);
+            const float2 D = __fmul2_rn(A, B);
+            float2 r;
+            r.x = rcp_approx(D.x); r.y = rcp_approx(D.y);
+            acc[j] = __ffma2_rn(__fmul2_rn(ww, __fadd2_rn(A, B)), r, acc[j]);
+        }
     }
-    return acc;
 }
 
 /* Lines much narrower than a node spacing (y < 1/8): near a node t_k the
@@ -276,21 +289,31 @@ __device__ __forceinline__ float gh_sum_f32(float x, float y2)
  * about 1e-7 x / |x - t_k| on it.  Here x is the unevaluated pair xs + xl
  * (x_pair below, error ~1e-13) and x - t_k is taken against the node split
  * the same way, so every difference keeps its relative accuracy. */
-template <int NODES>
-__device__ __forceinline__ float gh_sum_f32_pair(float xs, float xl, float y2)
+template <int NODES, int NP>
+__device__ __forceinline__ void gh_sum2_f32_pair(const float2 (&xs)[NP], const float2 (&xl)[NP],
+                                                 float y2, float2 (&acc)[NP])
 {
-    float acc = 0.f;
+    const float2 yy = make_float2(y2, y2);
+#pragma unroll
+    for (int j = 0; j < NP; ++j) acc[j] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < GH<NODES>::NP; ++k) {
         const double tk = gh_t<NODES>(k);
         const float th = (float)tk, tl = (float)(tk - (double)th), w = (float)gh_w<NODES>(k);
-        /* xs - th is exact when xs is within a factor 2 of th (Sterbenz) */
-        const float d1 = __fadd_rn(__fsub_rn(xs, th), __fsub_rn(xl, tl));
-        const float d2 = __fadd_rn(xs, th);
-        const float A = fmaf(d1, d1, y2), B = fmaf(d2, d2, y2);
-        acc = fmaf(w * (A + B), rcp_approx(A * B), acc);
+        const float2 tp = make_float2(th, th), tm = make_float2(-th, -th);
+        const float2 lm = make_float2(-tl, -tl), ww = make_float2(w, w);
+#pragma unroll
+        for (int j = 0; j < NP; ++j) {
+            /* xs - th is exact when xs is within a factor 2 of th (Sterbenz) */
+            const float2 d1 = __fadd2_rn(__fadd2_rn(xs[j], tm), __fadd2_rn(xl[j], lm));
+            const float2 d2 = __fadd2_rn(xs[j], tp);
+            const float2 A = __ffma2_rn(d1, d1, yy), B = __ffma2_rn(d2, d2, yy);
+            const float2 D = __fmul2_rn(A, B);
+            float2 r;
+            r.x = rcp_approx(D.x); r.y = rcp_approx(D.y);
+            acc[j] = __ffma2_rn(__fmul2_rn(ww, __fadd2_rn(A, B)), r, acc[j]);
+        }
     }
-    return acc;
 }
 
 /* x = (n - fc) dx as the pair xs + xl from n (an exact integer in float),

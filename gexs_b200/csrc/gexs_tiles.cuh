@@ -636,43 +636,62 @@ __device__ __forceinline__ void lines_f32(const RecF32* __restrict__ rec, int nr
             const float4 q1 = *reinterpret_cast<const float4*>(&rec[i].p);     /* p y amp fc */
             const float ncf = wbf - q0.x;
             constexpr int NODES = (PK == PK_GH16) ? 16 : 32;
+            const int a = lo16(qi.x);
+            const unsigned wn = (unsigned)(hi16(qi.x) - a);
+            const float t0 = lanef + ncf;
+            /* bins outside the window are evaluated and dropped */
+            const bool full = mask & ((bit << 8) | (bit << 16));
+            const float2 aa = make_float2(q0.w, q0.w);
+            auto add = [&](const float2 (&g)[B / 2]) {
+#pragma unroll
+                for (int j = 0; j < B / 2; ++j) {
+                    const int t = wb + lane + 64 * j;
+                    const float2 v = __ffma2_rn(aa, g[j], part[j]);
+                    if (full || (unsigned)(t - a) < wn) part[j].x = v.x;
+                    if (full || (unsigned)(t + 32 - a) < wn) part[j].y = v.y;
+                }
+            };
             if (mask & GH_PAIR_BIT) {
-                /* narrow line: x as a float pair, per-bin window test */
-                const int a = lo16(qi.x), b = hi16(qi.x);
-                const float t0 = lanef + ncf;
+                /* narrow line: x as a float pair */
+                float2 xs[B / 2], xl[B / 2], g[B / 2];
+#pragma unroll
+                for (int j = 0; j < B / 2; ++j) {
+                    x_pair(t0 + (float)(64 * j), q0.y, q1.y, q0.z, q1.z, xs[j].x, xl[j].x);
+                    x_pair(t0 + (float)(64 * j + 32), q0.y, q1.y, q0.z, q1.z, xs[j].y, xl[j].y);
+                }
+                gh_sum2_f32_pair<NODES, B / 2>(xs, xl, q1.x, g);
+                add(g);
+                continue;
+            }
+            if ((mask >> 24) & 1) {
+                /* |x| may exceed 1e8 */
 #pragma unroll
                 for (int k = 0; k < B; ++k) {
                     const int t = wb + lane + 32 * k;
-                    if (t < a || t >= b) continue;
-                    float xs, xl;
-                    x_pair(t0 + (float)(32 * k), q0.y, q1.y, q0.z, q1.z, xs, xl);
+                    if ((unsigned)(t - a) >= wn) continue;
+                    const float x = fabsf(((t0 + (float)(32 * k)) - q1.w) * q0.y);
                     float& acc = bin_acc<B>(part, k);
-                    acc = fmaf(q0.w, gh_sum_f32_pair<NODES>(xs, xl, q1.x), acc);
+                    acc = fmaf(q0.w, gh_sum_f32_wide<NODES>(x, q1.x), acc);
                 }
                 continue;
             }
+            float2 x[B / 2], g[B / 2];
             if (mask & (bit << 8)) {
                 const float x0 = fmaf(lanef, q0.y, fmaf(ncf, q0.y, q0.z));
 #pragma unroll
-                for (int k = 0; k < B; ++k) {
-                    float& acc = bin_acc<B>(part, k);
-                    acc = fmaf(q0.w, gh_sum_f32<NODES>(fabsf(fmaf((float)(32 * k), q0.y, x0)), q1.x),
-                               acc);
+                for (int j = 0; j < B / 2; ++j) {
+                    x[j].x = fabsf(fmaf((float)(64 * j), q0.y, x0));
+                    x[j].y = fabsf(fmaf((float)(64 * j + 32), q0.y, x0));
                 }
-                continue;
-            }
-            const int a = lo16(qi.x), b = hi16(qi.x);
-            const bool wide = (mask >> 24) & 1;
-            const float t0 = lanef + ncf;
+            } else {
 #pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const int t = wb + lane + 32 * k;
-                if (t < a || t >= b) continue;
-                const float x = fabsf(((t0 + (float)(32 * k)) - q1.w) * q0.y);
-                const float g = wide ? gh_sum_f32_wide<NODES>(x, q1.x) : gh_sum_f32<NODES>(x, q1.x);
-                float& acc = bin_acc<B>(part, k);
-                acc = fmaf(q0.w, g, acc);
+                for (int j = 0; j < B / 2; ++j) {
+                    x[j].x = fabsf(__fmul_rn(__fsub_rn(t0 + (float)(64 * j), q1.w), q0.y));
+                    x[j].y = fabsf(__fmul_rn(__fsub_rn(t0 + (float)(64 * j + 32), q1.w), q0.y));
+                }
             }
+            gh_sum2_f32<NODES, B / 2>(x, q1.x, g);
+            add(g);
         }
     }
 }
