@@ -238,6 +238,7 @@ struct Layout {
     size_t os_prefix = 0, os_counts = 0, os_rowbase = 0, os_ticket = 0, os_lohi = 0, os_nitems = 0,
            os_rows = 0;
     int max_rows = 0;
+    bool split = false;
     long long lines_per_slice = 0;
     /* the core kernel's slice tables */
     bool csliced = false;
@@ -267,6 +268,7 @@ static Layout group_layout(const Group& g, bool prep, const gexs_launch_cfg& cfg
     if (slices_apply(g.pk, g.prec) && nt > 0) {
         L.sliced = true;
         L.lines_per_slice = slice_lines(g.jobs.data(), (int)g.jobs.size(), g.prec, W, &L.max_rows);
+        L.split = g.pk == PK_ERF_CLASS && erf_split(g.jobs.data(), (int)g.jobs.size(), W);
         L.os_prefix = up(a); a = L.os_prefix + (nt + 1) * sizeof(int);
         L.os_counts = up(a); a = L.os_counts + nt * sizeof(int);
         L.os_rowbase = up(a); a = L.os_rowbase + nt * sizeof(int);
@@ -336,6 +338,7 @@ static cudaError_t enqueue_group(const Group& g, const Layout& L, unsigned char*
         sl.rows = (double*)(d + L.os_rows);
         sl.max_rows = L.max_rows;
         sl.lines_per_slice = L.lines_per_slice;
+        sl.split = L.split ? 1 : 0;
     }
     SliceTables csl;
     std::memset(&csl, 0, sizeof(csl));

@@ -324,19 +324,36 @@ static double tile_entries(const gexs_job& j, double reach, int tile_w)
 
 static const double kMaxRowBytes = (double)(1ull << 30);
 
+/* reach_range's reach at the job's highest frequency */
+static double scatter_reach(const gexs_job& j)
+{
+    const double z = j.profile == GEXS_VOIGT ? 15.0 : ERF_Z64, k = z * j.dop_coef;
+    const double nu_hi = j.nu_start + (double)(j.start_idx + j.n_points) * j.dnu + j.cutoff;
+    double reach = j.cutoff;
+    if (j.profile == GEXS_GAUSSIAN) reach = std::min(reach, z / j.inv_width);
+    else if (k < 1.0) reach = std::min(reach, (nu_hi + j.dnu) * k / (1.0 - k));
+    return reach;
+}
+
+bool erf_split(const gexs_job* jobs, int njobs, int tile_w)
+{
+    /* a part repeats its tile's item set-up and some of its lines: worth it
+     * where tiles are dense, or few and not nearly empty */
+    double lines = 0.0, tiles = 0.0;
+    for (int i = 0; i < njobs; ++i) {
+        lines += tile_entries(jobs[i], scatter_reach(jobs[i]), tile_w);
+        tiles += std::ceil((double)jobs[i].n_points / (double)tile_w);
+    }
+    return tiles < 1e8 && lines >= (tiles < 1184.0 ? 128.0 : 1024.0) * tiles;
+}
+
 int core_cut_shift(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows)
 {
-    /* a line's reach is reach_range's at the job's highest frequency */
     for (int shift = 0; shift < 40; ++shift) {
         double rows = 0.0;
         for (int i = 0; i < njobs; ++i) {
             const gexs_job& j = jobs[i];
-            const double z = j.profile == GEXS_VOIGT ? 15.0 : ERF_Z64, k = z * j.dop_coef;
-            const double nu_hi = j.nu_start + (double)(j.start_idx + j.n_points) * j.dnu + j.cutoff;
-            double reach = j.cutoff;
-            if (j.profile == GEXS_GAUSSIAN) reach = std::min(reach, z / j.inv_width);
-            else if (k < 1.0) reach = std::min(reach, (nu_hi + j.dnu) * k / (1.0 - k));
-            rows += row_bound(j, tile_entries(j, reach, tile_w), tile_w,
+            rows += row_bound(j, tile_entries(j, scatter_reach(j), tile_w), tile_w,
                               (double)core_cut(j.grid_points, tile_w, shift));
         }
         if (rows * row_doubles(prec, tile_w) * sizeof(double) <= kMaxRowBytes) {

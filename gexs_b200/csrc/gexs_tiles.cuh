@@ -53,9 +53,10 @@ struct __align__(16) RecF32 {   /* 48 bytes; Doppler/Gaussian and GH */
     float y;               /* GH: y ; Doppler: half bin in x units           */
     float amp;             /* GH: S*invw*out_scale ; Doppler: S*out_scale    */
     float fc;              /* tc - floor(tc) in [0, 1)                       */
-    int   win;             /* a | b << 16 : bins [a, b) of the tile          */
-    int   c1;              /* Doppler: bins whose xm <= the zero threshold   */
-    int   mask;            /* per warp w: bit w touches, bit 8+w fast tier,
+    int   win;             /* a | b << 16 : bins [a, b) of the tile; Doppler:
+                              those whose xm <= the zero threshold           */
+    int   c1;
+    int   mask;            /* GH, per warp w: bit w touches, bit 8+w fast tier,
                               bit 16+w mid tier; bit 24: |x| may exceed 1e8
                               in this tile (overflow-free forms); bit 25 (GH):
                               y < 1/8, x as a float pair (gh_sum_f32_pair)   */
@@ -423,17 +424,14 @@ template <int PK, int B, int WARPS>
 __device__ __forceinline__ int warp_mask(const Derived<PK>& d, int wide)
 {
     const int a = lo16(d.win), b = hi16(d.win);
-    const int c1a = lo16(d.c1), c1b = hi16(d.c1);
     const int ic = (int)fmin(fmax(floor(d.tc), -1e6), 1e6);
     int m = 0;
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) {
         const int r0 = 32 * B * w, r1 = r0 + 32 * B;
-        bool touch = a < r1 && b > r0;
-        if (PK == PK_ERF) touch = touch && c1a < r1 && c1b > r0 && c1a < c1b;
-        if (!touch) continue;
+        if (!(a < r1 && b > r0)) continue;
         m |= 1 << w;
-        if (PK == PK_ERF || wide) continue;
+        if (wide) continue;
         if (!(a <= r0 && b >= r1)) continue;
         /* GH: the single-FMA x of its fast tier keeps ~1e-7 relative
          * accuracy only when the centre is at least a warp span away */
@@ -472,11 +470,16 @@ __device__ __forceinline__ void make_rec(RecF32& q, const Derived<PK>& d, const 
         pair = d.y < 0.125;
     }
     q.fc = fc;
-    q.win = d.win; q.c1 = d.c1;
-    /* largest |x| the line reaches in this tile */
-    double dfar = fmax(fabs(d.nu - T.f0), fabs(d.nu - T.fl));
-    const int wide = (dfar * d.invw > 1e8) ? 1 : 0;
-    q.mask = (d.win == 0) ? 0 : (warp_mask<PK, B, WARPS>(d, wide) | (pair && !wide ? GH_PAIR_BIT : 0));
+    /* erf: the non-zero bins, a sub-range of the window */
+    q.win = PK == PK_ERF ? (d.win == 0 ? 0 : d.c1) : d.win;
+    q.c1 = 0;
+    q.mask = 0;
+    if constexpr (PK != PK_ERF) {
+        /* largest |x| the line reaches in this tile */
+        double dfar = fmax(fabs(d.nu - T.f0), fabs(d.nu - T.fl));
+        const int wide = (dfar * d.invw > 1e8) ? 1 : 0;
+        if (d.win != 0) q.mask = warp_mask<PK, B, WARPS>(d, wide) | (pair && !wide ? GH_PAIR_BIT : 0);
+    }
     q.pad = 0;
 }
 
@@ -593,33 +596,52 @@ __device__ __forceinline__ float& bin_acc(float2 (&part)[B / 2], int k)
  * GH fast tier: whole warp in the window, centre >= one warp span away:
  *   x_k = fma(32k, dx, fma(l, dx, q)); otherwise per-bin window tests and
  *   x = ((l+32k + wb-ic) - fc)*dx exactly. */
-template <int PK, int B>
-__device__ __forceinline__ void lines_f32(const RecF32* __restrict__ rec, int nrec, int warp,
-                                          int lane, float2 (&part)[B / 2])
+/* Bins of a lane: 32 B consecutive ones per warp, or for the erf profiles
+ * 32-bin chunks dealt to the warps in turn (a line reaches a few chunks
+ * only; with consecutive bins one warp at a time would have work).
+ * SPLIT: an item is one of the B parts of a tile (of a slice of a tile),
+ * the 32 WARPS bins at k = part, with its own, shorter line range; a dense
+ * tile, or a job of few tiles, is then several items.  Lines are derived
+ * for the whole tile and summed in the whole tile's groups, and a bin's sum
+ * does not depend on the lane that takes it: both forms give the same bits.
+ * 3e6 lines on 990,001 bins: 1.4 ms split, 2.0 ms not (the densest tiles
+ * ran on alone); 700 lines on 495,001 bins: 26 us split, 16 us not. */
+template <int PK, int B, int WARPS>
+__device__ __forceinline__ int tile_bin(int warp, int lane, int k)
 {
-    const int wb = warp * 32 * B;
-    const float wbf = (float)wb, lanef = (float)lane;
-    const int bit = 1 << warp;
+    return (PK == PK_ERF ? 32 * (warp + WARPS * k) : 32 * (warp * B + k)) + lane;
+}
+
+/* bins k = k0 .. k0 + KB - 1 of each lane (all B but for split erf tiles) */
+template <int PK, int B, int WARPS, int KB>
+__device__ __forceinline__ void lines_f32(const RecF32* __restrict__ rec, int nrec, int warp,
+                                          int lane, int k0, float2 (&part)[B / 2])
+{
     if constexpr (PK == PK_ERF) {
-        /* a line touches few warps of its tile: the records that touch this
-         * one, 32 at a time, in order */
+        /* the records that touch one of this warp's chunks, 32 at a time, in
+         * order; win holds the line's non-zero bins [a, b) */
+        const int w0 = warp + WARPS * k0;                  /* first chunk */
         for (int i0 = 0; i0 < nrec; i0 += 32) {
-            unsigned todo = __ballot_sync(0xffffffffu,
-                                          i0 + lane < nrec && (rec[min(i0 + lane, nrec - 1)].mask & bit));
+            const int mine = rec[min(i0 + lane, nrec - 1)].win;
+            const int f = lo16(mine) >> 5, l = (hi16(mine) + 31) >> 5;      /* chunks [f, l) */
+            bool touch = i0 + lane < nrec && hi16(mine) > lo16(mine);
+            if (KB == 1) touch = touch && w0 >= f && w0 < l;
+            else touch = touch && ((unsigned)(warp - f) & (WARPS - 1)) < (unsigned)(l - f);
+            unsigned todo = __ballot_sync(0xffffffffu, touch);
             while (todo) {
                 const int i = i0 + __ffs(todo) - 1;
                 todo &= todo - 1;
-                const int4 qi = *reinterpret_cast<const int4*>(&rec[i].win);   /* win c1 mask pad */
+                const int win = rec[i].win;
                 const float4 q0 = *reinterpret_cast<const float4*>(&rec[i].icf);   /* icf dx mfcdx a1 */
                 const float4 q1 = *reinterpret_cast<const float4*>(&rec[i].p);     /* p y amp fc */
-                const int a = lo16(qi.x), b = hi16(qi.x);
-                const int c1a = lo16(qi.y), c1b = hi16(qi.y);
-                const float t0 = lanef + (wbf - q0.x);
+                const int a = lo16(win), b = hi16(win);
 #pragma unroll
-                for (int k = 0; k < B; ++k) {
-                    const int t = wb + lane + 32 * k;
-                    if (t < a || t >= b || t < c1a || t >= c1b) continue;
-                    const float xd = fabsf(((t0 + (float)(32 * k)) - q1.w) * q0.y);
+                for (int k = 0; k < KB; ++k) {
+                    const int c = 32 * (w0 + WARPS * k), t = c + lane;
+                    if (KB > 1 && (c + 32 <= a || c >= b)) continue;   /* warp-uniform */
+                    if (t < a || t >= b) continue;
+                    const float t0 = (float)t - q0.x;                  /* exact integers */
+                    const float xd = fabsf((t0 - q1.w) * q0.y);
                     /* FP32 always takes the cancellation-free form: the literal
                      * erf difference loses ~1e-7 absolute in FP32 far wings */
                     float& acc = bin_acc<B>(part, k);
@@ -628,6 +650,9 @@ __device__ __forceinline__ void lines_f32(const RecF32* __restrict__ rec, int nr
             }
         }
     } else {
+        const int wb = warp * 32 * B;
+        const float wbf = (float)wb, lanef = (float)lane;
+        const int bit = 1 << warp;
         for (int i = 0; i < nrec; ++i) {
             const int4 qi = *reinterpret_cast<const int4*>(&rec[i].win);   /* win c1 mask pad */
             const int mask = qi.z;
@@ -1089,7 +1114,7 @@ constexpr int min_ctas()
     return WARPS == 8 ? (B >= 8 ? 2 : 3) : (B >= 8 ? 4 : 6);
 }
 
-template <int PK, int PREC, int B, int WARPS, bool PREP>
+template <int PK, int PREC, int B, int WARPS, bool PREP, bool SPLIT = false>
 __global__ void __launch_bounds__(WARPS * 32, min_ctas<B, WARPS, PREC>())
 tile_kernel(const KArgs args)
 {
@@ -1121,7 +1146,9 @@ tile_kernel(const KArgs args)
     for (;;) {
         if (tid == 0) s_item = atomicAdd(args.counter, 1);
         __syncthreads();
-        const int item = s_item;
+        /* Q items a tile, of KB bins a lane from k0 */
+        constexpr int Q = SPLIT ? B : 1, KB = B / Q;
+        const int item = s_item / Q, k0 = s_item % Q;
         if (item >= nitems) break;
         /* item -> (tile, slice): one item per tile unless sliced */
         int ti = item, sidx = 0, ns = 1;
@@ -1171,10 +1198,15 @@ tile_kernel(const KArgs args)
         }
         if constexpr (PK == PK_ERF) {
             if (warp >= 2 && warp < 4) {
-                double vlo, vhi;
-                reach_range(J, T.f0, T.fl, vlo, vhi);
-                const int64_t v = warp == 2 ? warp_bound<false>(J.lines.nu, nl, vlo, lane)
-                                            : warp_bound<true>(J.lines.nu, nl, vhi, lane);
+                const int b0 = 32 * WARPS * k0, b1 = min(b0 + 32 * WARPS * KB, T.jn);
+                int64_t v = 0;                      /* a part past the grid's end: no lines */
+                if (b0 < b1) {
+                    double vlo, vhi;
+                    reach_range(J, grid_f(J.nu_start, J.dnu, T.j0 + b0),
+                                grid_f(J.nu_start, J.dnu, T.j0 + b1 - 1), vlo, vhi);
+                    v = warp == 2 ? warp_bound<false>(J.lines.nu, nl, vlo, lane)
+                                  : warp_bound<true>(J.lines.nu, nl, vhi, lane);
+                }
                 if (lane == 0) s_near[warp - 2] = v;
             }
         }
@@ -1183,7 +1215,7 @@ tile_kernel(const KArgs args)
         const int64_t hi = max((int64_t)s_lohi[1], lo);
         const int nph = (int)((hi - lo + R - 1) / R);
         /* phases to run: all, or for the erf profiles those that hold a line
-         * whose non-zero bins can reach the tile (of the lines within the
+         * whose non-zero bins can reach the item (of the lines within the
          * cutoff about a tenth at 0.01 cm^-1 and 1500 K).  Phases stay those
          * of the whole range: a skipped one would add zeros, so the FP32
          * sums are the same bits. */
@@ -1200,16 +1232,16 @@ tile_kernel(const KArgs args)
             __syncthreads();
         } else {
 #pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const int t = warp * 32 * B + lane + 32 * k;
+            for (int k = 0; k < KB; ++k) {
+                const int t = tile_bin<PK, B, WARPS>(warp, lane, k0 + k);
                 s_hi[t] = 0.0; s_lo[t] = 0.0;
             }
         }
         /* the end of a line block: its sums into the (hi, lo) pairs */
         auto end_block = [&](double (&acc)[B]) {
 #pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const int t = warp * 32 * B + lane + 32 * k;
+            for (int k = 0; k < KB; ++k) {
+                const int t = tile_bin<PK, B, WARPS>(warp, lane, k0 + k);
                 dd_add(s_hi[t], s_lo[t], acc[k]);
                 acc[k] = 0.0;
             }
@@ -1218,9 +1250,9 @@ tile_kernel(const KArgs args)
         float2 part[B / 2];
         double acc[B], fbin[B];
 #pragma unroll
-        for (int k = 0; k < B; ++k) {
+        for (int k = 0; k < KB; ++k) {
             acc[k] = 0.0;
-            if (PREC == GEXS_FP64) fbin[k] = grid_f(J.nu_start, J.dnu, T.j0 + warp * 32 * B + lane + 32 * k);
+            if (PREC == GEXS_FP64) fbin[k] = grid_f(J.nu_start, J.dnu, T.j0 + tile_bin<PK, B, WARPS>(warp, lane, k0 + k));
         }
 #pragma unroll
         for (int j = 0; j < B / 2; ++j) part[j] = make_float2(0.f, 0.f);
@@ -1291,11 +1323,11 @@ tile_kernel(const KArgs args)
                 /* Kahan merge of FP32 partial sums every 128 lines */
                 for (int c0 = 0; c0 < nrec; c0 += 128) {
                     const int cn = min(128, nrec - c0);
-                    lines_f32<PK, B>(reinterpret_cast<const RecF32*>(s_rec) + c0, cn, warp,
-                                     lane, part);
+                    lines_f32<PK, B, WARPS, KB>(reinterpret_cast<const RecF32*>(s_rec) + c0, cn, warp,
+                                            lane, k0, part);
 #pragma unroll
-                    for (int k = 0; k < B; ++k) {
-                        const int t = warp * 32 * B + lane + 32 * k;
+                    for (int k = 0; k < KB; ++k) {
+                        const int t = tile_bin<PK, B, WARPS>(warp, lane, k0 + k);
                         float ks = s_ks[t], kc = s_kc[t];
                         kahan_add(ks, kc, bin_acc<B>(part, k));
                         s_ks[t] = ks; s_kc[t] = kc;
@@ -1329,8 +1361,8 @@ tile_kernel(const KArgs args)
         auto hi_of = [&](int t) { return DD ? s_hi[t] : (double)s_ks[t] - (double)s_kc[t]; };
         if (ns == 1) {
 #pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const int t = warp * 32 * B + lane + 32 * k;
+            for (int k = 0; k < KB; ++k) {
+                const int t = tile_bin<PK, B, WARPS>(warp, lane, k0 + k);
                 if (t < T.jn) {
                     const double v = DD ? s_hi[t] + s_lo[t] : hi_of(t);
                     int64_t j = T.j0 + t;
@@ -1344,8 +1376,8 @@ tile_kernel(const KArgs args)
             const int rb = args.sl.rowbase[ti];
             double* row = args.sl.rows + (size_t)(rb + sidx) * RS;
 #pragma unroll
-            for (int k = 0; k < B; ++k) {
-                const int t = warp * 32 * B + lane + 32 * k;
+            for (int k = 0; k < KB; ++k) {
+                const int t = tile_bin<PK, B, WARPS>(warp, lane, k0 + k);
                 if (t < T.jn) {
                     row[t] = hi_of(t);
                     if (DD) row[W + t] = s_lo[t];
@@ -1353,24 +1385,20 @@ tile_kernel(const KArgs args)
             }
             __threadfence();
             __syncthreads();
-            if (tid == 0) s_last = atomicAdd(args.sl.ticket + ti, 1) == ns - 1;
+            if (tid == 0) s_last = atomicAdd(args.sl.ticket + ti, 1) == ns * Q - 1;
             __syncthreads();
             if (s_last) {
                 __threadfence();
-#pragma unroll
-                for (int k = 0; k < B; ++k) {
-                    const int t = warp * 32 * B + lane + 32 * k;
-                    if (t < T.jn) {
-                        double hi = 0.0, lo = 0.0;
-                        for (int q = 0; q < ns; ++q) {
-                            const double* r = args.sl.rows + (size_t)(rb + q) * RS + t;
-                            if (DD) { dd_add(hi, lo, __ldcg(r)); lo = dadd(lo, __ldcg(r + W)); }
-                            else hi += __ldcg(r);
-                        }
-                        const double v = DD ? hi + lo : hi;
-                        int64_t j = T.j0 + t;
-                        out[j] = acc_mode ? out[j] + v : v;
+                for (int t = tid; t < T.jn; t += NT) {
+                    double hi = 0.0, lo = 0.0;
+                    for (int q = 0; q < ns; ++q) {
+                        const double* r = args.sl.rows + (size_t)(rb + q) * RS + t;
+                        if (DD) { dd_add(hi, lo, __ldcg(r)); lo = dadd(lo, __ldcg(r + W)); }
+                        else hi += __ldcg(r);
                     }
+                    const double v = DD ? hi + lo : hi;
+                    int64_t j = T.j0 + t;
+                    out[j] = acc_mode ? out[j] + v : v;
                 }
             }
         }
@@ -2236,6 +2264,8 @@ template <int PK, int PREC, int B, int WARPS, bool PREP>
 static cudaError_t launch_one(const KArgs& a, int ctas_per_sm, int nsm, cudaStream_t st)
 {
     auto kern = tile_kernel<PK, PREC, B, WARPS, PREP>;
+    if constexpr (PK == PK_ERF)
+        if (a.sl.prefix && a.sl.split) kern = tile_kernel<PK, PREC, B, WARPS, PREP, true>;
     const size_t smem = Smem<PK, PREC, B, WARPS, PREP>::bytes;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
