@@ -268,7 +268,10 @@ static Layout group_layout(const Group& g, bool prep, const gexs_launch_cfg& cfg
     if (slices_apply(g.pk, g.prec) && nt > 0) {
         L.sliced = true;
         L.lines_per_slice = slice_lines(g.jobs.data(), (int)g.jobs.size(), g.prec, W, &L.max_rows);
-        L.split = g.pk == PK_ERF_CLASS && erf_split(g.jobs.data(), (int)g.jobs.size(), W);
+        if (g.prec == GEXS_FP32 && g.pk == PK_ERF_CLASS)
+            L.split = erf_split(g.jobs.data(), (int)g.jobs.size(), W);
+        if (g.prec == GEXS_FP32 && g.pk == PK_VOIGT_CLASS)
+            L.split = ws_split(g.jobs.data(), (int)g.jobs.size(), W);
         L.os_prefix = up(a); a = L.os_prefix + (nt + 1) * sizeof(int);
         L.os_counts = up(a); a = L.os_counts + nt * sizeof(int);
         L.os_rowbase = up(a); a = L.os_rowbase + nt * sizeof(int);

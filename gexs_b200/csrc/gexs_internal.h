@@ -30,7 +30,7 @@ struct SliceTables {
     int        max_rows;
     long long  lines_per_slice;
     int        cut_shift;   /* core kernel: see core_cut                    */
-    int        split;       /* FP32 erf tiles: items of parts of a tile     */
+    int        split;       /* FP32 erf, Voigt: items are parts of a tile   */
 };
 
 /* One set-up launch (prep arrays, slice tables) where there is any to do,
@@ -77,8 +77,10 @@ __host__ __device__ inline long long core_cut(long long grid_points, int tile_w,
     return (tiles < 148 ? 256ll : tiles < 296 ? 512ll : 2048ll) << shift;
 }
 bool core_slices_apply(int pk, int prec, int tile_w);
-/* FP32 erf profiles: whether a tile's parts are items of their own */
+/* whether a tile's parts are items of their own: FP32 erf profiles, FP32
+ * Voigt region I (4 bins x 4 warps) */
 bool erf_split(const gexs_job* jobs, int njobs, int tile_w);
+bool ws_split(const gexs_job* jobs, int njobs, int tile_w);
 int core_cut_shift(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows);
 cudaError_t launch_count(const gexs_job* d_jobs, int njobs, unsigned long long* d_counts,
                          int nsm, cudaStream_t st);

@@ -347,6 +347,21 @@ bool erf_split(const gexs_job* jobs, int njobs, int tile_w)
     return tiles < 1e8 && lines >= (tiles < 1184.0 ? 128.0 : 1024.0) * tiles;
 }
 
+bool ws_split(const gexs_job* jobs, int njobs, int tile_w)
+{
+    /* a quarter takes about 0.4 of a whole tile's time: worth it while the
+     * whole tiles' items (about one per tile and 16384 lines) are fewer than
+     * 1.5 per SM (manager segments of 300 to 500 items, which share the chip:
+     * 14.7 against 13.7 ms with quarters), and a tile holds more than a few
+     * lines */
+    double lines = 0.0, tiles = 0.0;
+    for (int i = 0; i < njobs; ++i) {
+        lines += tile_entries(jobs[i], jobs[i].cutoff, tile_w);
+        tiles += std::ceil((double)jobs[i].n_points / (double)tile_w);
+    }
+    return tiles + lines / 16384.0 < 222.0 && lines >= 64.0 * tiles;
+}
+
 int core_cut_shift(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows)
 {
     for (int shift = 0; shift < 40; ++shift) {

@@ -833,13 +833,12 @@ __device__ __forceinline__ void voigt_full4(const RecV* __restrict__ r, float2 l
  * independent chains.  Tier bits stay per quarter of 32*B bins (quarter q
  * = the bins a warp owns in the bins-split form): quarter q of a lane is
  * pairs q*B/2 .. q*B/2 + B/2 - 1. */
-template <int B, int Q, int NPAIR>
-__device__ __forceinline__ void voigt_quarter(const RecV& q, int tier, int lane, float2 n2,
-                                              float2 (&part)[NPAIR])
+template <int B>
+__device__ __forceinline__ void voigt_quarter(const RecV& q, int tier, int tl, float2 n2,
+                                              float2* part)
 {
     const float2 step = make_float2(64.f, 64.f);
     const float2 dx = q.dx, mf = q.mf, c = q.c, y2 = q.y2, a2 = q.a;
-    constexpr int J0 = Q * (B / 2);
     if (tier == 1) {
 #pragma unroll
         for (int j = 0; j < B / 2; ++j) {
@@ -848,14 +847,13 @@ __device__ __forceinline__ void voigt_quarter(const RecV& q, int tier, int lane,
             const float2 d = __ffma2_rn(m, m, y2);
             float2 r;
             r.x = rcp_approx(d.x); r.y = rcp_approx(d.y);
-            part[J0 + j] = __ffma2_rn(__ffma2_rn(m, r, r), a2, part[J0 + j]);
+            part[j] = __ffma2_rn(__ffma2_rn(m, r, r), a2, part[j]);
             n2 = __fadd2_rn(n2, step);
         }
         return;
     }
     const int a = lo16(q.win), b = hi16(q.win);
     const int c1a = lo16(q.c1), c1b = hi16(q.c1);
-    const int tl = 32 * B * Q + lane;
     if (tier == 2) {
         const unsigned wn = (unsigned)(b - a);
         const unsigned cn = c1b > c1a ? (unsigned)(c1b - c1a) : 0u;
@@ -870,8 +868,8 @@ __device__ __forceinline__ void voigt_quarter(const RecV& q, int tier, int lane,
             const int t0 = tl + 64 * j, t1 = t0 + 32;
             const bool in0 = (unsigned)(t0 - a) < wn && !((unsigned)(t0 - c1a) < cn);
             const bool in1 = (unsigned)(t1 - a) < wn && !((unsigned)(t1 - c1a) < cn);
-            part[J0 + j].x += in0 ? v.x : 0.f;
-            part[J0 + j].y += in1 ? v.y : 0.f;
+            part[j].x += in0 ? v.x : 0.f;
+            part[j].y += in1 ? v.y : 0.f;
             n2 = __fadd2_rn(n2, step);
         }
         return;
@@ -885,7 +883,7 @@ __device__ __forceinline__ void voigt_quarter(const RecV& q, int tier, int lane,
         const float x = fabsf(((n2.x + (float)(32 * k)) - fc) * dx.x);
         const float x2 = x * x;
         const float num = x2 + p;
-        float& acc = (k & 1) ? part[J0 + (k >> 1)].y : part[J0 + (k >> 1)].x;
+        float& acc = (k & 1) ? part[k >> 1].y : part[k >> 1].x;
         acc += (x < 1e18f) ? a2.x / (num - 2.f * (x2 / num)) : 0.f;
     }
 }
@@ -898,8 +896,8 @@ struct RsQuarters {
     {
         const int t = (tiers >> (2 * Q)) & 3;
         /* quarter Q starts 32 B Q bins further: exact in float */
-        if (t) voigt_quarter<B, Q>(r, t, lane, __fadd2_rn(n0, make_float2(32.f * B * Q, 32.f * B * Q)),
-                                   part);
+        if (t) voigt_quarter<B>(r, t, 32 * B * Q + lane,
+                                __fadd2_rn(n0, make_float2(32.f * B * Q, 32.f * B * Q)), part + Q * (B / 2));
         RsQuarters<B, Q + 1, CONS>::run(r, tiers, lane, n0, part);
     }
 };
@@ -1446,6 +1444,7 @@ struct StageHdr {
     int flags;             /* 1 first stage of the tile, 2 last, 4 end,
                               8 the item is one slice of a split tile       */
     int item, tile;        /* work item and its tile                        */
+    int quarter;           /* of the tile, in the kernel of quarters        */
 };
 
 __device__ __forceinline__ unsigned smem_u32(const void* p)
@@ -1500,7 +1499,13 @@ struct WsSmem {
     static constexpr size_t bytes = off_kahan + (size_t)(RS ? CONS : 1) * 2 * W * sizeof(float);
 };
 
-template <int B, int CONS, int PROD, bool PREP, int SR>
+/* Q = CONS (512-bin tiles): an item is one quarter of a tile (of a slice),
+ * bins [32 B q, 32 B (q + 1)), each warp taking every CONS-th record as for
+ * the whole tile, so the sums are the same bits; the producers derive the
+ * tile's lines once per quarter.  For launches of fewer items than CTAs
+ * (ws_split): 981 lines on 15 tiles 36 -> 24 us, 60,000 lines on 16 tiles
+ * 1.47 -> 0.61 ms. */
+template <int B, int CONS, int PROD, bool PREP, int SR, int Q = 1>
 __global__ void __launch_bounds__((CONS + PROD) * 32, CONS == 4 ? (B >= 8 ? 3 : 4) : 2)
 voigt_ws_kernel(const KArgs args)
 {
@@ -1553,13 +1558,14 @@ voigt_ws_kernel(const KArgs args)
         for (;;) {
             if (ptid == 0) s_item = atomicAdd(args.counter, 1);
             if (!psync()) { fail(); return; }
-            const int item = s_item;
+            const int item = s_item / Q;
             if (item >= nitems) {
                 if (!mbar_wait(s_empty + st, ph, args.spin)) { fail(); return; }
                 if (ptid == 0) { s_hdr[st].flags = 4; s_hdr[st].nrec = 0; }
                 mbar_arrive(s_full + st);
                 return;
             }
+            const int quarter = s_item % Q;
             /* item -> (tile, slice): one item per tile unless sliced */
             int ti = item, sidx = 0, ns = 1;
             if (sliced) {
@@ -1666,6 +1672,7 @@ voigt_ws_kernel(const KArgs args)
                     h.j0 = T.j0; h.jl = jl; h.jn = T.jn; h.nrec = nrec;
                     h.flags = (c == 0 ? 1 : 0) | (c == nchunk - 1 ? 2 : 0) | (ns > 1 ? 8 : 0);
                     h.item = item;
+                    h.quarter = Q > 1 ? quarter : 0;
                     h.tile = ti;
                     s_hdr[st] = h;
                 }
@@ -1691,7 +1698,83 @@ voigt_ws_kernel(const KArgs args)
         cph ^= 1;
         return ok;
     };
-    if constexpr (L::RS) {
+    if constexpr (L::RS && Q > 1) {
+        /* one quarter: as below on its 32 B bins, of which warp w writes every
+         * CONS-th group of 32 */
+        static_assert(B == CONS && Q == CONS, "a quarter is 32 bins per consumer warp");
+        float* my_ks = s_ks + (size_t)warp * 2 * W;
+        float* my_kc = my_ks + W;
+        float2 part[B / 2];
+#pragma unroll
+        for (int j = 0; j < B / 2; ++j) part[j] = make_float2(0.f, 0.f);
+        for (;;) {
+            if (!mbar_wait(s_full + st, ph, args.spin)) { atomicOr(args.err, GEXS_KERR_PIPELINE); return; }
+            const StageHdr h = s_hdr[st];
+            if (h.flags & 4) return;
+            const int q0 = 32 * B * h.quarter, tl = q0 + lane, sh = 2 * h.quarter;
+            if (h.flags & 1) {
+#pragma unroll
+                for (int k = 0; k < B; ++k) { my_ks[tl + 32 * k] = 0.f; my_kc[tl + 32 * k] = 0.f; }
+            }
+            const RecV* rec = s_rec + st * WS_R;
+            const float2 lw2 = make_float2((float)lane, (float)lane);
+            const float2 qo = make_float2((float)q0, (float)q0);
+#pragma unroll 2
+            for (int i = warp; i < h.nrec; i += CONS) {
+                const int tier = (rec[i].tiers >> sh) & 3;
+                /* n as for the whole tile: exact small integers */
+                if (tier) voigt_quarter<B>(rec[i], tier, tl, __fadd2_rn(__fadd2_rn(rec[i].nb, lw2), qo), part);
+            }
+#pragma unroll
+            for (int k = 0; k < B; ++k) {
+                const int t = tl + 32 * k;
+                float ks = my_ks[t], kc = my_kc[t];
+                kahan_add(ks, kc, (k & 1) ? part[k >> 1].y : part[k >> 1].x);
+                my_ks[t] = ks; my_kc[t] = kc;
+            }
+#pragma unroll
+            for (int j = 0; j < B / 2; ++j) part[j] = make_float2(0.f, 0.f);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(s_empty + st);
+            if (++st == WS_STAGES) { st = 0; ph ^= 1; }
+            if (!(h.flags & 2)) continue;
+            if (!csync()) { atomicOr(args.err, GEXS_KERR_PIPELINE); return; }
+            const int t = tl + 32 * warp;
+            double v = 0.0;
+#pragma unroll
+            for (int w = 0; w < CONS; ++w)
+                v += (double)s_ks[(size_t)w * 2 * W + t] - (double)s_ks[(size_t)w * 2 * W + W + t];
+            const gexs_job& J = args.jobs[h.jl];
+            double* out = J.out;
+            if (!(h.flags & 8)) {
+                if (t < h.jn) {
+                    const int64_t j = h.j0 + t;
+                    out[j] = J.accumulate ? out[j] + v : v;
+                }
+            } else {
+                const int base = args.sl.prefix[h.tile];
+                const int ns = args.sl.prefix[h.tile + 1] - base;
+                const int rb = args.sl.rowbase[h.tile];
+                if (t < h.jn) args.sl.rows[(size_t)(rb + (h.item - base)) * W + t] = v;
+                __threadfence();
+                if (!csync()) { atomicOr(args.err, GEXS_KERR_PIPELINE); return; }
+                if (tid == 0) s_last = atomicAdd(args.sl.ticket + h.tile, 1) == ns * Q - 1;
+                if (!csync()) { atomicOr(args.err, GEXS_KERR_PIPELINE); return; }
+                if (s_last) {
+                    __threadfence();
+                    for (int u = tid; u < h.jn; u += CONS * 32) {
+                        double acc = 0.0;
+                        for (int q = 0; q < ns; ++q) acc += __ldcg(args.sl.rows + (size_t)(rb + q) * W + u);
+                        const int64_t j = h.j0 + u;
+                        out[j] = J.accumulate ? out[j] + acc : acc;
+                    }
+                }
+            }
+            /* every warp has read the Kahan pairs before the next tile clears them */
+            if (!csync()) { atomicOr(args.err, GEXS_KERR_PIPELINE); return; }
+        }
+    }
+    else if constexpr (L::RS) {
         /* record-split: warp w adds records w, w + CONS, ... of every stage
          * into its own Kahan pairs of all W bins; at the end of a tile the
          * warps meet, and warp w writes bins [32 B w, 32 B (w+1)) as the sum
@@ -2286,6 +2369,8 @@ static cudaError_t launch_ws_sr(const KArgs& a, int ctas_per_sm, int nsm, cudaSt
 {
     constexpr int PROD = 2;
     auto kern = voigt_ws_kernel<B, CONS, PROD, PREP, SR>;
+    if constexpr (B == 4 && CONS == 4)
+        if (a.sl.prefix && a.sl.split) kern = voigt_ws_kernel<B, CONS, PROD, PREP, SR, CONS>;
     const size_t smem = WsSmem<B, CONS, PROD, PREP, SR>::bytes;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
