@@ -1017,12 +1017,10 @@ def our_arm(args):
                        "launch_cfg": {"bins_per_lane": cfg[0], "warps": cfg[1],
                                       "long_stages": bool(len(cfg) > 3 and
                                                           cfg[3] & capi.LAUNCH_LONG_STAGES)}},
-            # per step: put_blob_kernel (launch table), prep_kernel (S(T),
-            # width, y per line), slice_plan_kernel and slice_scan_kernel
-            # (line slices), voigt_ws_kernel (region I), zero_ints_kernel
-            # (core work counter), core_slice_plan_kernel and
-            # slice_scan_kernel (core slices), core_kernel (regions II-IV)
-            "gpu_launches": 9 * args.steps,
+            # per step: put_blob_kernel (launch table), setup_kernel (S(T),
+            # width, y per line; line slices of both kernels),
+            # voigt_ws_kernel (region I), core_kernel (regions II-IV)
+            "gpu_launches": 4 * args.steps,
             "roofline": {"bound": "fp32", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
                          "traffic": traffic,
@@ -1031,7 +1029,7 @@ def our_arm(args):
                                         "no FP32 figure",
                          "flop_per_eval": fpe, "region_fractions": frac,
                          "launch_ms": launch_ms,
-                         "timed": "one cross-section per step: prep_kernel + voigt_ws_kernel "
+                         "timed": "one cross-section per step: setup_kernel + voigt_ws_kernel "
                                   "(region I) + core_kernel (regions II-IV), CUDA events on "
                                   "the launching stream; per-kernel shares in the ncu launch "
                                   "list under profiles/",

@@ -387,7 +387,7 @@ long long slice_lines(const gexs_job* jobs, int njobs, int prec, int tile_w, int
      * workload is indifferent to 16k-128k, a dense band of 1e6 lines in 80
      * cm^-1 runs 25% faster than at 65536.
      * FP64 (any cut gives the same sums): about eight items for each of the
-     * 888 CTAs that fit, of 512 to 4096 lines.  2e5 lines on 194 tiles
+     * CTAs that fit (888 of 740 to 888), of 512 to 4096 lines.  2e5 lines on 194 tiles
      * (GH32): 8.2 ms against 34 ms uncut. */
     double m = 0.0;
     for (int i = 0; i < njobs; ++i) m += tile_entries(jobs[i], jobs[i].cutoff, tile_w);

@@ -74,8 +74,8 @@ struct __align__(16) RecF64 {   /* 48 bytes; GH */
     int    win;
     int    mask;           /* bit w: touches warp w; 8 + w: its bins all at
                               |x| >= GH_FAR; 16 + w: all in the window;
-                              bit 24: IEEE form (y < 1e-100, or |x| or y may
-                              exceed 1e60)                                   */
+                              bit 24: IEEE form (y < 1e-100, |x| or y may
+                              exceed 1e60, or a 1e300)                       */
     int    pad0, pad1;
 };
 
@@ -107,7 +107,7 @@ struct __align__(16) RecV64 {
                               out_scale)                                     */
     int    tiers;          /* 2 bits per warp, as RecV.tiers; 3 is per bin,
                               with IEEE divisions: |x| or y may exceed 1e60,
-                              or y < 0 (the line's core included)            */
+                              amp 1e240, or y < 0 (the line's core included) */
     int    win;
     int    c1, pad;
     double y;
@@ -417,6 +417,8 @@ __device__ __forceinline__ void dd_add(double& hi, double& lo, double v)
     lo = dadd(lo, dadd(dsub(hi, dsub(s, bb)), dsub(v, bb)));
     hi = s;
 }
+/* the sum's value; lo is meaningless once hi has overflowed */
+__device__ __forceinline__ double dd_value(double hi, double lo) { return isfinite(hi) ? hi + lo : hi; }
 
 /* per-warp tiers of a line (bits of RecF*.mask).  Warp w owns bins
  * [32*B*w, 32*B*(w+1)) of the tile. */
@@ -548,7 +550,8 @@ __device__ __forceinline__ void make_rec(RecF64& q, const Derived<PK>& d, const 
     q.pad0 = q.pad1 = 0;
     const int a = lo16(d.win), b = hi16(d.win);
     const double dfar = fmax(fabs(d.nu - T.f0), fabs(d.nu - T.fl));
-    const bool general = !(d.y >= 1e-100) || !(d.y < 1e60) || !(dfar * d.invw < 1e60);
+    const bool general = !(d.y >= 1e-100) || !(d.y < 1e60) || !(dfar * d.invw < 1e60) ||
+                         !(fabs(q.a) < 1e300);
     /* distance of GH_FAR in bins */
     const double reach = GH_FAR / d.invw * T.inv_dnu + 1.0;
     int m = general ? 1 << 24 : 0;
@@ -571,7 +574,8 @@ __device__ __forceinline__ void make_rec(RecV64& q, const Derived<PK>& d, const 
     const double dfar = fmax(fabs(d.nu - T.f0), fabs(d.nu - T.fl));
     /* beyond: x^4 or y^4 could overflow, or (y < 0) the core kernel's line
      * search, which assumes y >= 0, could miss the line */
-    const bool general = !(dfar * d.invw < 1e60) || !(d.y < 1e60) || d.y < 0.0;
+    const bool general = !(dfar * d.invw < 1e60) || !(d.y < 1e60) || d.y < 0.0 ||
+                         !(fabs(amp) < 1e240);
     q.nu = d.nu; q.invw = d.invw; q.y = d.y;
     q.c = d.y * d.y - 0.5;
     q.y2 = 2.0 * d.y * d.y;
@@ -1008,7 +1012,7 @@ __device__ __forceinline__ void lines_f64(const RecF64* __restrict__ rec, int nr
             for (int k = 0; k < B; ++k) {
                 const double v = gh_sum_f64_far<NODES>((fbin[k] - nu) * invw, y2);
                 const bool in = full || (unsigned)(tl + 32 * k - wa) < wn;
-                acc[k] = fma(a, in ? v : 0.0, acc[k]);
+                acc[k] = fma(a, in ? v : 0.0, acc[k]);     /* a is finite */
             }
         } else {
 #pragma unroll
@@ -1032,6 +1036,7 @@ __device__ __forceinline__ void lines_voigt_f64(const RecV64* __restrict__ rec, 
                                                 int lane, const double (&fbin)[B], double (&acc)[B])
 {
     const int sh = 2 * warp, tl = warp * 32 * B + lane;
+#pragma unroll 2
     for (int i = 0; i < nrec; ++i) {
         const RecV64& q = rec[i];
         const double a = q.a;
@@ -1079,7 +1084,7 @@ __device__ __forceinline__ void lines_voigt_f64(const RecV64* __restrict__ rec, 
             const double r = rcp_f64(fma(m, m, y2));
             const double v = fma(m, r, r);
             const bool in = (unsigned)(t - wa) < wn && !((unsigned)(t - ca) < cn);
-            acc[k] = fma(a, in ? v : 0.0, acc[k]);
+            acc[k] = fma(a, in ? v : 0.0, acc[k]);     /* a is finite */
         }
     }
 }
@@ -1108,8 +1113,8 @@ struct Smem {
 template <int B, int WARPS, int PREC>
 constexpr int min_ctas()
 {
-    (void)PREC;
-    return WARPS == 8 ? (B >= 8 ? 2 : 3) : (B >= 8 ? 4 : 6);
+    /* FP64 with four warps: five (5e6 Voigt lines 19.2 ms; six 20.0, four 20.4) */
+    return WARPS == 8 ? (B >= 8 ? 2 : 3) : (B >= 8 ? 4 : PREC == GEXS_FP64 ? 5 : 6);
 }
 
 template <int PK, int PREC, int B, int WARPS, bool PREP, bool SPLIT = false>
@@ -1362,7 +1367,7 @@ tile_kernel(const KArgs args)
             for (int k = 0; k < KB; ++k) {
                 const int t = tile_bin<PK, B, WARPS>(warp, lane, k0 + k);
                 if (t < T.jn) {
-                    const double v = DD ? s_hi[t] + s_lo[t] : hi_of(t);
+                    const double v = DD ? dd_value(s_hi[t], s_lo[t]) : hi_of(t);
                     int64_t j = T.j0 + t;
                     out[j] = acc_mode ? out[j] + v : v;
                 }
@@ -1394,7 +1399,7 @@ tile_kernel(const KArgs args)
                         if (DD) { dd_add(hi, lo, __ldcg(r)); lo = dadd(lo, __ldcg(r + W)); }
                         else hi += __ldcg(r);
                     }
-                    const double v = DD ? hi + lo : hi;
+                    const double v = DD ? dd_value(hi, lo) : hi;
                     int64_t j = T.j0 + t;
                     out[j] = acc_mode ? out[j] + v : v;
                 }
@@ -2305,7 +2310,7 @@ core_kernel(const KArgs args)
                 for (int t = tid; t < T.jn; t += NT) {
                     double hi, lo;
                     total(t, hi, lo);
-                    put(t, hi + lo);
+                    put(t, DD ? dd_value(hi, lo) : hi);
                 }
             } else {
                 /* a slice of a split tile: its totals into its partial row, a
@@ -2333,7 +2338,7 @@ core_kernel(const KArgs args)
                             if (DD) { dd_add(hi, lo, __ldcg(r)); lo = dadd(lo, __ldcg(r + W)); }
                             else hi += __ldcg(r);
                         }
-                        put(t, hi + lo);
+                        put(t, DD ? dd_value(hi, lo) : hi);
                     }
                 }
             }

@@ -77,3 +77,28 @@ def test_fp64_general_tier(gpu_ctx, dop, gamma):
     assert np.isfinite(want).all()
     worst, nbad = H.fp64_mismatch(out.cpu().numpy(), want, abs_floor=1e-13 * np.max(np.abs(want)))
     assert nbad == 0, worst
+
+
+@pytest.mark.parametrize("profile", [capi.VOIGT, capi.VOIGT_QUAD])
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_fp64_infinite_line_stays_in_its_window(gpu_ctx, profile, bad):
+    """A line whose intensity is infinite or not a number makes the bins of
+    its window so, and no others, as in the oracle."""
+    n, g = 700, 3000
+    rng = np.random.Generator(np.random.PCG64(11))
+    L = {"nu": np.sort(rng.uniform(1000.0, 1030.0, n)), "elow": np.full(n, 50.0),
+         "aif": 10.0 ** rng.uniform(-2, 1, n), "gns": np.full(n, 3, dtype=np.int32),
+         "gamma": np.full(n, 0.05), "n": np.full(n, 0.5)}
+    L["aif"][n // 2] = bad
+    out = torch.zeros(g, dtype=torch.float64, device="cuda")
+    job = Job(LineList.from_dict(L), out, convention=capi.CONV_PHYSICAL, profile=profile,
+              temperature=900.0, pressure=0.2, partition=100.0, mass=18.0, nu_start=1000.0,
+              dnu=0.01, grid_points=g, precision=capi.FP64, cutoff=2.3)
+    gpu_ctx.run([job])
+    gpu_ctx.check()
+    want, got = H.oracle_of(job, L), out.cpu().numpy()
+    fine = np.isfinite(want)
+    assert 0 < fine.sum() < g
+    assert np.array_equal(got[~fine], want[~fine], equal_nan=True)
+    worst, nbad = H.fp64_mismatch(got[fine], want[fine])
+    assert nbad == 0, worst
