@@ -52,6 +52,11 @@ class GexsLaunchCfg(C.Structure):
     _fields_ = [("bins_per_lane", C.c_int32), ("warps", C.c_int32),
                 ("ctas_per_sm", C.c_int32), ("flags", C.c_int32), ("wait_spins", C.c_int32)]
 
+
+class GexsUploadPiece(C.Structure):
+    _fields_ = [("dst", C.c_void_p), ("src", C.c_void_p), ("bytes", C.c_size_t),
+                ("event", C.c_void_p)]
+
 LAUNCH_DERIVE_ON_LOAD = 1
 LAUNCH_LONG_STAGES = 2
 LAUNCH_JOB_MAJOR = 4
@@ -99,6 +104,7 @@ SIGNATURES = [
     ("gexs_ctx_create", C.c_int, [C.c_int, C.POINTER(C.c_void_p)]),
     ("gexs_ctx_destroy", C.c_int, [C.c_void_p]),
     ("gexs_ctx_check", C.c_int, [C.c_void_p, C.c_void_p]),
+    ("gexs_ctx_upload", C.c_int, [C.c_void_p, C.POINTER(GexsUploadPiece), C.c_int, C.c_void_p]),
     ("gexs_run_noalloc", C.c_int, [C.POINTER(GexsJob), C.c_int, C.POINTER(GexsLaunchCfg),
                                    C.c_void_p]),
     ("gexs_noalloc_status", C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),

@@ -9,16 +9,11 @@ import numpy as np
 import pytest
 import torch
 
-from gexs_b200._capi import check, lib
+from gexs_b200._capi import GexsUploadPiece as Piece, check, lib
 
 pytestmark = pytest.mark.gpu
 
 MIB = 1 << 20
-
-
-class Piece(C.Structure):
-    _fields_ = [("dst", C.c_void_p), ("src", C.c_void_p), ("bytes", C.c_size_t),
-                ("event", C.c_void_p)]
 
 
 def _upload(ctx, arrays, stream):
