@@ -65,7 +65,7 @@ extern "C" int gexs_run_noalloc(const gexs_job* jobs, int njobs, const gexs_laun
         return set_error(GEXS_ERR_INVALID, "gexs_run_noalloc: njobs must be 1.." +
                                                std::to_string(GEXS_NOALLOC_MAX_JOBS));
     const int pk = profile_class(jobs[0]), prec = jobs[0].precision;
-    /* gexs_run's defaults: 4 bins per lane, 4 warps (FP32) or 8 (FP64) */
+    /* 4 bins per lane, 4 warps (FP32) or 8 (FP64) */
     gexs_launch_cfg c{};
     c.bins_per_lane = 4; c.warps = (prec == GEXS_FP64) ? 8 : 4;
     if (cfg) c = *cfg;

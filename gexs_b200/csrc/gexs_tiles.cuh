@@ -26,7 +26,10 @@
  *    slice order (deterministic, independent of other jobs);
  *  - FP32 form: FP32 partial sums of up to 128 lines merged into a
  *    Kahan-compensated (sum, compensation) pair per bin in shared memory;
- *    FP64 form: plain FP64 sums in registers.
+ *    FP64 form: sums of blocks of SUM_BLOCK lines in registers, the blocks
+ *    added as (hi, lo) pairs.
+ * The Voigt core and the FP64 erf profiles go line by line instead
+ * (core_kernel).
  */
 #pragma once
 #include <algorithm>
@@ -1028,9 +1031,10 @@ __device__ __forceinline__ void lines_f64(const RecF64* __restrict__ rec, int nr
  * 1/2 (the rational of hum_region1 without its cancellation), with 1/d from
  * rcp_f64: nine FP64 instructions per evaluation (x two, m, d, three of the
  * reciprocal, two of the sum), so the FP64 pipe bounds the loop at 64 / 9
- * evaluations per SM-clock.  Per-bin region tests and IEEE divisions took
- * about 45 issue slots per evaluation.  The core is core_kernel's, as in
- * the FP32 form. */
+ * evaluations per SM-clock; it reaches 67% of that pipe.  With per-bin
+ * region tests and IEEE divisions, about 45 issue slots per evaluation, 5e6
+ * lines on 990,001 bins took 66 ms, now 19.2.  The core is core_kernel's,
+ * as in the FP32 form. */
 template <int B>
 __device__ __forceinline__ void lines_voigt_f64(const RecV64* __restrict__ rec, int nrec, int warp,
                                                 int lane, const double (&fbin)[B], double (&acc)[B])
@@ -1969,11 +1973,11 @@ voigt_ws_kernel(const KArgs args)
  * all lanes of a step are in the same region, and neighbouring lines have
  * nearly equal ranges, so most lanes work.  Stepping the union of the 32
  * cores bin by bin instead (every lane at the same bin, a butterfly per
- * bin) ran each region's code at nearly every step: 10.0 against 4.4 ms for
+ * bin) ran each region's code at nearly every step: 10.0 against 2.9 ms for
  * eight (T, P) pairs of a 1e6-line list (sparse, fine grids), 6.0 against
- * 4.6 ms for a dense 2e7-line list at 1 bar, 33 against 21 us for 3000
- * lines on 6001 bins.  Two bins per step made the code too long for the
- * instruction cache (5.4 ms on the dense list). */
+ * 5.0 ms for a dense 2e7-line list at 1 bar, 33 against 23 us for 3000
+ * lines on 6001 bins.  Instruction fetches bound the dense case: two bins
+ * per step made it 18% slower. */
 constexpr int CORE_W = 1024;
 constexpr int CORE_WARPS = 4;
 
