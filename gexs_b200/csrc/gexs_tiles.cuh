@@ -1114,15 +1114,20 @@ struct Smem {
 
 /* ---------------------------------------------------------------- kernel */
 /* resident CTAs per SM the register budget is sized for */
-template <int B, int WARPS, int PREC>
+template <int PK, int B, int WARPS, int PREC>
 constexpr int min_ctas()
 {
-    /* FP64 with four warps: five (5e6 Voigt lines 19.2 ms; six 20.0, four 20.4) */
-    return WARPS == 8 ? (B >= 8 ? 2 : 3) : (B >= 8 ? 4 : PREC == GEXS_FP64 ? 5 : 6);
+    /* four warps: FP64 five (5e6 Voigt lines 19.2 ms; six 20.0, four 20.4);
+     * FP32 quadrature four, so that two pairs of bins and a node's constants
+     * stay in registers (1e6 lines, GH16: 14.4 ms; six 17.0; narrow lines
+     * 19.0 and 22.9); FP32 erf six (1.40 ms; five 1.57) */
+    if (WARPS == 8) return B >= 8 ? 2 : 3;
+    if (B >= 8) return 4;
+    return PREC == GEXS_FP64 ? 5 : PK == PK_ERF ? 6 : 4;
 }
 
 template <int PK, int PREC, int B, int WARPS, bool PREP, bool SPLIT = false>
-__global__ void __launch_bounds__(WARPS * 32, min_ctas<B, WARPS, PREC>())
+__global__ void __launch_bounds__(WARPS * 32, min_ctas<PK, B, WARPS, PREC>())
 tile_kernel(const KArgs args)
 {
     typedef Smem<PK, PREC, B, WARPS, PREP> L;
