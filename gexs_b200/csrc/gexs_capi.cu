@@ -244,7 +244,7 @@ struct Layout {
     bool csliced = false;
     size_t oc_prefix = 0, oc_counts = 0, oc_rowbase = 0, oc_ticket = 0, oc_lohi = 0, oc_nitems = 0,
            oc_rows = 0;
-    int cmax_rows = 0, ccut_shift = 0;
+    CoreRows crows = {0, 0, 0};
 };
 
 static Layout group_layout(const Group& g, bool prep, const gexs_launch_cfg& cfg)
@@ -280,16 +280,16 @@ static Layout group_layout(const Group& g, bool prep, const gexs_launch_cfg& cfg
         L.os_nitems = up(a); a = L.os_nitems + 256;
         L.os_rows = up(a);   a = L.os_rows + (size_t)L.max_rows * row_doubles(g.prec, W) * sizeof(double);
     }
-    if (core_slices_apply(g.pk, g.prec, W) && nt > 0) {
+    if (core_slices_apply(g.pk, g.prec, W) && nt > 0 &&
+        core_rows(g.jobs.data(), (int)g.jobs.size(), g.prec, W, &L.crows)) {
         L.csliced = true;
-        L.ccut_shift = core_cut_shift(g.jobs.data(), (int)g.jobs.size(), g.prec, W, &L.cmax_rows);
         L.oc_prefix = up(a); a = L.oc_prefix + (nt + 1) * sizeof(int);
         L.oc_counts = up(a); a = L.oc_counts + nt * sizeof(int);
         L.oc_rowbase = up(a); a = L.oc_rowbase + nt * sizeof(int);
         L.oc_ticket = up(a); a = L.oc_ticket + nt * sizeof(int);
         L.oc_lohi = up(a);   a = L.oc_lohi + 2 * nt * sizeof(long long);
         L.oc_nitems = up(a); a = L.oc_nitems + 256;
-        L.oc_rows = up(a);   a = L.oc_rows + (size_t)L.cmax_rows * row_doubles(g.prec, W) * sizeof(double);
+        L.oc_rows = up(a);   a = L.oc_rows + (size_t)L.crows.alloc * row_doubles(g.prec, W) * sizeof(double);
     }
     L.bytes = a + 256;
     return L;
@@ -353,8 +353,8 @@ static cudaError_t enqueue_group(const Group& g, const Layout& L, unsigned char*
         csl.lohi = (long long*)(d + L.oc_lohi);
         csl.nitems = (int*)(d + L.oc_nitems);
         csl.rows = (double*)(d + L.oc_rows);
-        csl.max_rows = L.cmax_rows;
-        csl.cut_shift = L.ccut_shift;
+        csl.max_rows = L.crows.bound;
+        csl.round_rows = L.crows.round_rows;
     }
     return launch_tiles(g.pk, g.prec, (const gexs_job*)d, (const int*)(d + L.op),
                         (int)g.jobs.size(), g.nitems, (int*)(d + L.oc), d_err,

@@ -29,7 +29,7 @@ struct SliceTables {
     double*    rows;        /* max_rows x tile bins: partial rows        */
     int        max_rows;
     long long  lines_per_slice;
-    int        cut_shift;   /* core kernel: see core_cut                    */
+    int        round_rows;  /* core kernel: rows of a round (core_rows), 0: one round */
     int        split;       /* FP32 erf, Voigt: items are parts of a tile   */
 };
 
@@ -58,30 +58,61 @@ cudaError_t launch_tiles(int pk, int prec, const gexs_job* d_jobs, const int* d_
 constexpr int SUM_BLOCK = 512;
 
 /* doubles of a partial row: a value per bin, (hi, lo) in the FP64 forms */
-inline int row_doubles(int prec, int tile_w) { return prec == GEXS_FP64 ? 2 * tile_w : tile_w; }
+__host__ __device__ inline int row_doubles(int prec, int tile_w)
+{
+    return prec == GEXS_FP64 ? 2 * tile_w : tile_w;
+}
 
 /* which groups are sliced; lines_per_slice for a group and the bound on the
  * rows of its split tiles */
 bool slices_apply(int pk, int prec);
 long long slice_lines(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows);
 
+/* bytes of partial rows held at a time */
+constexpr long long ROW_BYTES = 1ll << 30;
+
 /* the core kernel's own slices (its line range per tile is reach_range's):
- * only when a tile is one core sub-tile (tile_w <= 1024).  Lines per slice
- * by the tiles of the job's whole grid, so that a sub-range of it and a
- * batch are cut alike: a job of few tiles has only its lines to fill the
- * chip with.  The shift grows when the rows would pass 1 GiB. */
-__host__ __device__ inline long long core_cut(long long grid_points, int tile_w, int shift)
+ * only when a tile is one core sub-tile (tile_w <= 1024).  FP32 sums depend
+ * on the cut, so it depends on the tile's lines and on the size of the job's
+ * whole grid alone: a batch, a sub-range and a sub-list of a job are cut
+ * alike.  Lines per slice by the tiles of the grid: a job of few tiles has
+ * only its lines to fill the chip with. */
+__host__ __device__ inline long long core_cut(long long grid_points, int tile_w)
 {
     const long long tiles = (grid_points + tile_w - 1) / tile_w;
-    if (shift >= 40) return 1ll << 62;
-    return (tiles < 148 ? 256ll : tiles < 296 ? 512ll : 2048ll) << shift;
+    return tiles < 148 ? 256ll : tiles < 296 ? 512ll : 2048ll;
+}
+/* most slices of a tile (longer ones beyond): the rows of one job stay
+ * within ROW_BYTES, and a thousand items, eight thousand for a job of few
+ * tiles, fill the ~900 CTAs that fit */
+__host__ __device__ inline long long core_max_slices(long long grid_points, int tile_w, int prec)
+{
+    const long long tiles = grid_points > tile_w ? (grid_points + tile_w - 1) / tile_w : 1;
+    const long long fit = ROW_BYTES / (long long)sizeof(double) / (tiles * row_doubles(prec, tile_w));
+    const long long use = 8192 / tiles > 1024 ? 8192 / tiles : 1024;
+    return fit < 1 ? 1 : fit < use ? fit : use;
+}
+/* slices of a tile with n lines */
+__host__ __device__ inline int core_slices(long long n, long long grid_points, int tile_w, int prec)
+{
+    const long long per = core_cut(grid_points, tile_w);
+    if (n <= per) return 1;
+    const long long ns = (n + per - 1) / per, most = core_max_slices(grid_points, tile_w, prec);
+    return (int)(ns < most ? ns : most);
 }
 bool core_slices_apply(int pk, int prec, int tile_w);
+/* partial rows of a launch's core slices: a bound on their number (false:
+ * more than an int holds), the rows of a round (0: all fit in ROW_BYTES and
+ * there is one round) and those to allocate.  With several rounds the core
+ * kernel is launched once for each range of round_rows rows, over the tiles
+ * whose rows begin there, and the ranges share the memory; the last tile's
+ * rows may reach past the range. */
+struct CoreRows { int bound, round_rows, alloc; };
+bool core_rows(const gexs_job* jobs, int njobs, int prec, int tile_w, CoreRows* out);
 /* whether a tile's parts are items of their own: FP32 erf profiles, FP32
  * Voigt region I (4 bins x 4 warps) */
 bool erf_split(const gexs_job* jobs, int njobs, int tile_w);
 bool ws_split(const gexs_job* jobs, int njobs, int tile_w);
-int core_cut_shift(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows);
 cudaError_t launch_count(const gexs_job* d_jobs, int njobs, unsigned long long* d_counts,
                          int nsm, cudaStream_t st);
 cudaError_t launch_partition(const double* d_e, const int32_t* d_g, int64_t n,

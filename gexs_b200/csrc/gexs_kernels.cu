@@ -171,10 +171,9 @@ __device__ __forceinline__ void plan_core_tile(const KArgs& a, const gexs_job& J
     const int64_t hi = max(warp_bound<true>(J.lines.nu, nl, vhi, lane), lo);
     if (lane == 0) {
         const long long n = hi - lo;
-        const long long per = core_cut(J.grid_points, a.tile_w, a.csl.cut_shift);
         a.csl.lohi[2 * ti] = lo;
         a.csl.lohi[2 * ti + 1] = hi;
-        a.csl.counts[ti] = n > per ? (int)((n + per - 1) / per) : 1;
+        a.csl.counts[ti] = core_slices(n, J.grid_points, a.tile_w, J.precision);
         a.csl.ticket[ti] = 0;
     }
 }
@@ -283,6 +282,7 @@ cudaError_t launch_tiles(int pk, int prec, const gexs_job* d_jobs, const int* d_
     a.order = njobs > 1 ? d_order : nullptr;
     a.counter = d_counter; a.err = d_err; a.prep = d_prep;
     a.tile_w = tile_bins(cfg);
+    a.row0 = 0;
     a.spin = cfg.wait_spins > 0 ? cfg.wait_spins : WS_SPIN;
     std::memset(&a.sl, 0, sizeof(a.sl));
     std::memset(&a.csl, 0, sizeof(a.csl));
@@ -322,7 +322,7 @@ static double tile_entries(const gexs_job& j, double reach, int tile_w)
     return (double)j.lines.count * tpl;
 }
 
-static const double kMaxRowBytes = (double)(1ull << 30);
+static const double kMaxRowBytes = (double)ROW_BYTES;
 
 /* reach_range's reach at the job's highest frequency */
 static double scatter_reach(const gexs_job& j)
@@ -362,22 +362,29 @@ bool ws_split(const gexs_job* jobs, int njobs, int tile_w)
     return tiles + lines / 16384.0 < 222.0 && lines >= 64.0 * tiles;
 }
 
-int core_cut_shift(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows)
+bool core_rows(const gexs_job* jobs, int njobs, int prec, int tile_w, CoreRows* out)
 {
-    for (int shift = 0; shift < 40; ++shift) {
-        double rows = 0.0;
-        for (int i = 0; i < njobs; ++i) {
-            const gexs_job& j = jobs[i];
-            rows += row_bound(j, tile_entries(j, scatter_reach(j), tile_w), tile_w,
-                              (double)core_cut(j.grid_points, tile_w, shift));
-        }
-        if (rows * row_doubles(prec, tile_w) * sizeof(double) <= kMaxRowBytes) {
-            *max_rows = (int)rows;
-            return shift;
-        }
+    double total = 0.0;
+    long long most = 1;
+    for (int i = 0; i < njobs; ++i) {
+        const gexs_job& j = jobs[i];
+        const double tiles = std::ceil((double)j.n_points / (double)tile_w);
+        /* reach_range's margins hold 2e-9 of the frequency as well */
+        const double nu_hi = j.nu_start + (double)(j.start_idx + j.n_points) * j.dnu + j.cutoff;
+        const double reach = scatter_reach(j) + 2e-9 * (std::fabs(nu_hi) + j.cutoff);
+        const double m = std::min(tile_entries(j, reach, tile_w), (double)j.lines.count * tiles);
+        const long long cap = core_max_slices(j.grid_points, tile_w, prec);
+        if (cap < 2) continue;
+        total += std::min(row_bound(j, m, tile_w, (double)core_cut(j.grid_points, tile_w)),
+                          tiles * (double)cap);
+        most = std::max(most, cap);
     }
-    *max_rows = 0;
-    return 40;
+    if (!(total < (double)INT32_MAX)) return false;
+    const long long fit = ROW_BYTES / ((long long)sizeof(double) * row_doubles(prec, tile_w));
+    out->bound = (int)total;
+    out->round_rows = total <= (double)fit ? 0 : (int)fit;
+    out->alloc = out->round_rows ? (int)(fit + most) : out->bound;
+    return true;
 }
 
 long long slice_lines(const gexs_job* jobs, int njobs, int prec, int tile_w, int* max_rows)

@@ -372,7 +372,8 @@ struct KArgs {
     double* const*  prep;      /* per job S|invw|y arrays, or NULL       */
     int             tile_w;    /* bins per work item (core kernel)       */
     SliceTables     sl;        /* line slices (sl.prefix NULL: none)     */
-    SliceTables     csl;       /* FP32 Voigt core kernel's slices        */
+    SliceTables     csl;       /* core kernel's slices                   */
+    int             row0;      /* core kernel: first row of its round    */
     int             spin;      /* try_wait attempts of every bounded wait */
     const int*      order;     /* tile-major order tables F|R|P, or NULL
                                   for job-major items (gexs_capi.cu
@@ -2137,6 +2138,17 @@ __device__ __forceinline__ void scatter_phase(int a, int b, int lane, const Core
     }
 }
 
+/* the first tile whose rows begin at row or later */
+__device__ __forceinline__ int row_tile(const KArgs& a, long long row)
+{
+    int lo = 0, hi = a.nitems;
+    while (lo < hi) {
+        const int m = (lo + hi) >> 1;
+        if (__ldg(a.csl.rowbase + m) < row) lo = m + 1; else hi = m;
+    }
+    return lo;
+}
+
 template <int PK, int PREC, bool PREP, bool ORDER>
 __global__ void __launch_bounds__(CORE_WARPS * 32, 24 / CORE_WARPS)
 core_kernel(const KArgs args)
@@ -2156,10 +2168,17 @@ core_kernel(const KArgs args)
     if (!DD) for (int z = lane; z < SCR_D; z += 32) scr[z] = 0.0;
     /* sliced (host-enabled only when a tile is one sub-tile of CORE_W) */
     const bool sliced = args.csl.prefix != nullptr;
-    const int nitems = sliced ? *(volatile const int*)args.csl.nitems : args.nitems;
     __shared__ int s_last;
+    /* read by every thread: a branch of thread 0 here would run into the one
+     * at the loop's head, and warp 0 then reached the barriers in two parts */
+    int first = 0, nitems = sliced ? *(volatile const int*)args.csl.nitems : args.nitems;
+    if (sliced && args.csl.round_rows && nitems > 0) {
+        /* the tiles whose rows begin in [row0, row0 + round_rows) */
+        first = __ldg(args.csl.prefix + row_tile(args, args.row0));
+        nitems = __ldg(args.csl.prefix + row_tile(args, (long long)args.row0 + args.csl.round_rows));
+    }
     for (;;) {
-        if (tid == 0) s_item = atomicAdd(args.counter, 1);
+        if (tid == 0) s_item = first + atomicAdd(args.counter, 1);
         __syncthreads();
         const int item = s_item;
         if (item >= nitems) break;
@@ -2325,7 +2344,7 @@ core_kernel(const KArgs args)
                 /* a slice of a split tile: its totals into its partial row, a
                  * ticket, and the last slice adds the partial rows in slice
                  * order (a zero total adds nothing, as above) */
-                const int rb = args.csl.rowbase[ti];
+                const int rb = args.csl.rowbase[ti] - args.row0;
                 const int W = args.tile_w, RS = DD ? 2 * W : W;
                 double* prow = args.csl.rows + (size_t)(rb + sidx) * RS;
                 for (int t = tid; t < T.jn; t += NT) {
@@ -2482,8 +2501,16 @@ static cudaError_t launch_core(const KArgs& a, int nsm, cudaStream_t st)
     const int grid = a.csl.prefix ? max(occ, 1) * nsm : max(1, min(a.nitems, max(occ, 1) * nsm));
     KArgs c = a;
     c.counter = a.counter + CORE_COUNTER_OFFSET;
-    kern<<<grid, CORE_WARPS * 32, smem, st>>>(c);
-    return cudaGetLastError();
+    const int step = a.csl.prefix ? a.csl.round_rows : 0;
+    for (long long row = 0;; row += step) {
+        c.row0 = (int)row;
+        kern<<<grid, CORE_WARPS * 32, smem, st>>>(c);
+        e = cudaGetLastError();
+        /* a row range may hold tiles that are not split: row max_rows too */
+        if (e != cudaSuccess || step == 0 || row + step > a.csl.max_rows) return e;
+        e = zero_ints(c.counter, 1, st);
+        if (e != cudaSuccess) return e;
+    }
 }
 
 /* every launch shape of one profile class, both precisions, both
