@@ -70,36 +70,34 @@ __device__ __forceinline__ double rcp_f64(double d)
     return fma(r, fma(e, e, e), r);
 }
 
-template <typename R>
-__device__ __forceinline__ R re_div(R nr, R ni, R dr, R di)
+/* Regions II-IV with every rounding written out: a bin's value depends on
+ * which products the compiler contracts, and the core kernel has two copies
+ * of each region (its dense and its sparse walk), chosen by the 32 lines of
+ * a group.  Left to the compiler, 1183 of 80,001 bins of a 2000-line FP64
+ * list differed between tile shapes, by up to 47 ulp (region IV cancels). */
+__device__ __forceinline__ double re_div(double nr, double ni, double dr, double di)
 {
-    /* FP64; |d|^2 is between ~1e-1 and ~1e30 in regions II-IV */
-    return fma(nr, dr, ni * di) * rcp_f64(fma(dr, dr, di * di));
-}
-/* FP32: one approximate reciprocal (1 ulp) instead of an IEEE division */
-template <>
-__device__ __forceinline__ float re_div<float>(float nr, float ni, float dr, float di)
-{
-    return fmaf(nr, dr, ni * di) * rcp_approx(fmaf(dr, dr, di * di));
+    /* |d|^2 is between ~1e-1 and ~1e30 in regions II-IV */
+    return dmul(fma(nr, dr, dmul(ni, di)), rcp_f64(fma(dr, dr, dmul(di, di))));
 }
 
-template <typename R>
-__device__ __forceinline__ R hum_region2(R x, R y)
+template <typename R> __device__ __forceinline__ R hum_region2(R x, R y);
+template <>
+__device__ __forceinline__ double hum_region2<double>(double x, double y)
 {
     /* T (1.410474 + .5641896 U) / (.75 + U (3 + U)), U = T^2 */
-    R ur = y * y - x * x, ui = R(-2) * x * y;
-    R ar = HC<R>::k(1.410474) + HC<R>::k(.5641896) * ur, ai = HC<R>::k(.5641896) * ui;
+    const double ur = fma(-x, x, dmul(y, y)), ui = dmul(dmul(-2.0, x), y);
+    const double ar = fma(.5641896, ur, 1.410474), ai = dmul(.5641896, ui);
     /* N = T * a, T = (y, -x) */
-    R nr = y * ar + x * ai, ni = y * ai - x * ar;
+    const double nr = fma(x, ai, dmul(y, ar)), ni = fma(y, ai, -dmul(x, ar));
     /* D = .75 + U*(3+U) */
-    R br = R(3) + ur;
-    R dr = HC<R>::k(.75) + (ur * br - ui * ui);
-    R di = ur * ui + ui * br;
+    const double br = dadd(3.0, ur);
+    const double dr = dadd(.75, fma(ur, br, -dmul(ui, ui)));
+    const double di = fma(ur, ui, dmul(ui, br));
     return re_div(nr, ni, dr, di);
 }
 
-/* FP32 region II with every rounding written out, so that the sums do not
- * depend on which products the compiler contracts at a call site */
+/* FP32: one approximate reciprocal (1 ulp) instead of an IEEE division */
 template <>
 __device__ __forceinline__ float hum_region2<float>(float x, float y)
 {
@@ -114,61 +112,56 @@ __device__ __forceinline__ float hum_region2<float>(float x, float y)
                      rcp_approx(__fmaf_rn(dr, dr, __fmul_rn(di, di))));
 }
 
-template <typename R>
-__device__ __forceinline__ void cmul_add(R& pr, R& pi, R tr, R ti, R c)
+/* p = c + t*p */
+__device__ __forceinline__ void cmul_add(double& pr, double& pi, double tr, double ti, double c)
 {
-    /* p = c + t*p */
-    R r = tr * pr - ti * pi;
-    R i = tr * pi + ti * pr;
-    pr = c + r; pi = i;
+    const double r = fma(tr, pr, -dmul(ti, pi));
+    pi = fma(tr, pi, dmul(ti, pr));
+    pr = dadd(c, r);
 }
 
-template <typename R>
-__device__ __forceinline__ R hum_region3(R x, R y)
+__device__ __forceinline__ double hum_region3(double x, double y)
 {
-    R tr = y, ti = -x;
-    R nr = HC<R>::k(.5642236), ni = R(0);
-    cmul_add(nr, ni, tr, ti, HC<R>::k(3.778987));
-    cmul_add(nr, ni, tr, ti, HC<R>::k(11.96482));
-    cmul_add(nr, ni, tr, ti, HC<R>::k(20.20933));
-    cmul_add(nr, ni, tr, ti, HC<R>::k(16.4955));
-    R dr = R(1), di = R(0);
-    cmul_add(dr, di, tr, ti, HC<R>::k(6.699398));
-    cmul_add(dr, di, tr, ti, HC<R>::k(21.69274));
-    cmul_add(dr, di, tr, ti, HC<R>::k(39.27121));
-    cmul_add(dr, di, tr, ti, HC<R>::k(38.82363));
-    cmul_add(dr, di, tr, ti, HC<R>::k(16.4955));
+    const double tr = y, ti = -x;
+    double nr = .5642236, ni = 0.0;
+    cmul_add(nr, ni, tr, ti, 3.778987);
+    cmul_add(nr, ni, tr, ti, 11.96482);
+    cmul_add(nr, ni, tr, ti, 20.20933);
+    cmul_add(nr, ni, tr, ti, 16.4955);
+    double dr = 1.0, di = 0.0;
+    cmul_add(dr, di, tr, ti, 6.699398);
+    cmul_add(dr, di, tr, ti, 21.69274);
+    cmul_add(dr, di, tr, ti, 39.27121);
+    cmul_add(dr, di, tr, ti, 38.82363);
+    cmul_add(dr, di, tr, ti, 16.4955);
     return re_div(nr, ni, dr, di);
 }
 
-template <typename R> __device__ __forceinline__ R expcos(R a, R b);
-template <> __device__ __forceinline__ float expcos<float>(float a, float b) { return expf(a) * cosf(b); }
-template <> __device__ __forceinline__ double expcos<double>(double a, double b) { return exp(a) * cos(b); }
+__device__ __forceinline__ float expcos(float a, float b) { return expf(a) * cosf(b); }
 
-template <typename R>
-__device__ __forceinline__ R hum_region4(R x, R y)
+__device__ __forceinline__ double hum_region4(double x, double y)
 {
     /* exp(U) - T P(U)/Q(U); P, Q written as polynomials in V = -U */
-    R ur = y * y - x * x, ui = R(-2) * x * y;
-    R vr = -ur, vi = -ui;
-    R pr = HC<R>::k(.56419), pi = R(0);
-    cmul_add(pr, pi, vr, vi, HC<R>::k(1.320522));
-    cmul_add(pr, pi, vr, vi, HC<R>::k(35.76683));
-    cmul_add(pr, pi, vr, vi, HC<R>::k(219.0313));
-    cmul_add(pr, pi, vr, vi, HC<R>::k(1540.787));
-    cmul_add(pr, pi, vr, vi, HC<R>::k(3321.9905));
-    cmul_add(pr, pi, vr, vi, HC<R>::k(36183.31));
-    R qr = R(1), qi = R(0);
-    cmul_add(qr, qi, vr, vi, HC<R>::k(1.841439));
-    cmul_add(qr, qi, vr, vi, HC<R>::k(61.57037));
-    cmul_add(qr, qi, vr, vi, HC<R>::k(364.2191));
-    cmul_add(qr, qi, vr, vi, HC<R>::k(2186.181));
-    cmul_add(qr, qi, vr, vi, HC<R>::k(9022.228));
-    cmul_add(qr, qi, vr, vi, HC<R>::k(24322.84));
-    cmul_add(qr, qi, vr, vi, HC<R>::k(32066.6));
+    const double ur = fma(-x, x, dmul(y, y)), ui = dmul(dmul(-2.0, x), y);
+    const double vr = -ur, vi = -ui;
+    double pr = .56419, pi = 0.0;
+    cmul_add(pr, pi, vr, vi, 1.320522);
+    cmul_add(pr, pi, vr, vi, 35.76683);
+    cmul_add(pr, pi, vr, vi, 219.0313);
+    cmul_add(pr, pi, vr, vi, 1540.787);
+    cmul_add(pr, pi, vr, vi, 3321.9905);
+    cmul_add(pr, pi, vr, vi, 36183.31);
+    double qr = 1.0, qi = 0.0;
+    cmul_add(qr, qi, vr, vi, 1.841439);
+    cmul_add(qr, qi, vr, vi, 61.57037);
+    cmul_add(qr, qi, vr, vi, 364.2191);
+    cmul_add(qr, qi, vr, vi, 2186.181);
+    cmul_add(qr, qi, vr, vi, 9022.228);
+    cmul_add(qr, qi, vr, vi, 24322.84);
+    cmul_add(qr, qi, vr, vi, 32066.6);
     /* T * P, T = (y, -x) */
-    R nr = y * pr + x * pi, ni = y * pi - x * pr;
-    return expcos(ur, ui) - re_div(nr, ni, qr, qi);
+    const double nr = fma(x, pi, dmul(y, pr)), ni = fma(y, pi, -dmul(x, pr));
+    return dsub(dmul(exp(ur), cos(ui)), re_div(nr, ni, qr, qi));
 }
 
 /* p(z) of a polynomial with real coefficients c[0..N] (ascending) at the
@@ -222,7 +215,7 @@ __device__ __forceinline__ double hum_region4_core(double x, double y)
     quad_horner<7>(cq, s, q, qu, qv);
     const double pr = fma(vr, pv, pu), pi = vi * pv, qr = fma(vr, qv, qu), qi = vi * qv;
     const double nr = fma(y, pr, x * pi), ni = fma(y, pi, -(x * pr));
-    return (double)expcos<float>((float)-vr, (float)-vi) -
+    return (double)expcos((float)-vr, (float)-vi) -
            fma(nr, qr, ni * qi) * rcp_f64(fma(qr, qr, qi * qi));
 }
 
@@ -230,8 +223,8 @@ __device__ __forceinline__ double hum_region4_core(double x, double y)
 static __device__ __noinline__ double hum_core_f64(double x, double y)
 {
     if (dadd(x, y) >= 5.5) return hum_region2<double>(x, y);
-    if (y >= dsub(dmul(0.195, x), 0.176)) return hum_region3<double>(x, y);
-    return hum_region4<double>(x, y);
+    if (y >= dsub(dmul(0.195, x), 0.176)) return hum_region3(x, y);
+    return hum_region4(x, y);
 }
 
 /* --------------------------------------------------- Gauss-Hermite Voigt

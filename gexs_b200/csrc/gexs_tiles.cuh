@@ -2046,8 +2046,8 @@ template <int PREC, int REGION>
 __device__ __noinline__ double core_term(double x, double y, double amp)
 {
     if (REGION == 2) return amp * hum_region2<double>(x, y);
-    if (REGION == 3) return amp * (PREC == GEXS_FP64 ? hum_region3<double>(x, y) : hum_region3_core(x, y));
-    return amp * (PREC == GEXS_FP64 ? hum_region4<double>(x, y) : hum_region4_core(x, y));
+    if (REGION == 3) return amp * (PREC == GEXS_FP64 ? hum_region3(x, y) : hum_region3_core(x, y));
+    return amp * (PREC == GEXS_FP64 ? hum_region4(x, y) : hum_region4_core(x, y));
 }
 __device__ __forceinline__ double core_term2_f32(const CoreLine& l, int t)
 {
@@ -2296,7 +2296,7 @@ core_kernel(const KArgs args)
                     scatter_phase<PREC>(side ? c3b : c2a, side ? c2b : c3a, lane, L, row, LO, scr,
                         [&](const CoreLine& l, int t) {
                             const double x = x_of(l, t);
-                            return l.amp * (PREC == GEXS_FP64 ? hum_region4<double>(x, l.y)
+                            return l.amp * (PREC == GEXS_FP64 ? hum_region4(x, l.y)
                                                               : hum_region4_core(x, l.y));
                         },
                         [&](const CoreLine& l, int t) {
@@ -2305,7 +2305,7 @@ core_kernel(const KArgs args)
                 scatter_phase<PREC>(c3a, c3b, lane, L, row, LO, scr,
                     [&](const CoreLine& l, int t) {
                         const double x = x_of(l, t);
-                        return l.amp * (PREC == GEXS_FP64 ? hum_region3<double>(x, l.y)
+                        return l.amp * (PREC == GEXS_FP64 ? hum_region3(x, l.y)
                                                           : hum_region3_core(x, l.y));
                     },
                     [&](const CoreLine& l, int t) {
