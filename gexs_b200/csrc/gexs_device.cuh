@@ -363,9 +363,9 @@ __device__ __forceinline__ double gh_sum_f64_near(double x, double y2)
     double acc = 0.0;
 #pragma unroll
     for (int k = 0; k < GH<NODES>::NP; ++k) {
-        const double d1 = x - gh_t<NODES>(k), d2 = x + gh_t<NODES>(k);
+        const double d1 = dsub(x, gh_t<NODES>(k)), d2 = dadd(x, gh_t<NODES>(k));
         const double A = fma(d1, d1, y2), B = fma(d2, d2, y2);
-        acc = fma(gh_w<NODES>(k) * (A + B), rcp_f64(A * B), acc);
+        acc = fma(dmul(gh_w<NODES>(k), dadd(A, B)), rcp_f64(dmul(A, B)), acc);
     }
     return acc;
 }
@@ -396,10 +396,11 @@ __device__ __forceinline__ double gh_sum_f64_far(double x, double y2)
     constexpr double c[7] = {gh_moment<NODES>(0), gh_moment<NODES>(1), gh_moment<NODES>(2),
                              gh_moment<NODES>(3), gh_moment<NODES>(4), gh_moment<NODES>(5),
                              gh_moment<NODES>(6)};
-    const double x2 = x * x, inv = rcp_f64(x2 + y2), i2 = inv * inv;
+    /* every rounding written out: two copies give the same bits */
+    const double x2 = dmul(x, x), inv = rcp_f64(fma(x, x, y2)), i2 = dmul(inv, inv);
     double a, b;
-    quad_horner<6>(c, 2.0 * (x2 - y2) * i2, i2, a, b);
-    return fma(b, fma(3.0, x2, -y2) * i2, a) * inv;
+    quad_horner<6>(c, dmul(dmul(2.0, fma(x, x, -y2)), i2), i2, a, b);
+    return dmul(fma(b, dmul(fma(3.0, x2, -y2), i2), a), inv);
 }
 
 /* ------------------------------------------------ bin-averaged erf difference */

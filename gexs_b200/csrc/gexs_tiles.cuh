@@ -79,7 +79,7 @@ struct __align__(16) RecF64 {   /* 48 bytes; GH */
                               |x| >= GH_FAR; 16 + w: all in the window;
                               bit 24: IEEE form (y < 1e-100, |x| or y may
                               exceed 1e60, or a 1e300)                       */
-    int    pad0, pad1;
+    int    na, nb;         /* bins t < na or t >= nb: |x| >= GH_FAR           */
 };
 
 /* FP32 Voigt record (64 bytes): the main-loop constants of a line in a
@@ -551,20 +551,23 @@ __device__ __forceinline__ void make_rec(RecF64& q, const Derived<PK>& d, const 
     q.nu = d.nu; q.invw = d.invw; q.y2 = d.y * d.y;
     q.a = dmul(dmul(d.S, d.invw), J.out_scale) * dmul(d.y, GEXS_INV_PI);
     q.win = d.win;
-    q.pad0 = q.pad1 = 0;
     const int a = lo16(d.win), b = hi16(d.win);
     const double dfar = fmax(fabs(d.nu - T.f0), fabs(d.nu - T.fl));
     const bool general = !(d.y >= 1e-100) || !(d.y < 1e60) || !(dfar * d.invw < 1e60) ||
                          !(fabs(q.a) < 1e300);
-    /* distance of GH_FAR in bins */
+    /* GH_FAR in bins of the grid, so that a bin takes the same form in a
+     * tile of any shape */
     const double reach = GH_FAR / d.invw * T.inv_dnu + 1.0;
+    const double at = dmul(dsub(d.nu, J.nu_start), T.inv_dnu), j0 = (double)T.j0;
+    q.na = (int)fmin(fmax(dsub(floor(dsub(at, reach)), j0), -1.0), 65536.0);
+    q.nb = (int)fmin(fmax(dsub(ceil(dadd(at, reach)), j0), -1.0), 65536.0);
     int m = general ? 1 << 24 : 0;
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) {
         const int r0 = 32 * B * w, r1 = r0 + 32 * B;
         if (!(a < r1 && b > r0)) continue;
         m |= 1 << w;
-        if (d.tc + reach < (double)r0 || d.tc - reach > (double)r1) m |= 1 << (8 + w);
+        if (r1 <= q.na || r0 >= q.nb) m |= 1 << (8 + w);
         if (a <= r0 && b >= r1) m |= 1 << (16 + w);
     }
     q.mask = d.win == 0 ? 0 : m;
@@ -1014,15 +1017,21 @@ __device__ __forceinline__ void lines_f64(const RecF64* __restrict__ rec, int nr
             const bool full = mask & (1 << 16);
 #pragma unroll
             for (int k = 0; k < B; ++k) {
-                const double v = gh_sum_f64_far<NODES>((fbin[k] - nu) * invw, y2);
+                const double v = gh_sum_f64_far<NODES>(dmul(dsub(fbin[k], nu), invw), y2);
                 const bool in = full || (unsigned)(tl + 32 * k - wa) < wn;
                 acc[k] = fma(a, in ? v : 0.0, acc[k]);     /* a is finite */
             }
         } else {
+            /* groups of 32 bins, as in every launch shape: far or near */
+            const int na = q.na, nb = q.nb;
 #pragma unroll
             for (int k = 0; k < B; ++k) {
-                if ((unsigned)(tl + 32 * k - wa) >= wn) continue;
-                acc[k] = fma(a, gh_sum_f64_near<NODES>((fbin[k] - nu) * invw, y2), acc[k]);
+                const int c = warp * 32 * B + 32 * k;
+                if ((unsigned)(c + lane - wa) >= wn) continue;
+                const double x = dmul(dsub(fbin[k], nu), invw);
+                const double v = c + 32 <= na || c >= nb ? gh_sum_f64_far<NODES>(x, y2)
+                                                         : gh_sum_f64_near<NODES>(x, y2);
+                acc[k] = fma(a, v, acc[k]);
             }
         }
     }
