@@ -201,7 +201,7 @@ __device__ __forceinline__ void reach_range(const gexs_job& J, double f0, double
         if (k < 1.0) vhi = fmin(vhi, (fl + h) / (1.0 - k));
     }
     vlo -= margin; vhi += margin;
-    if (vlo < 1e-6 + margin) vlo = -1.0;       /* nu == 0 lines count as 1e-6 */
+    if (vlo < 1e-6 + margin) vlo = fmin(vlo, -1.0);   /* nu == 0 lines count as 1e-6 */
 }
 
 /* window of a line inside the tile as [a, b) (tile-relative) */
