@@ -55,7 +55,7 @@ cudaError_t launch_tiles(int pk, int prec, const gexs_job* d_jobs, const int* d_
  * rounded total does not depend on their order: a result is the same for
  * every tile shape, slice length and batch.  Sub-lists of one list start
  * at multiples of it. */
-constexpr int SUM_BLOCK = 512;
+constexpr int SUM_BLOCK = GEXS_LINE_BLOCK;
 
 /* doubles of a partial row: a value per bin, (hi, lo) in the FP64 forms */
 __host__ __device__ inline int row_doubles(int prec, int tile_w)

@@ -16,8 +16,6 @@ namespace {
 const int kCopyChunks = 64;                     /* pieces of an overlapped line copy */
 const int kSegments = 6;                        /* grid segments of the first launch  */
 const double kSegmentFrac[kSegments] = {1.0 / 64, 1.0 / 32, 1.0 / 8, 1.0 / 4, 1.0 / 2, 1.0};
-const size_t kLineBlock = 512;                  /* SUM_BLOCK of csrc/gexs_internal.h: the FP64
-                                                   sums' line blocks start at its multiples */
 const int64_t kSegmentAlign = 4096;             /* widest tile: 32 lanes x 16 bins x 8 warps */
 const size_t kSegmentMinLines = (size_t)1 << 21;
 const size_t kSamples = 8192;
@@ -297,7 +295,7 @@ int B200Manager::run_segmented()
             const double m = 8.0 * j.dnu + 1e-8 * (std::fabs(fl) + j.cutoff);
             size_t L0 = std::min(lines_below(f0 - j.cutoff - m), ne);
             size_t L1 = std::min(lines_upto(fl + j.cutoff + m), ne);
-            L0 &= ~(size_t)(kLineBlock - 1);
+            L0 &= ~(size_t)(GEXS_LINE_BLOCK - 1);
             if (L1 < L0) L1 = L0;
             gexs_job p = j;
             p.start_idx = b0;

@@ -104,9 +104,6 @@ void B200MultiManager::TransferVectors(size_t Nener, double* h_energies, double*
     int st = gexs_shard_plan(h_nu, (int64_t)Nener, freq_[0], dfreq_, 0, npoints_, reach, kAlign,
                              n, bounds_.data(), lo_.data(), hi_.data());
     if (st) { fail(st); return; }
-    /* the FP64 sums' line blocks (SUM_BLOCK of csrc/gexs_internal.h) as on
-     * one device */
-    for (int64_t& l : lo_) l &= ~(int64_t)511;
     for (int g = 0; g < n; ++g) {
         const size_t a = (size_t)lo_[g];
         m_[g]->TransferVectors((size_t)(hi_[g] - lo_[g]), h_energies + a, h_nu + a, h_aif + a,

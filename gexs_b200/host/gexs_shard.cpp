@@ -12,8 +12,10 @@
  * number of lines within `reach` of it, sampled every 256th bin from the
  * sorted centres; interior cuts fall on multiples of `align` bins from
  * start_idx, so the tiles of every shard are tiles of the unsplit launch
- * (tile widths divide 4096) and a shard computes exactly the sums that the
- * single launch computes for its bins.
+ * (tile widths divide 4096), and a shard's lines begin at a multiple of
+ * GEXS_LINE_BLOCK (the FP64 form sums blocks of that many lines by list
+ * index), so a shard computes exactly the sums that the single launch
+ * computes for its bins.
  */
 #include <algorithm>
 #include <cmath>
@@ -59,7 +61,7 @@ extern "C" int gexs_shard_plan(const double* h_nu, int64_t nlines, double nu_sta
             continue;
         }
         const double fa = f(bounds[r]), fb = f(bounds[r + 1] - 1);
-        line_lo[r] = (int64_t)(std::lower_bound(nb, ne, fa - reach) - nb);
+        line_lo[r] = (int64_t)(std::lower_bound(nb, ne, fa - reach) - nb) / GEXS_LINE_BLOCK * GEXS_LINE_BLOCK;
         line_hi[r] = (int64_t)(std::upper_bound(nb, ne, fb + reach) - nb);
     }
     return GEXS_OK;

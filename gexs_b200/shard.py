@@ -10,6 +10,10 @@ line chunks to GPUs and sums full-size grids on the host
 """
 import numpy as np
 
+#: GEXS_LINE_BLOCK of include/gexs_b200.h: FP64 sums are taken over blocks of
+#: this many lines by list index, so a sub-list begins at a multiple of it
+LINE_BLOCK = 512
+
 
 def equal_slices(grid_points, world):
     """[start_idx, n_points) per rank, equal bin counts."""
@@ -38,12 +42,12 @@ def balanced_slices(nu_sorted, nu_start, dnu, grid_points, cutoff, world, sample
 
 def line_range(nu_sorted, nu_start, dnu, start_idx, n_points, cutoff):
     """Indices [lo, hi) of the lines a bin range can reach (for ranks that
-    hold only their own part of the list)."""
+    hold only their own part of the list); lo is a multiple of LINE_BLOCK."""
     nu = np.asarray(nu_sorted)
     f0 = nu_start + start_idx * dnu
     f1 = nu_start + (start_idx + max(n_points, 1) - 1) * dnu
     margin = 2.0 * dnu + 1e-9 * (abs(f1) + cutoff)
-    lo = int(np.searchsorted(nu, f0 - cutoff - margin, side="left"))
+    lo = int(np.searchsorted(nu, f0 - cutoff - margin, side="left")) // LINE_BLOCK * LINE_BLOCK
     hi = int(np.searchsorted(nu, f1 + cutoff + margin, side="right"))
     return lo, hi
 

@@ -112,8 +112,12 @@ typedef struct gexs_lines {
  *   Voigt-Quad: same with K = Gauss-Hermite K_N
  *   Doppler, Gaussian: term_j = (S*(erf(xp)-erf(xm)))*out_scale,
  *               xp = invw*(|f_j-nu0|+dnu/2), xm = invw*(|f_j-nu0|-dnu/2)
- *   out[j] = (accumulate ? out[j] : 0) + sum over lines in nu order of term_j
+ *   out[j] = (accumulate ? out[j] : 0) + sum over lines of term_j
+ * FP64 sums are taken over blocks of GEXS_LINE_BLOCK lines by list index, so
+ * a bin range computed from a part of the list has the bits of the whole
+ * list's when that part begins at a multiple of it.
  */
+#define GEXS_LINE_BLOCK 512
 typedef struct gexs_job {
     gexs_lines lines;        /* device pointers                                   */
     double*    out;          /* device, grid_points doubles                        */
@@ -433,8 +437,9 @@ int gexs_partition(gexs_ctx* ctx, const double* d_energy, const int32_t* d_g,
  * centres h_nu (host) - interior cuts on multiples of `align` bins from
  * start_idx (4096 makes every shard's tiles the tiles of one unsplit
  * launch), and give each range the index range [line_lo[r], line_hi[r]) of
- * the lines within `reach` of it.  Host computation.  No counterpart in
- * the reference (its multi-GPU manager splits by line chunks,
+ * the lines within `reach` of it, line_lo[r] rounded down to a multiple of
+ * GEXS_LINE_BLOCK.  Host computation.  No counterpart in the reference (its
+ * multi-GPU manager splits by line chunks,
  * Managers/Accel/GPU/MultiGPUManager.cpp:59-63). */
 int gexs_shard_plan(const double* h_nu, int64_t nlines, double nu_start, double dnu,
                     int64_t start_idx, int64_t n_points, double reach, int align, int nshards,
