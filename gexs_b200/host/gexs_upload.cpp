@@ -122,6 +122,12 @@ cudaError_t upload(Uploader* u, const gexs_upload_piece* pieces, int n, cudaStre
     std::vector<char> pg(n, 0);
     for (int i = 0; i < n; ++i)
         if (pieces[i].bytes && pageable(pieces[i].src)) { pg[i] = 1; total += pieces[i].bytes; }
+    if (total) {
+        /* a captured copy would read its source, or the slot, at each replay */
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+        if (cap != cudaStreamCaptureStatusNone) return cudaErrorStreamCaptureUnsupported;
+    }
     std::unique_lock<std::mutex> lock(g_ring.use, std::defer_lock);
     const unsigned hw = std::thread::hardware_concurrency();
     const int nt = (int)std::min<size_t>(kThreads, hw > 1 ? hw - 1 : 1);

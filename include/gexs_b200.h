@@ -238,8 +238,9 @@ int gexs_ctx_check(gexs_ctx* ctx, void* stream);
  * `event` (a cudaEvent_t, or NULL) is recorded there.  Pageable sources go
  * through a ring of pinned buffers that several host threads fill (8 MiB
  * per process, allocated by the first call of 4 MiB or more, freed with the
- * last context) and have been read when the call returns; pinned sources are copied directly and must
- * stay valid until the stream has passed the copy. */
+ * last context) and have been read when the call returns; they are refused
+ * (GEXS_ERR_CUDA) on a capturing stream.  Pinned sources are copied directly
+ * and must stay valid until the stream has passed the copy. */
 typedef struct gexs_upload_piece {
     void*       dst;      /* device */
     const void* src;      /* host   */

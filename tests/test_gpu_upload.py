@@ -65,3 +65,21 @@ def test_threads_share_a_context(gpu_ctx):
         t.join()
     for g, w in zip(got, want):
         assert np.array_equal(g.cpu().numpy()[:w.size], w)
+
+
+def test_pageable_source_is_refused_under_capture(gpu_ctx):
+    """A captured copy would read the staging slot at each replay; later
+    uploads are unaffected."""
+    rng = np.random.Generator(np.random.PCG64(12))
+    want = rng.integers(0, 256, 17 * MIB, dtype=np.uint8)
+    dev = torch.zeros(want.size, dtype=torch.uint8, device="cuda")
+    p = (Piece * 1)(Piece(dev.data_ptr(), want.ctypes.data, want.size, None))
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        status = lib().gexs_ctx_upload(gpu_ctx.h, p, 1, C.c_void_p(stream.cuda_stream))
+    assert status != 0
+    got = _upload(gpu_ctx, [want], stream)[0]
+    stream.synchronize()
+    assert np.array_equal(got.cpu().numpy(), want)
