@@ -14,6 +14,8 @@
  */
 #include <algorithm>
 #include <atomic>
+#include <chrono>
+#include <condition_variable>
 #include <cstring>
 #include <mutex>
 #include <thread>
@@ -113,6 +115,60 @@ void uploader_destroy(Uploader* u)
     delete u;
 }
 
+/* Waits poll for kPoll and then sleep: a chunk takes some 25 us, and a sleep
+ * and wake-up at every chunk made the manager pass 24 ms long (13.5 with
+ * polling, 20.3 with the driver's staging); but the stream may have other
+ * work before the copies, and the host's cores may be fewer than the
+ * threads (a quota). */
+constexpr std::chrono::microseconds kPoll(1000);
+
+template <typename F>
+static bool poll(const F& done)
+{
+    const auto end = std::chrono::steady_clock::now() + kPoll;
+    do {
+        if (done()) return true;
+        std::this_thread::yield();
+    } while (std::chrono::steady_clock::now() < end);
+    return false;
+}
+
+struct Waiters {
+    std::mutex mu;
+    std::condition_variable cv;
+    std::atomic<int> asleep{0};
+    template <typename F>
+    void wait(const F& done)
+    {
+        if (poll(done)) return;
+        std::unique_lock<std::mutex> g(mu);
+        asleep.fetch_add(1);
+        cv.wait(g, done);
+        asleep.fetch_sub(1);
+    }
+    /* after the change that a waiter looks for: a waiter counts itself before
+     * it looks for the last time, so one of the two sees the other */
+    void wake()
+    {
+        if (asleep.load() == 0) return;
+        { std::lock_guard<std::mutex> g(mu); }
+        cv.notify_all();
+    }
+};
+
+/* the event's work is done (waited for) */
+static bool passed(cudaEvent_t e)
+{
+    cudaError_t r = cudaErrorNotReady;
+    int n = 0;
+    poll([&] { return n++ % 32 == 0 && (r = cudaEventQuery(e)) != cudaErrorNotReady; });
+    while (r == cudaErrorNotReady) {
+        std::this_thread::sleep_for(std::chrono::microseconds(200));
+        r = cudaEventQuery(e);
+    }
+    return r == cudaSuccess;
+}
+
 cudaError_t upload(Uploader* u, const gexs_upload_piece* pieces, int n, cudaStream_t s)
 {
     struct Chunk { void* dst; const void* src; size_t bytes; cudaEvent_t after; bool staged; };
@@ -151,22 +207,21 @@ cudaError_t upload(Uploader* u, const gexs_upload_piece* pieces, int n, cudaStre
     for (auto& f : filled) f.store(0, std::memory_order_relaxed);
     std::atomic<size_t> next{0}, queued{0};
     std::atomic<bool> stop{false};
+    Waiters room, ready;
     auto work = [&]() {
         cudaSetDevice(u->device);
         for (;;) {
             const size_t k = next.fetch_add(1);
             if (k >= staged.size()) return;
-            while (queued.load(std::memory_order_acquire) + kSlots <= k) {
-                if (stop.load(std::memory_order_relaxed)) return;
-                std::this_thread::yield();
-            }
-            if (stop.load(std::memory_order_relaxed)) return;
+            room.wait([&] { return stop.load() || queued.load() + kSlots > k; });
+            if (stop.load()) return;
             const int slot = (int)(k % kSlots);
             const cudaEvent_t last = g_ring.last[slot];
-            const bool ok = !last || cudaEventSynchronize(last) == cudaSuccess;
+            const bool ok = !last || passed(last);
             const Chunk& c = chunks[staged[k]];
             if (ok) std::memcpy(g_ring.pinned + slot * kSlotBytes, c.src, c.bytes);
-            filled[k].store(ok ? 1 : -1, std::memory_order_release);
+            filled[k].store(ok ? 1 : -1);
+            ready.wake();
             if (!ok) return;
         }
     };
@@ -183,21 +238,22 @@ cudaError_t upload(Uploader* u, const gexs_upload_piece* pieces, int n, cudaStre
     for (const Chunk& c : chunks) {
         const void* src = c.src;
         if (c.staged && !th.empty()) {
-            int f;
-            while ((f = filled[k].load(std::memory_order_acquire)) == 0) std::this_thread::yield();
-            if (f < 0) { e = cudaErrorUnknown; break; }
+            ready.wait([&] { return filled[k].load() != 0; });
+            if (filled[k].load() < 0) { e = cudaErrorUnknown; break; }
             src = g_ring.pinned + (k % kSlots) * kSlotBytes;
         }
         if (c.bytes) e = cudaMemcpyAsync(c.dst, src, c.bytes, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess && c.staged && !th.empty()) {
             e = cudaEventRecord(u->ev[k % kSlots], s);
             g_ring.last[k % kSlots] = u->ev[k % kSlots];
-            queued.store(++k, std::memory_order_release);
+            queued.store(++k);
+            room.wake();
         }
         if (e == cudaSuccess && c.after) e = cudaEventRecord(c.after, s);
         if (e != cudaSuccess) break;
     }
     stop.store(true);
+    room.wake();
     for (std::thread& t : th) t.join();
     return e;
 }

@@ -4,6 +4,7 @@ MiB), with empty and odd pieces; a pageable source may be overwritten as soon
 as the call returns; calls from several threads on one context."""
 import ctypes as C
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -83,3 +84,24 @@ def test_pageable_source_is_refused_under_capture(gpu_ctx):
     got = _upload(gpu_ctx, [want], stream)[0]
     stream.synchronize()
     assert np.array_equal(got.cpu().numpy(), want)
+
+
+def test_waiting_for_the_stream_costs_no_processor_time(gpu_ctx):
+    """With other work queued before the copies the threads sleep: the process
+    takes far less processor time than one core spinning for that long."""
+    stream = torch.cuda.Stream()
+    want = np.full(40 * MIB, 7, dtype=np.uint8)
+    _upload(gpu_ctx, [want], stream)
+    stream.synchronize()
+    dev = torch.zeros(want.size, dtype=torch.uint8, device="cuda")
+    p = (Piece * 1)(Piece(dev.data_ptr(), want.ctypes.data, want.size, None))
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(1000000000)                     # about half a second
+    wall, cpu = time.perf_counter(), time.process_time()
+    check(lib().gexs_ctx_upload(gpu_ctx.h, p, 1, C.c_void_p(stream.cuda_stream)), "upload")
+    wall, cpu = time.perf_counter() - wall, time.process_time() - cpu
+    stream.synchronize()
+    assert wall > 0.2
+    assert cpu < 0.5 * wall, (cpu, wall)
+    assert np.array_equal(dev.cpu().numpy(), want)
