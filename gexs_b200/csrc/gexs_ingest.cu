@@ -480,7 +480,19 @@ struct DevBuf {
         if (pooled) cudaFreeAsync(p, stream);
         else cudaFree(p);
     }
-    cudaError_t alloc(size_t n) { return cudaMalloc(&p, n ? n : 1); }
+    cudaError_t alloc(gexs_ctx* ctx, size_t n)
+    {
+        cudaError_t e = cudaMalloc(&p, n ? n : 1);
+        if (e == cudaErrorMemoryAllocation && ctx_pool(ctx)) {
+            /* the pool may hold scratch that is no longer in use */
+            cudaGetLastError();
+            cudaStreamSynchronize(0);
+            cudaMemPoolTrimTo(ctx_pool(ctx), 0);
+            e = cudaMalloc(&p, n ? n : 1);
+        }
+        if (e != cudaSuccess) p = nullptr;
+        return e;
+    }
     cudaError_t scratch(gexs_ctx* ctx, size_t n, cudaStream_t s)
     {
         pooled = true; stream = s;
@@ -550,7 +562,7 @@ int sort_lines(gexs_ctx* ctx, int64_t nrec, DevBuf& nu, DevBuf& el, DevBuf& A, D
 {
     const size_t n8 = sizeof(double) * nrec;
     DevBuf k2, i1, i2, t2;
-    if (k2.alloc(n8) != cudaSuccess || i1.scratch(ctx, sizeof(int64_t) * nrec, s) != cudaSuccess ||
+    if (k2.alloc(ctx, n8) != cudaSuccess || i1.scratch(ctx, sizeof(int64_t) * nrec, s) != cudaSuccess ||
         i2.scratch(ctx, sizeof(int64_t) * nrec, s) != cudaSuccess)
         return set_error(GEXS_ERR_OOM, "ingest: sort buffers");
     iota_kernel<<<grid_for(ctx, nrec, 256), 256, 0, s>>>(i1.as<int64_t>(), nrec);
@@ -562,7 +574,7 @@ int sort_lines(gexs_ctx* ctx, int64_t nrec, DevBuf& nu, DevBuf& el, DevBuf& A, D
                                     i2.as<int64_t>(), nrec, 0, 64, s);
     const int gg = grid_for(ctx, nrec, 256);
     DevBuf tmp;
-    if (tmp.alloc(n8) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: gather");
+    if (tmp.alloc(ctx, n8) != cudaSuccess) return set_error(GEXS_ERR_OOM, "ingest: gather");
     auto regather8 = [&](DevBuf& arr) {
         gather_kernel<double><<<gg, 256, 0, s>>>(arr.as<double>(), i2.as<int64_t>(), nrec, tmp.as<double>());
         std::swap(arr.p, tmp.p);
@@ -575,10 +587,26 @@ int sort_lines(gexs_ctx* ctx, int64_t nrec, DevBuf& nu, DevBuf& el, DevBuf& A, D
     return e == cudaSuccess ? GEXS_OK : cuda_error(e, "ingest: sort");
 }
 
-/* scratch beyond 1 GiB goes back to the device after a parse */
+/* After a parse the context's pool keeps at most 1 GiB, or what it held
+ * before if that is more; the rest goes back to the device.  Declared before
+ * the buffers, so that it runs after their frees; a free counts once the
+ * host has seen the stream pass it. */
 struct TrimPool {
     gexs_ctx* ctx;
-    ~TrimPool() { if (ctx_pool(ctx)) cudaMemPoolTrimTo(ctx_pool(ctx), (size_t)1 << 30); }
+    uint64_t keep = (uint64_t)1 << 30;
+    static uint64_t reserved(gexs_ctx* c)
+    {
+        uint64_t v = 0;
+        if (ctx_pool(c)) cudaMemPoolGetAttribute(ctx_pool(c), cudaMemPoolAttrReservedMemCurrent, &v);
+        return v;
+    }
+    explicit TrimPool(gexs_ctx* c) : ctx(c) { keep = std::max(keep, reserved(c)); }
+    ~TrimPool()
+    {
+        if (reserved(ctx) <= keep) return;
+        cudaStreamSynchronize(0);
+        cudaMemPoolTrimTo(ctx_pool(ctx), (size_t)keep);
+    }
 };
 
 /* records = non-empty lines, numbered in order: rec[i] for line i, *nrec */
@@ -673,14 +701,14 @@ int gexs_exomol_parse_states(gexs_ctx* ctx, const char* h_text, int64_t nbytes,
     std::memset(out, 0, sizeof(*out));
     cudaSetDevice(ctx_device(ctx));
     cudaStream_t s = 0;
-    const TrimPool trim = {ctx};
+    const TrimPool trim(ctx);
     DevBuf d_text, d_end;
     int64_t nl = 0;
     int st = index_text(ctx, h_text, nbytes, d_text, d_end, &nl, s);
     if (st) return st;
     DevBuf dE, dg, dJ, derr;
-    if (dE.alloc(sizeof(double) * nl) != cudaSuccess || dg.alloc(sizeof(int32_t) * nl) != cudaSuccess ||
-        dJ.alloc(sizeof(int32_t) * nl) != cudaSuccess || derr.scratch(ctx, sizeof(int), s) != cudaSuccess)
+    if (dE.alloc(ctx, sizeof(double) * nl) != cudaSuccess || dg.alloc(ctx, sizeof(int32_t) * nl) != cudaSuccess ||
+        dJ.alloc(ctx, sizeof(int32_t) * nl) != cudaSuccess || derr.scratch(ctx, sizeof(int), s) != cudaSuccess)
         return set_error(GEXS_ERR_OOM, "gexs_exomol_parse_states: tables");
     cudaMemsetAsync(derr.p, 0, sizeof(int), s);
     if (nl > 0)
@@ -712,7 +740,7 @@ int gexs_exomol_parse_trans(gexs_ctx* ctx, const gexs_state_table* states, const
     std::memset(out, 0, sizeof(*out));
     cudaSetDevice(ctx_device(ctx));
     cudaStream_t s = 0;
-    const TrimPool trim = {ctx};
+    const TrimPool trim(ctx);
     DevBuf d_text, d_end;
     int64_t nl = 0;
     int st = index_text(ctx, h_text, nbytes, d_text, d_end, &nl, s);
@@ -753,8 +781,8 @@ int gexs_exomol_parse_trans(gexs_ctx* ctx, const gexs_state_table* states, const
 
     DevBuf nu, el, A, g, gm, nx, derr;
     const size_t n8 = sizeof(double) * nrec, n4 = sizeof(int32_t) * nrec;
-    if (nu.alloc(n8) != cudaSuccess || el.alloc(n8) != cudaSuccess || A.alloc(n8) != cudaSuccess ||
-        g.alloc(n4) != cudaSuccess || gm.alloc(n8) != cudaSuccess || nx.alloc(n8) != cudaSuccess ||
+    if (nu.alloc(ctx, n8) != cudaSuccess || el.alloc(ctx, n8) != cudaSuccess || A.alloc(ctx, n8) != cudaSuccess ||
+        g.alloc(ctx, n4) != cudaSuccess || gm.alloc(ctx, n8) != cudaSuccess || nx.alloc(ctx, n8) != cudaSuccess ||
         derr.scratch(ctx, sizeof(int), s) != cudaSuccess)
         return set_error(GEXS_ERR_OOM, "gexs_exomol_parse_trans: line arrays");
     cudaMemsetAsync(derr.p, 0, sizeof(int), s);
@@ -832,6 +860,7 @@ int gexs_hitran_parse(gexs_ctx* ctx, const char* h_text, int64_t nbytes, double 
     }
     cudaSetDevice(ctx_device(ctx));
     cudaStream_t s = 0;
+    const TrimPool trim(ctx);
     DevBuf d_text, d_end, d_rec;
     int64_t nl = 0, nrec = 0;
     int st = index_text(ctx, h_text, nbytes, d_text, d_end, &nl, s);
@@ -839,8 +868,8 @@ int gexs_hitran_parse(gexs_ctx* ctx, const char* h_text, int64_t nbytes, double 
     if ((st = number_records(ctx, d_text, nbytes, d_end, nl, d_rec, &nrec, s))) return st;
     DevBuf nu, el, A, g, gm, nx;
     const size_t n8 = sizeof(double) * nrec, n4 = sizeof(int32_t) * nrec;
-    if (nu.alloc(n8) != cudaSuccess || el.alloc(n8) != cudaSuccess || A.alloc(n8) != cudaSuccess ||
-        g.alloc(n4) != cudaSuccess || gm.alloc(n8) != cudaSuccess || nx.alloc(n8) != cudaSuccess)
+    if (nu.alloc(ctx, n8) != cudaSuccess || el.alloc(ctx, n8) != cudaSuccess || A.alloc(ctx, n8) != cudaSuccess ||
+        g.alloc(ctx, n4) != cudaSuccess || gm.alloc(ctx, n8) != cudaSuccess || nx.alloc(ctx, n8) != cudaSuccess)
         return set_error(GEXS_ERR_OOM, "gexs_hitran_parse: line arrays");
     if (nl > 0)
         hitran_kernel<<<grid_for(ctx, nl, 256), 256, 0, s>>>(

@@ -200,7 +200,9 @@ typedef struct gexs_launch_cfg {
  * pool keeps its memory between calls (no remapping per call) and never
  * makes an allocation on one stream wait for a free on another, so
  * gexs_run calls on different streams overlap; its memory goes back to the
- * device at gexs_ctx_destroy. */
+ * device at gexs_ctx_destroy.  The text readers take their scratch from it
+ * too (the text, a few words per line) and give back, before they return,
+ * what it then holds beyond 1 GiB and beyond what it held before. */
 int         gexs_ctx_create(int device, gexs_ctx** out);
 int         gexs_ctx_destroy(gexs_ctx* ctx);
 const char* gexs_status_string(int status);
