@@ -280,16 +280,18 @@ static Layout group_layout(const Group& g, bool prep, const gexs_launch_cfg& cfg
         L.os_nitems = up(a); a = L.os_nitems + 256;
         L.os_rows = up(a);   a = L.os_rows + (size_t)L.max_rows * row_doubles(g.prec, W) * sizeof(double);
     }
-    if (core_slices_apply(g.pk, g.prec, W) && nt > 0 &&
-        core_rows(g.jobs.data(), (int)g.jobs.size(), g.prec, W, &L.crows)) {
+    const int cw = core_width(W);
+    const size_t nc = nt * core_subtiles(W);
+    if (core_slices_apply(g.pk, g.prec, W) && nt > 0 && nc <= (size_t)INT32_MAX &&
+        core_rows(g.jobs.data(), (int)g.jobs.size(), g.prec, cw, &L.crows)) {
         L.csliced = true;
-        L.oc_prefix = up(a); a = L.oc_prefix + (nt + 1) * sizeof(int);
-        L.oc_counts = up(a); a = L.oc_counts + nt * sizeof(int);
-        L.oc_rowbase = up(a); a = L.oc_rowbase + nt * sizeof(int);
-        L.oc_ticket = up(a); a = L.oc_ticket + nt * sizeof(int);
-        L.oc_lohi = up(a);   a = L.oc_lohi + 2 * nt * sizeof(long long);
+        L.oc_prefix = up(a); a = L.oc_prefix + (nc + 1) * sizeof(int);
+        L.oc_counts = up(a); a = L.oc_counts + nc * sizeof(int);
+        L.oc_rowbase = up(a); a = L.oc_rowbase + nc * sizeof(int);
+        L.oc_ticket = up(a); a = L.oc_ticket + nc * sizeof(int);
+        L.oc_lohi = up(a);   a = L.oc_lohi + 2 * nc * sizeof(long long);
         L.oc_nitems = up(a); a = L.oc_nitems + 256;
-        L.oc_rows = up(a);   a = L.oc_rows + (size_t)L.crows.alloc * row_doubles(g.prec, W) * sizeof(double);
+        L.oc_rows = up(a);   a = L.oc_rows + (size_t)L.crows.alloc * row_doubles(g.prec, cw) * sizeof(double);
     }
     L.bytes = a + 256;
     return L;

@@ -71,12 +71,17 @@ long long slice_lines(const gexs_job* jobs, int njobs, int prec, int tile_w, int
 /* bytes of partial rows held at a time */
 constexpr long long ROW_BYTES = 1ll << 30;
 
-/* the core kernel's own slices (its line range per tile is reach_range's):
- * only when a tile is one core sub-tile (tile_w <= 1024).  FP32 sums depend
- * on the cut, so it depends on the tile's lines and on the size of the job's
+/* The core kernel takes a tile in sub-tiles of at most CORE_W bins (a row of
+ * doubles per warp in shared memory); a sliced tile of more bins is
+ * core_subtiles core tiles.
+ * Its own slices (its line range per core tile is reach_range's): FP32 only
+ * when a tile is one sub-tile.  FP32 sums depend on the cut, so it depends on the tile's lines and on the size of the job's
  * whole grid alone: a batch, a sub-range and a sub-list of a job are cut
  * alike.  Lines per slice by the tiles of the grid: a job of few tiles has
  * only its lines to fill the chip with. */
+constexpr int CORE_W = 1024;
+__host__ __device__ constexpr int core_width(int tile_w) { return tile_w < CORE_W ? tile_w : CORE_W; }
+__host__ __device__ constexpr int core_subtiles(int tile_w) { return (tile_w + CORE_W - 1) / CORE_W; }
 __host__ __device__ inline long long core_cut(long long grid_points, int tile_w)
 {
     const long long tiles = (grid_points + tile_w - 1) / tile_w;
@@ -92,7 +97,7 @@ __host__ __device__ inline long long core_max_slices(long long grid_points, int 
     const long long use = 8192 / tiles > 1024 ? 8192 / tiles : 1024;
     return fit < 1 ? 1 : fit < use ? fit : use;
 }
-/* slices of a tile with n lines */
+/* slices of a core tile with n lines (tile_w here and above: core_width) */
 __host__ __device__ inline int core_slices(long long n, long long grid_points, int tile_w, int prec)
 {
     const long long per = core_cut(grid_points, tile_w);

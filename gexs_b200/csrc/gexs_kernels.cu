@@ -156,11 +156,19 @@ __device__ __forceinline__ void plan_tile(const KArgs& a, const gexs_job& J, int
     }
 }
 
-/* the same for the core kernel, with its own search (reach_range) */
-__device__ __forceinline__ void plan_core_tile(const KArgs& a, const gexs_job& J, int ti, int tj, int lane)
+/* the same for core tile ti of the core kernel, bins [t0, t0 + CORE_W) of a
+ * tile that ends at tend, with its own search (reach_range) */
+__device__ __forceinline__ void plan_core_tile(const KArgs& a, const gexs_job& J, int ti, int64_t t0,
+                                               int64_t tend, int lane)
 {
-    const int64_t t0 = J.start_idx + (int64_t)tj * a.tile_w;
-    const int64_t tend = min((int64_t)(t0 + a.tile_w), J.start_idx + J.n_points);
+    if (t0 >= tend) {
+        if (lane == 0) {
+            a.csl.lohi[2 * ti] = a.csl.lohi[2 * ti + 1] = 0;
+            a.csl.counts[ti] = 1;
+            a.csl.ticket[ti] = 0;
+        }
+        return;
+    }
     const int jn = (int)min((int64_t)CORE_W, tend - t0);
     const double f0 = grid_f(J.nu_start, J.dnu, t0);
     const double fl = grid_f(J.nu_start, J.dnu, t0 + jn - 1);
@@ -173,7 +181,7 @@ __device__ __forceinline__ void plan_core_tile(const KArgs& a, const gexs_job& J
         const long long n = hi - lo;
         a.csl.lohi[2 * ti] = lo;
         a.csl.lohi[2 * ti + 1] = hi;
-        a.csl.counts[ti] = core_slices(n, J.grid_points, a.tile_w, J.precision);
+        a.csl.counts[ti] = core_slices(n, J.grid_points, core_width(a.tile_w), J.precision);
         a.csl.ticket[ti] = 0;
     }
 }
@@ -241,7 +249,13 @@ __global__ void __launch_bounds__(SETUP_NT) setup_kernel(const KArgs a, int npla
         int tj = 0;
         const gexs_job& J = a.jobs[tile_job(a, ti, &tj)];
         if (a.sl.prefix) plan_tile(a, J, ti, tj, lane);
-        if (a.csl.prefix) plan_core_tile(a, J, ti, tj, lane);
+        if (a.csl.prefix) {
+            const int64_t t0 = J.start_idx + (int64_t)tj * a.tile_w;
+            const int64_t tend = min((int64_t)(t0 + a.tile_w), J.start_idx + J.n_points);
+            const int ns = core_subtiles(a.tile_w);
+            for (int k = 0; k < ns; ++k)
+                plan_core_tile(a, J, ti * ns + k, t0 + (int64_t)k * CORE_W, tend, lane);
+        }
     }
     __threadfence();
     __syncthreads();
@@ -251,7 +265,7 @@ __global__ void __launch_bounds__(SETUP_NT) setup_kernel(const KArgs a, int npla
     __threadfence();
     if (a.sl.prefix) scan_slices(a.sl, a.nitems, a.err, tmp);
     __syncthreads();
-    if (a.csl.prefix) scan_slices(a.csl, a.nitems, a.err, tmp);
+    if (a.csl.prefix) scan_slices(a.csl, a.nitems * core_subtiles(a.tile_w), a.err, tmp);
 }
 }  // namespace
 
@@ -303,7 +317,8 @@ bool slices_apply(int pk, int prec) { return !(pk == PK_ERF && prec == GEXS_FP64
 
 bool core_slices_apply(int pk, int prec, int tile_w)
 {
-    return (pk == PK_VOIGT || (pk == PK_ERF && prec == GEXS_FP64)) && tile_w <= CORE_W;
+    return (pk == PK_VOIGT || (pk == PK_ERF && prec == GEXS_FP64)) &&
+           (tile_w <= CORE_W || prec == GEXS_FP64);
 }
 
 /* A split tile of n lines has ceil(n / per) <= n / per + 1 slices, so for m

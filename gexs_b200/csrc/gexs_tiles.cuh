@@ -1993,11 +1993,7 @@ voigt_ws_kernel(const KArgs args)
  * 5.0 ms for a dense 2e7-line list at 1 bar, 33 against 23 us for 3000
  * lines on 6001 bins.  Instruction fetches bound the dense case: two bins
  * per step made it 18% slower. */
-constexpr int CORE_W = 1024;
 constexpr int CORE_WARPS = 4;
-
-/* one row of doubles per warp, as wide as a sub-tile */
-__host__ __device__ constexpr int core_row(int tile_w) { return tile_w < CORE_W ? tile_w : CORE_W; }
 
 /* the core of a line as single-region bin ranges, c3 within c2 within c1
  * (an empty inner range collapses to a point):
@@ -2150,7 +2146,7 @@ __device__ __forceinline__ void scatter_phase(int a, int b, int lane, const Core
 /* the first tile whose rows begin at row or later */
 __device__ __forceinline__ int row_tile(const KArgs& a, long long row)
 {
-    int lo = 0, hi = a.nitems;
+    int lo = 0, hi = a.nitems * core_subtiles(a.tile_w);
     while (lo < hi) {
         const int m = (lo + hi) >> 1;
         if (__ldg(a.csl.rowbase + m) < row) lo = m + 1; else hi = m;
@@ -2169,14 +2165,15 @@ core_kernel(const KArgs args)
     __shared__ long long s_lohi[2];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int RW = core_row(args.tile_w);      /* doubles per warp row */
+    const int RW = core_width(args.tile_w);      /* doubles per warp row */
     double* row = s_rows + warp * RW;
     constexpr bool DD = PREC == GEXS_FP64;
     const int LO = DD ? CORE_WARPS * RW : 0;   /* the low parts' rows */
     double* scr = s_rows + CORE_WARPS * RW + warp * SCR_D;
     if (!DD) for (int z = lane; z < SCR_D; z += 32) scr[z] = 0.0;
-    /* sliced (host-enabled only when a tile is one sub-tile of CORE_W) */
+    /* sliced: an item is a core tile, or a slice of one; else a whole tile */
     const bool sliced = args.csl.prefix != nullptr;
+    const bool subs = PREC == GEXS_FP64 && sliced && args.tile_w > CORE_W;
     __shared__ int s_last;
     /* read by every thread: a branch of thread 0 here would run into the one
      * at the loop's head, and warp 0 then reached the barriers in two parts */
@@ -2193,19 +2190,20 @@ core_kernel(const KArgs args)
         if (item >= nitems) break;
         int ti = item, sidx = 0, ns = 1;
         if (sliced) {
-            int tl = 0, th = args.nitems;
+            int tl = 0, th = subs ? args.nitems * core_subtiles(args.tile_w) : args.nitems;
             while (th - tl > 1) { int m = (tl + th) >> 1; if (__ldg(args.csl.prefix + m) <= item) tl = m; else th = m; }
             ti = tl;
             sidx = item - __ldg(args.csl.prefix + tl);
             ns = __ldg(args.csl.prefix + tl + 1) - __ldg(args.csl.prefix + tl);
         }
         int tj = 0;
-        const int jl = tile_job<ORDER>(args, ti, &tj);
+        const int jl = tile_job<ORDER>(args, subs ? ti / core_subtiles(args.tile_w) : ti, &tj);
         const gexs_job* Jp = args.jobs + jl;
         const gexs_job& J = *Jp;
-        /* the region-I kernel's tile of this item */
-        const int64_t t0 = J.start_idx + (int64_t)tj * args.tile_w;
-        const int64_t tend = min((int64_t)(t0 + args.tile_w), J.start_idx + J.n_points);
+        /* the region-I kernel's tile of this item, or its sub-tile */
+        const int64_t t0 = J.start_idx + (int64_t)tj * args.tile_w +
+                           (subs ? ti % core_subtiles(args.tile_w) * CORE_W : 0);
+        const int64_t tend = min((int64_t)(t0 + (subs ? CORE_W : args.tile_w)), J.start_idx + J.n_points);
         const int64_t nl = J.lines.count;
         const double* pb = PREP ? args.prep[jl] : nullptr;
         for (int64_t s0 = t0; s0 < tend; s0 += CORE_W) {
@@ -2354,7 +2352,7 @@ core_kernel(const KArgs args)
                  * ticket, and the last slice adds the partial rows in slice
                  * order (a zero total adds nothing, as above) */
                 const int rb = args.csl.rowbase[ti] - args.row0;
-                const int W = args.tile_w, RS = DD ? 2 * W : W;
+                const int W = DD ? RW : args.tile_w, RS = DD ? 2 * W : W;
                 double* prow = args.csl.rows + (size_t)(rb + sidx) * RS;
                 for (int t = tid; t < T.jn; t += NT) {
                     double hi, lo;
@@ -2500,7 +2498,7 @@ static cudaError_t launch_core(const KArgs& a, int nsm, cudaStream_t st)
 {
     auto kern = a.order ? core_kernel<PK, PREC, PREP, true> : core_kernel<PK, PREC, PREP, false>;
     const size_t smem = (size_t)CORE_WARPS * sizeof(double) *
-                        (PREC == GEXS_FP64 ? 2 * core_row(a.tile_w) : core_row(a.tile_w) + SCR_D);
+                        (PREC == GEXS_FP64 ? 2 * core_width(a.tile_w) : core_width(a.tile_w) + SCR_D);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int occ = 0;
