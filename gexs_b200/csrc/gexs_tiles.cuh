@@ -2488,13 +2488,14 @@ static cudaError_t launch_cfg(const KArgs& a, const gexs_launch_cfg& c, int nsm,
     }
 }
 
-/* the FP32 Voigt core kernel after the tile kernel, on the same stream; its
- * work counter is the int 128 bytes after the tile kernel's (the launch
- * tables reserve 256 bytes for counters) */
+/* the core kernel after the tile kernel, on the same stream, or alone where
+ * it is the whole profile (ctas_per_sm holds for it then); its work counter
+ * is the int 128 bytes after the tile kernel's (the launch tables reserve
+ * 256 bytes for counters) */
 constexpr int CORE_COUNTER_OFFSET = 32;
 
 template <int PK, int PREC, bool PREP>
-static cudaError_t launch_core(const KArgs& a, int nsm, cudaStream_t st)
+static cudaError_t launch_core(const KArgs& a, int ctas_per_sm, int nsm, cudaStream_t st)
 {
     auto kern = a.order ? core_kernel<PK, PREC, PREP, true> : core_kernel<PK, PREC, PREP, false>;
     const size_t smem = (size_t)CORE_WARPS * sizeof(double) *
@@ -2504,8 +2505,10 @@ static cudaError_t launch_core(const KArgs& a, int nsm, cudaStream_t st)
     int occ = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, CORE_WARPS * 32, smem);
     if (e != cudaSuccess) return e;
+    if (occ < 1) occ = 1;
+    if (PK == PK_ERF && ctas_per_sm > 0) occ = min(occ, ctas_per_sm);
     /* sliced: the item count is known on the device only */
-    const int grid = a.csl.prefix ? max(occ, 1) * nsm : max(1, min(a.nitems, max(occ, 1) * nsm));
+    const int grid = a.csl.prefix ? occ * nsm : max(1, min(a.nitems, occ * nsm));
     KArgs c = a;
     c.counter = a.counter + CORE_COUNTER_OFFSET;
     const int step = a.csl.prefix ? a.csl.round_rows : 0;
@@ -2532,8 +2535,8 @@ static cudaError_t launch_pk(int prec, const KArgs& a, const gexs_launch_cfg& cf
                              : launch_cfg<PK, GEXS_FP32, false>(a, cfg, nsm, st);
         if constexpr (PK == PK_VOIGT) {
             if (e != cudaSuccess) return e;
-            return prep ? launch_core<PK, GEXS_FP32, true>(a, nsm, st)
-                        : launch_core<PK, GEXS_FP32, false>(a, nsm, st);
+            return prep ? launch_core<PK, GEXS_FP32, true>(a, cfg.ctas_per_sm, nsm, st)
+                        : launch_core<PK, GEXS_FP32, false>(a, cfg.ctas_per_sm, nsm, st);
         }
         return e;
     }
@@ -2543,8 +2546,8 @@ static cudaError_t launch_pk(int prec, const KArgs& a, const gexs_launch_cfg& cf
         if (PK != PK_VOIGT || e != cudaSuccess) return e;
     }
     if constexpr (PK == PK_VOIGT || PK == PK_ERF)
-        return prep ? launch_core<PK, GEXS_FP64, true>(a, nsm, st)
-                    : launch_core<PK, GEXS_FP64, false>(a, nsm, st);
+        return prep ? launch_core<PK, GEXS_FP64, true>(a, cfg.ctas_per_sm, nsm, st)
+                    : launch_core<PK, GEXS_FP64, false>(a, cfg.ctas_per_sm, nsm, st);
     return cudaErrorInvalidValue;
 }
 
