@@ -328,7 +328,8 @@ static int64_t max_lines(const Group& g)
 
 /* the kernels of one group whose image is at d */
 static cudaError_t enqueue_group(const Group& g, const Layout& L, unsigned char* d, bool prep,
-                                 const gexs_launch_cfg& cfg, int* d_err, int nsm, cudaStream_t s)
+                                 const gexs_launch_cfg& cfg, int* d_err, int nsm, cudaStream_t s,
+                                 cudaEvent_t tiles_after = nullptr)
 {
     double* const* pp = reinterpret_cast<double* const*>(d + L.opp);
     SliceTables sl;
@@ -363,7 +364,7 @@ static cudaError_t enqueue_group(const Group& g, const Layout& L, unsigned char*
                         prep ? pp : nullptr, cfg, nsm, s, L.sliced ? &sl : nullptr,
                         L.csliced ? &csl : nullptr,
                         g.order.empty() ? nullptr : (const int*)(d + L.op) + g.prefix.size(),
-                        prep ? max_lines(g) : 0);
+                        prep ? max_lines(g) : 0, tiles_after);
 }
 
 extern "C" {
@@ -577,7 +578,7 @@ int gexs::run_scratch_bytes(gexs_ctx* ctx, const gexs_job* jobs, int njobs,
 }
 
 int gexs::run_jobs(gexs_ctx* ctx, const gexs_job* jobs, int njobs, const gexs_launch_cfg* cfg,
-                   void* stream, int* d_err)
+                   void* stream, int* d_err, cudaEvent_t tiles_after)
 {
     if (!ctx) return set_error(GEXS_ERR_INVALID, "ctx is NULL");
     if (!d_err) d_err = ctx->d_err;
@@ -601,7 +602,7 @@ int gexs::run_jobs(gexs_ctx* ctx, const gexs_job* jobs, int njobs, const gexs_la
         std::vector<unsigned char> h = group_image(g, L, (unsigned char*)d, prep);
         e = put_bytes(d, h.data(), h.size(), s);
         if (e != cudaSuccess) { cudaFreeAsync(d, s); return cuda_error(e, "upload launch tables"); }
-        e = enqueue_group(g, L, (unsigned char*)d, prep, cfgs[gi], d_err, ctx->nsm, s);
+        e = enqueue_group(g, L, (unsigned char*)d, prep, cfgs[gi], d_err, ctx->nsm, s, tiles_after);
         cudaFreeAsync(d, s);
         if (e != cudaSuccess) return cuda_error(e, "tile kernel launch");
     }

@@ -42,13 +42,14 @@ struct SliceTables {
  * 3 njobs + 1 ints, see tile_order in gexs_capi.cu), or NULL for job-major
  * items.
  * d_counter: a 256-byte block of work counters, zeroed by the caller: int 0
- * the tile kernel's, 16 the set-up kernel's, 32 the core kernel's. */
+ * the tile kernel's, 16 the set-up kernel's, 32 the core kernel's.
+ * tiles_after: an event that the kernels after the set-up wait for, or NULL. */
 cudaError_t launch_tiles(int pk, int prec, const gexs_job* d_jobs, const int* d_prefix,
                          int njobs, int nitems, int* d_counter, int* d_err,
                          double* const* d_prep, const gexs_launch_cfg& cfg, int nsm,
                          cudaStream_t st, const SliceTables* sl = nullptr,
                          const SliceTables* csl = nullptr, const int* d_order = nullptr,
-                         int64_t prep_lines = 0);
+                         int64_t prep_lines = 0, cudaEvent_t tiles_after = nullptr);
 /* The FP64 tile kernel sums a bin's lines in order within blocks of this
  * many lines of the list (by index, so that a tile of any shape or cut has
  * the same block sums) and the blocks' sums as (hi, lo) pairs, whose
@@ -135,9 +136,10 @@ cudaError_t zero_ints(int* p, int n, cudaStream_t st);
 cudaError_t take_word(int* word, int* out, cudaStream_t st);
 
 /* gexs_run with the kernels' error flags going to d_err (device int)
- * instead of the context's own word (NULL: the context's) */
+ * instead of the context's own word (NULL: the context's); the kernels after
+ * the set-up wait for the event tiles_after (NULL: none) */
 int run_jobs(gexs_ctx* ctx, const gexs_job* jobs, int njobs, const gexs_launch_cfg* cfg,
-             void* stream, int* d_err);
+             void* stream, int* d_err, cudaEvent_t tiles_after = nullptr);
 
 /* device scratch run_jobs takes from the context's pool for these jobs
  * (launch tables, per-job prep arrays, line-slice rows), in bytes */

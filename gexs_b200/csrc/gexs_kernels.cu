@@ -289,7 +289,7 @@ cudaError_t launch_tiles(int pk, int prec, const gexs_job* d_jobs, const int* d_
                          int njobs, int nitems, int* d_counter, int* d_err,
                          double* const* d_prep, const gexs_launch_cfg& cfg, int nsm,
                          cudaStream_t st, const SliceTables* sl, const SliceTables* csl,
-                         const int* d_order, int64_t prep_lines)
+                         const int* d_order, int64_t prep_lines, cudaEvent_t tiles_after)
 {
     KArgs a;
     a.jobs = d_jobs; a.prefix = d_prefix; a.njobs = njobs; a.nitems = nitems;
@@ -302,7 +302,8 @@ cudaError_t launch_tiles(int pk, int prec, const gexs_job* d_jobs, const int* d_
     std::memset(&a.csl, 0, sizeof(a.csl));
     if (sl && slices_apply(pk, prec)) a.sl = *sl;
     if (csl && core_slices_apply(pk, prec, a.tile_w)) a.csl = *csl;
-    const cudaError_t e = launch_setup(a, prep_lines, nsm, st);
+    cudaError_t e = launch_setup(a, prep_lines, nsm, st);
+    if (e == cudaSuccess && tiles_after) e = cudaStreamWaitEvent(st, tiles_after, 0);
     if (e != cudaSuccess) return e;
     switch (pk) {
     case PK_VOIGT: return launch_tiles_voigt(prec, a, cfg, nsm, st);

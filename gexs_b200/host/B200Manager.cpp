@@ -11,11 +11,13 @@
 #include <thread>
 #include <vector>
 #include <cuda_runtime.h>
+#include "../csrc/gexs_internal.h"
 
 namespace {
 const int kCopyChunks = 64;                     /* pieces of an overlapped line copy */
 const int kSegments = 6;                        /* grid segments of the first launch  */
 const double kSegmentFrac[kSegments] = {1.0 / 64, 1.0 / 32, 1.0 / 8, 1.0 / 4, 1.0 / 2, 1.0};
+const double kLongSegment = 1e11;               /* evaluations of a last segment that waits, see below */
 const int64_t kSegmentAlign = 4096;             /* widest tile: 32 lanes x 16 bins x 8 warps */
 const size_t kSegmentMinLines = (size_t)1 << 21;
 const size_t kSamples = 8192;
@@ -262,7 +264,18 @@ int B200Manager::flush()
  * each tile's own search selects, so each tile finds the same lines in the
  * same order) and started once the pieces holding that sub-list have
  * arrived.  Segment boundaries sit at start_idx + k * kSegmentAlign, so
- * every tile is the tile of a single launch over the pair. */
+ * every tile is the tile of a single launch over the pair.
+ *
+ * The FP32 Voigt region-I kernel's CTAs stay for the whole launch, four per
+ * SM with 54 of its 228 KB of shared memory each.  Started while the core
+ * kernel of the segment before drains (35 KB a CTA), they are placed in the
+ * holes of pairs of those and three of them fill an SM, to the end: the last
+ * segment of 1e8 lines, half of them, took 89.5 ms instead of 84.9.  So a
+ * long last segment's kernels, its set-up apart, wait for the segment
+ * before: 206.3 -> 201.8 ms for the whole pass.  A short one would lose more
+ * by the wait than it gains (1e7 lines 23.2 -> 23.8 ms, 3e7 63.2 -> 63.7),
+ * and one whose lines arrive well before the segment before has drained
+ * loses a little (5e7 lines at 0.005 cm^-1 179.6 -> 180.2 ms). */
 int B200Manager::run_segmented()
 {
     cudaStream_t s0 = (cudaStream_t)stream_;
@@ -317,6 +330,7 @@ int B200Manager::run_segmented()
         if (cudaStreamWaitEvent((cudaStream_t)sk, (cudaEvent_t)fork_ev_, 0) != cudaSuccess)
             return GEXS_ERR_CUDA;
     int st = GEXS_OK;
+    cudaEvent_t before = nullptr;       /* the segment before has finished */
     for (int k = 0; k < kSegments && st == GEXS_OK; ++k) {
         if (seg[k].empty()) continue;
         cudaStream_t s = k == 0 ? s0 : (cudaStream_t)seg_stream_[k - 1];
@@ -324,7 +338,16 @@ int B200Manager::run_segmented()
             const size_t c = std::min((size_t)nchunks_ - 1, (need[k] - 1) / chunk_lines_);
             if (cudaStreamWaitEvent(s, (cudaEvent_t)chunk_ev_[c], 0) != cudaSuccess) { st = GEXS_ERR_CUDA; break; }
         }
-        st = gexs_run(ctx_, seg[k].data(), (int)seg[k].size(), nullptr, s);
+        double evals = 0.0;
+        for (const gexs_job& p : seg[k]) evals += (double)p.lines.count * 2.0 * p.cutoff / p.dnu;
+        const bool wait = k == kSegments - 1 && precision_ == GEXS_FP32 && profile == VOIGT &&
+                          evals >= kLongSegment;
+        st = gexs::run_jobs(ctx_, seg[k].data(), (int)seg[k].size(), nullptr, s, nullptr,
+                            wait ? before : nullptr);
+        if (k > 0 && k < kSegments - 1 && st == GEXS_OK) {
+            before = (cudaEvent_t)join_ev_[k - 1];
+            if (cudaEventRecord(before, s) != cudaSuccess) st = GEXS_ERR_CUDA;
+        }
     }
     /* stream_ joins every segment stream and has seen every piece arrive */
     bool ok = true;
