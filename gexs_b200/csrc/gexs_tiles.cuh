@@ -2060,6 +2060,15 @@ __device__ __forceinline__ double core_term2_f32(const CoreLine& l, int t)
     return (double)__fmul_rn(l.ampf, hum_region2<float>(x, l.yf));
 }
 
+/* n / m for 0 <= n <= 2048 and 1 <= m <= 32 as n c >> 16 with c = div_of(m):
+ * 2^16 / m rounded down, plus one (m a power of two: or 2^16 / m itself), for
+ * which every n and m was checked.  Five divisions by variables for each
+ * phase of a group cost a quarter of the walk where ranges are short: core
+ * of 1e8 lines on 3e6 bins at 100 K, 1e-5 bar 18.2 ms with them, 15.7 ms so,
+ * and 14.2 with M down to 2 instead of 4; at 3000 K 31.7 and 27.5. */
+__device__ __forceinline__ int div_of(int m) { return (int)(65536.f * rcp_approx((float)m)) + 1; }
+__device__ __forceinline__ int div_small(int n, int c) { return (n * c) >> 16; }
+
 /* LO = 0: plain sums.  LO > 0 (the FP64 form): row[t] and row[LO + t] are a
  * (hi, lo) sum, because that form's results are the same for every tile
  * shape and cut (SUM_BLOCK) and the order of the terms here is not; no
@@ -2077,9 +2086,11 @@ __device__ __forceinline__ void scatter_phase(int a, int b, int lane, const Core
      * after another, a bin per lane; a step of this form costs about a third
      * more (the line's values travel by shuffles, the term is a call).
      * 564 lines on 2.7e5 bins: 20 against 66 us for the bin-by-bin form. */
-    const int steps = (int)__reduce_add_sync(ALL, (unsigned)(max(b - a, 0) + 31) / 32);
+    const unsigned active = __ballot_sync(ALL, a < b);
+    const int steps = longest <= 32 ? __popc(active)
+                                    : (int)__reduce_add_sync(ALL, (unsigned)(max(b - a, 0) + 31) / 32);
     if (steps * 4 < longest * 3) {
-        unsigned todo = __ballot_sync(ALL, a < b);
+        unsigned todo = active;
         while (todo) {
             const int src = __ffs(todo) - 1;
             todo &= todo - 1;
@@ -2095,11 +2106,16 @@ __device__ __forceinline__ void scatter_phase(int a, int b, int lane, const Core
         }
         return;
     }
-    const int passes = (longest + 31) / 32;
-    const int M = max((longest + passes - 1) / passes, 4);
-    const int groups = (31 + M) / M, mine = lane / M;
+    /* FP32: ranges of one or two bins in steps as many */
+    int M = max(longest, DD ? 4 : 2);
+    if (longest > 32) {
+        const int passes = (longest + 31) / 32;
+        M = (longest + passes - 1) / passes;
+    }
+    const int by_m = div_of(M);
+    const int groups = div_small(31 + M, by_m), mine = div_small(lane, by_m);
     int lo = 0, span = 0;
-    const int strip = SCR_D / groups;
+    const int strip = div_small(SCR_D, div_of(groups));
     if (!DD && groups > 1) {
         lo = __reduce_min_sync(ALL, a < b ? a : INT32_MAX);
         span = __reduce_max_sync(ALL, a < b ? b : INT32_MIN) - lo;
@@ -2107,8 +2123,9 @@ __device__ __forceinline__ void scatter_phase(int a, int b, int lane, const Core
     const bool strips = !DD && groups > 1 && span <= strip;
     double* dst = strips ? scr + mine * strip - lo : row;
     const int rounds = strips ? 1 : groups;
-    int o = (lane - a) % M;
-    if (o < 0) o += M;
+    int o = a + 32 * M - lane;              /* (lane - a) mod M */
+    o -= M * div_small(o, by_m);
+    if (o) o = M - o;
     for (int base = 0; base < longest; base += M) {
 #pragma unroll 1
         for (int k = 0; k < M; ++k) {
