@@ -143,6 +143,7 @@ def _cfg(cfg):
 class Batch:
     def __init__(self, ctx, jobs, cfg=None):
         self._jobs = list(jobs)
+        self._ctx = ctx              # the batch's kernels and its destruction use it
         self.h = C.c_void_p()
         arr = _job_array(self._jobs)
         check(lib().gexs_batch_create(ctx.h, arr, len(arr), _cfg(cfg), C.byref(self.h)),
