@@ -297,6 +297,7 @@ cudaError_t launch_tiles(int pk, int prec, const gexs_job* d_jobs, const int* d_
     a.counter = d_counter; a.err = d_err; a.prep = d_prep;
     a.tile_w = tile_bins(cfg);
     a.row0 = 0;
+    a.subs = 1;
     a.spin = cfg.wait_spins > 0 ? cfg.wait_spins : WS_SPIN;
     std::memset(&a.sl, 0, sizeof(a.sl));
     std::memset(&a.csl, 0, sizeof(a.csl));
@@ -410,8 +411,9 @@ long long slice_lines(const gexs_job* jobs, int njobs, int prec, int tile_w, int
      * workload is indifferent to 16k-128k, a dense band of 1e6 lines in 80
      * cm^-1 runs 25% faster than at 65536.
      * FP64 (any cut gives the same sums): about eight items for each of the
-     * CTAs that fit (888 of 740 to 888), of 512 to 4096 lines.  2e5 lines on 194 tiles
-     * (GH32): 8.2 ms against 34 ms uncut. */
+     * 740 (Voigt, 4 x 4) to 444 (quadrature, 4 x 8) CTAs that fit, of 512 to
+     * 4096 lines.  Uncut, 2e5 lines on 194 tiles (GH32) took four times as
+     * long. */
     double m = 0.0;
     for (int i = 0; i < njobs; ++i) m += tile_entries(jobs[i], jobs[i].cutoff, tile_w);
     long long per = 16384;

@@ -58,7 +58,7 @@ struct __align__(16) RecF32 {   /* 48 bytes; Doppler/Gaussian and GH */
     float fc;              /* tc - floor(tc) in [0, 1)                       */
     int   win;             /* a | b << 16 : bins [a, b) of the tile; Doppler:
                               those whose xm <= the zero threshold           */
-    int   c1;
+    int   pad0;
     int   mask;            /* GH, per warp w: bit w touches, bit 8+w fast tier,
                               bit 16+w mid tier; bit 24: |x| may exceed 1e8
                               in this tile (overflow-free forms); bit 25 (GH):
@@ -374,6 +374,8 @@ struct KArgs {
     SliceTables     sl;        /* line slices (sl.prefix NULL: none)     */
     SliceTables     csl;       /* core kernel's slices                   */
     int             row0;      /* core kernel: first row of its round    */
+    int             subs;      /* core kernel: core tiles of a tile, whose
+                                  width tile_w then is                   */
     int             spin;      /* try_wait attempts of every bounded wait */
     const int*      order;     /* tile-major order tables F|R|P, or NULL
                                   for job-major items (gexs_capi.cu
@@ -413,8 +415,9 @@ __device__ __forceinline__ void kahan_add(float& s, float& c, float v)
     s = t;
 }
 
-/* (hi, lo) += v with the rounding error kept (Knuth's TwoSum): sums of the
- * same terms in another order round to the same double */
+/* (hi, lo) += v with the rounding error kept (Knuth's TwoSum; the errors are
+ * summed in plain FP64): sums of the same terms in another order round to
+ * the same double unless hi + lo lies within some 2^-105 of a tie */
 __device__ __forceinline__ void dd_add(double& hi, double& lo, double v)
 {
     const double s = dadd(hi, v), bb = dsub(s, hi);
@@ -478,7 +481,7 @@ __device__ __forceinline__ void make_rec(RecF32& q, const Derived<PK>& d, const 
     q.fc = fc;
     /* erf: the non-zero bins, a sub-range of the window */
     q.win = PK == PK_ERF ? (d.win == 0 ? 0 : d.c1) : d.win;
-    q.c1 = 0;
+    q.pad0 = 0;
     q.mask = 0;
     if constexpr (PK != PK_ERF) {
         /* largest |x| the line reaches in this tile */
@@ -665,7 +668,7 @@ __device__ __forceinline__ void lines_f32(const RecF32* __restrict__ rec, int nr
         const float wbf = (float)wb, lanef = (float)lane;
         const int bit = 1 << warp;
         for (int i = 0; i < nrec; ++i) {
-            const int4 qi = *reinterpret_cast<const int4*>(&rec[i].win);   /* win c1 mask pad */
+            const int4 qi = *reinterpret_cast<const int4*>(&rec[i].win);   /* win pad0 mask pad */
             const int mask = qi.z;
             if (!(mask & bit)) continue;
             const float4 q0 = *reinterpret_cast<const float4*>(&rec[i].icf);   /* icf dx mfcdx a1 */
@@ -2163,7 +2166,7 @@ __device__ __forceinline__ void scatter_phase(int a, int b, int lane, const Core
 /* the first tile whose rows begin at row or later */
 __device__ __forceinline__ int row_tile(const KArgs& a, long long row)
 {
-    int lo = 0, hi = a.nitems * core_subtiles(a.tile_w);
+    int lo = 0, hi = a.nitems * a.subs;
     while (lo < hi) {
         const int m = (lo + hi) >> 1;
         if (__ldg(a.csl.rowbase + m) < row) lo = m + 1; else hi = m;
@@ -2190,7 +2193,6 @@ core_kernel(const KArgs args)
     if (!DD) for (int z = lane; z < SCR_D; z += 32) scr[z] = 0.0;
     /* sliced: an item is a core tile, or a slice of one; else a whole tile */
     const bool sliced = args.csl.prefix != nullptr;
-    const bool subs = PREC == GEXS_FP64 && sliced && args.tile_w > CORE_W;
     __shared__ int s_last;
     /* read by every thread: a branch of thread 0 here would run into the one
      * at the loop's head, and warp 0 then reached the barriers in two parts */
@@ -2207,20 +2209,20 @@ core_kernel(const KArgs args)
         if (item >= nitems) break;
         int ti = item, sidx = 0, ns = 1;
         if (sliced) {
-            int tl = 0, th = subs ? args.nitems * core_subtiles(args.tile_w) : args.nitems;
+            int tl = 0, th = args.nitems * args.subs;
             while (th - tl > 1) { int m = (tl + th) >> 1; if (__ldg(args.csl.prefix + m) <= item) tl = m; else th = m; }
             ti = tl;
             sidx = item - __ldg(args.csl.prefix + tl);
             ns = __ldg(args.csl.prefix + tl + 1) - __ldg(args.csl.prefix + tl);
         }
         int tj = 0;
-        const int jl = tile_job<ORDER>(args, subs ? ti / core_subtiles(args.tile_w) : ti, &tj);
+        const int jl = tile_job<ORDER>(args, args.subs > 1 ? ti / args.subs : ti, &tj);
+        if (args.subs > 1) tj = tj * args.subs + ti % args.subs;
         const gexs_job* Jp = args.jobs + jl;
         const gexs_job& J = *Jp;
         /* the region-I kernel's tile of this item, or its sub-tile */
-        const int64_t t0 = J.start_idx + (int64_t)tj * args.tile_w +
-                           (subs ? ti % core_subtiles(args.tile_w) * CORE_W : 0);
-        const int64_t tend = min((int64_t)(t0 + (subs ? CORE_W : args.tile_w)), J.start_idx + J.n_points);
+        const int64_t t0 = J.start_idx + (int64_t)tj * args.tile_w;
+        const int64_t tend = min((int64_t)(t0 + args.tile_w), J.start_idx + J.n_points);
         const int64_t nl = J.lines.count;
         const double* pb = PREP ? args.prep[jl] : nullptr;
         for (int64_t s0 = t0; s0 < tend; s0 += CORE_W) {
@@ -2369,7 +2371,7 @@ core_kernel(const KArgs args)
                  * ticket, and the last slice adds the partial rows in slice
                  * order (a zero total adds nothing, as above) */
                 const int rb = args.csl.rowbase[ti] - args.row0;
-                const int W = DD ? RW : args.tile_w, RS = DD ? 2 * W : W;
+                const int W = args.tile_w, RS = DD ? 2 * W : W;
                 double* prow = args.csl.rows + (size_t)(rb + sidx) * RS;
                 for (int t = tid; t < T.jn; t += NT) {
                     double hi, lo;
@@ -2528,6 +2530,10 @@ static cudaError_t launch_core(const KArgs& a, int ctas_per_sm, int nsm, cudaStr
     const int grid = a.csl.prefix ? occ * nsm : max(1, min(a.nitems, occ * nsm));
     KArgs c = a;
     c.counter = a.counter + CORE_COUNTER_OFFSET;
+    if (a.csl.prefix) {
+        c.subs = core_subtiles(a.tile_w);
+        c.tile_w = core_width(a.tile_w);
+    }
     const int step = a.csl.prefix ? a.csl.round_rows : 0;
     for (long long row = 0;; row += step) {
         c.row0 = (int)row;
