@@ -1991,10 +1991,12 @@ voigt_ws_kernel(const KArgs args)
  * all lanes of a step are in the same region, and neighbouring lines have
  * nearly equal ranges, so most lanes work.  Stepping the union of the 32
  * cores bin by bin instead (every lane at the same bin, a butterfly per
- * bin) ran each region's code at nearly every step: 10.0 against 2.9 ms for
+ * bin) ran each region's code at nearly every step: 10.0 against 2.7 ms for
  * eight (T, P) pairs of a 1e6-line list (sparse, fine grids), 6.0 against
- * 5.0 ms for a dense 2e7-line list at 1 bar, 33 against 23 us for 3000
- * lines on 6001 bins.  Instruction fetches bound the dense case: two bins
+ * 4.3 ms for a dense 2e7-line list at 1 bar, 33 against 18 us for 3000
+ * lines on 6001 bins.  Only where lines are both dense and narrow is the
+ * union hardly longer than a range: 1e8 lines on 3e6 bins at 100 K, 12.3
+ * against 14.3 ms.  Instruction fetches bound the dense case: two bins
  * per step made it 18% slower. */
 constexpr int CORE_WARPS = 4;
 
