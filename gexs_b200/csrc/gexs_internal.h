@@ -112,8 +112,8 @@ __host__ __device__ inline int core_slices(long long n, long long grid_points, i
 }
 bool core_slices_apply(int pk, int prec, int tile_w);
 /* partial rows of a launch's core slices: a bound on their number (false:
- * more than an int holds), the rows of a round (0: all fit in ROW_BYTES and
- * there is one round) and those to allocate.  With several rounds the core
+ * more than an int holds), the rows of a round (0: all are held and there is
+ * one round) and those to allocate.  With several rounds the core
  * kernel is launched once for each range of round_rows rows, over the tiles
  * whose rows begin there, and the ranges share the memory; the last tile's
  * rows may reach past the range. */

@@ -399,7 +399,8 @@ bool core_rows(const gexs_job* jobs, int njobs, int prec, int tile_w, CoreRows* 
     if (!(total < (double)INT32_MAX)) return false;
     const long long fit = ROW_BYTES / ((long long)sizeof(double) * row_doubles(prec, tile_w));
     out->bound = (int)total;
-    out->round_rows = total <= (double)fit ? 0 : (int)fit;
+    /* never more than the jobs would take one by one */
+    out->round_rows = total <= (double)(fit + most) ? 0 : (int)fit;
     out->alloc = out->round_rows ? (int)(fit + most) : out->bound;
     return true;
 }
